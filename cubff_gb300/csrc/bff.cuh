@@ -1,12 +1,793 @@
 // bff.cuh — the BFF family interpreters (bff, bff_noheads, bff_noheads_4bit,
-// bff_perm, bff8, bff8_noheads, bff_selfmove) as resumable machines.
+// bff_perm, bff8, bff8_noheads, bff_selfmove).
 //
 // Semantics: Evaluate (bff.inc.h:356-389), InitialState (bff.inc.h:269-283),
 // EvaluateOne: default (bff.inc.h:289-349), bff8 / bff8_noheads (bff8.cu:23-65),
 // bff_selfmove (bff_selfmove.cu:47-98).  The op of a byte comes from the
 // language's table (optab, BffOp values).
 //
-// Work per step is reduced without changing results:
+// Three machines with the same results:
+//  * BffLane, one pair per lane: runs a program until it ends or first jumps
+//    (most random programs never do);
+//  * BffWarp, one pair per warp, which takes over from there;
+//  * BffBasic, the one-shot one of the per-epoch kernels (bff_eval).
+#pragma once
+
+#include "coop.cuh"
+#include "languages.cuh"
+
+namespace cubff {
+
+enum BffLogic { kLogicScan, kLogicJump8, kLogicSelfmove };
+
+// Where a program stands, handed from one machine to the next.
+struct BffState {
+  int q;             // position of the command to execute
+  int h0, h1;        // heads
+  uint32_t i, n;     // raw steps before q's command (the no-ops before it included: the
+                     // reference counts each as a step and a skip); commands executed,
+                     // which is the reference's op count
+  uint32_t mods;     // writes that changed a byte
+};
+
+// The forward part of a program on one lane.  The lanes of a warp are at
+// different commands, so a step is one straight line of instructions for all
+// of them: head moves and value writes all computed and selected.  S marks
+// the positions that hold, or once held, a command (a write only ever sets
+// bits; a command overwritten by a no-op costs a step that counts no op), so
+// a run of no-ops is crossed by finding the next one.
+template <bool kHeads, int kLogic, uint32_t kNullMask>
+struct BffLane {
+  enum Status : uint32_t { kRuns, kEnds, kJumps };
+  BffState st;
+  uint32_t status;
+  uint32_t c;         // op of the command at q
+  uint32_t v0, v1;    // bytes under the heads
+  Mask128 S;
+
+  // cmd_mask: bit p set iff tape byte p is a command (op < kNull).
+  template <class Tape>
+  __host__ __device__ __forceinline__ void begin(const Tape t, Mask128 cmd_mask,
+                                                 const uint8_t *__restrict__ optab) {
+    S = cmd_mask;
+    st.h0 = kHeads ? t.get(0) & (kPair - 1) : 0;  // no heads: 2 * kSingleTapeSize, masked
+    st.h1 = kHeads ? t.get(1) & (kPair - 1) : 0;
+    st.i = st.n = st.mods = 0;
+    fetch(t, optab, kHeads ? 2 : 0);
+  }
+
+  // Moves on to the command at or after position p.
+  template <class Tape>
+  __host__ __device__ __forceinline__ void fetch(const Tape t,
+                                                 const uint8_t *__restrict__ optab, int p) {
+    v0 = t.get(st.h0);
+    v1 = t.get(st.h1);
+    st.q = mask_next(S, p);
+    st.i += static_cast<uint32_t>(st.q - p);
+    c = optab[t.get(st.q & (kPair - 1))];
+    const bool zero = (v0 & kNullMask) == 0;
+    const bool jumps = c == kLoopStart ? zero : c == kLoopEnd && !zero;
+    status = st.q >= kPair ? kEnds : jumps ? kJumps : kRuns;
+  }
+
+  // One command that does not jump (fewer than kPair run, so the step limit is
+  // never reached).
+  template <class Tape>
+  __host__ __device__ __forceinline__ void step(const Tape t,
+                                                const uint8_t *__restrict__ optab) {
+    st.h0 = (st.h0 + (c == kInc0) - (c == kDec0)) & (kPair - 1);
+    st.h1 = (st.h1 + (c == kInc1 || (kLogic == kLogicSelfmove && c == kCopy10)) - (c == kDec1)) &
+            (kPair - 1);
+    const bool to1 = c == kCopy01, from1 = c == kCopy10;
+    const uint32_t v = ((from1 ? v1 : v0) + (c == kPlus) - (c == kMinus)) & 0xFF;
+    const uint32_t o = to1 ? v1 : v0;
+    if (c - kPlus < 4u && v != o) {
+      const int a = to1 ? st.h1 : st.h0;
+      t.set(a, v);
+      st.mods++;
+      if (optab[v] < kNull) mask_assign(S, a, true);
+    }
+    st.n += c < kNull;
+    st.i++;
+    fetch(t, optab, st.q + 1);
+  }
+
+  // A taken ']' with no '[' before it ends the program (bff8: one that would
+  // jump off the tape): tells that from a jump that goes on.
+  template <class Tape>
+  __host__ __device__ __forceinline__ void resolve(const Tape t,
+                                                   const uint8_t *__restrict__ optab) {
+    if (c != kLoopEnd) return;
+    if (kLogic == kLogicJump8) {
+      if (st.q >= 8) return;
+    } else {
+      for (int b = mask_prev(S, st.q - 1); b >= 0; b = mask_prev(S, b - 1))
+        if (optab[t.get(b)] == kLoopStart) return;
+    }
+    st.n++;
+    st.i++;
+    status = kEnds;
+  }
+};
+
+// Shared memory of one warp's BffWarp.
+struct alignas(16) BffMem {
+  uint8_t T[kPair];      // the pair tape
+  uint8_t snap[kPair];   // its snapshot at a taken ']'
+  uint8_t top[kPair];    // its snapshot at the top of a loop
+  uint16_t E[kPair];     // op | position of the next command << 8 (kPair: none)
+  uint8_t D[kPair];      // '[' minus ']' up to and including the position, mod 256
+  uint16_t M[kPair];     // bracket matches: position | straight << 7, kNone or kUnknown
+  uint32_t P[8];         // micro-ops of the compiled loop
+  uint8_t X[kWarp];      // one byte per lane
+};
+static_assert(sizeof(BffMem) % 16 == 0, "BffMem");
+
+// One pair on a whole warp, from its first jump on.
+//
+// What bounds it: the chain of dependent instructions of one program (~4.4
+// cycles each), so the lanes are used to make that chain short:
+//  * decoding (the ops, the next command after every position, bracket
+//    depths) is done for all 128 positions at once.  A write that changes a
+//    byte's op only widens the range [dlo, dhi] of positions changed since;
+//    what is used of the decode must lie outside it, else it is redone (a
+//    replicator writes the other program's bytes while it runs its own);
+//  * a bracket's match is found on bit masks, or over the depths when other
+//    brackets lie between, and kept;
+//  * a loop [ ... ] without inner brackets is compiled to micro-ops (the net
+//    head moves up to the next '+' / '-' run, copy or the ']', and that
+//    command, at most 8) and counts once per iteration.  Bodies with at most
+//    one copy run up to 32 iterations at a time, one per lane; a body that only
+//    counts the tested byte is solved; others go micro-op by micro-op.  A write
+//    into the loop's own code leaves the loop before the command that does it
+//    (a byte changed to another of the same op does not count);
+//  * exact cycle fast-forward at other taken ']'s, on Brent's schedule
+//    (cycle.cuh): the state is (position, heads, tape), and the tape is
+//    compared with a snapshot four bytes per lane.  Head 1 may differ when no
+//    copy used it since the snapshot (every ']' tests the byte under head 0):
+//    control flow depends only on the rest, so the segment since the snapshot
+//    repeats with that head shifted by the same amount each time; k
+//    repetitions advance i, n and the head by k times the segment's;
+//  * a compiled loop moves its heads by the same net amounts each iteration,
+//    so they are back after `period` iterations (at most 128).  As many
+//    iterations in a row without a changed byte and without leaving mean that
+//    none will ever come: the loop runs to the step limit.
+//
+// Uniform stores are made by all lanes together (the same value to the same
+// place; every branch here is uniform, so the lanes stay together), and every
+// lane reads its own; lane-wise ones are followed by a sync.
+template <class W, int kLogic, uint32_t kNullMask>
+struct BffWarp {
+  static constexpr uint32_t kSettle = 8;  // micro-op loop iterations before the first visit
+  // Micro-ops: the net moves mod 128 at bits 0 and 8, act at 16, and what kAdd
+  // adds (a run of '+' or '-'), mod 256, at 24.
+  enum Act : uint32_t { kAdd, kTo0, kTest, kTo1 };  // (bit 0: a copy; both bits: to head 1)
+  enum Kind : uint32_t { kGeneric, kCopyOne, kCount };
+  static constexpr int kEnd = -1, kRedo = -2;
+  static constexpr uint32_t kNone = 0x100, kUnknown = 0x200;
+
+  const W w;
+  BffMem &m;
+  const uint8_t *const optab;
+  BffState st;
+  uint32_t v0, v1;    // bytes under the heads (not kept up to date in loops)
+  int dlo, dhi;       // positions whose op changed since the decode (none: dlo > dhi)
+  uint32_t open[4], close[4];  // brackets, 32 positions a word
+  bool used1;         // a copy used head 1 since the snapshot
+  // The compiled loop: '[' at ls, ']' at le (-1: none), its micro-ops (m.P),
+  // the commands of an iteration, the net moves, its period and kind.
+  int ls, le, net0, net1;
+  uint32_t lcmds, period, kind;
+  bool copies;        // it has copies
+  // Taken ']'s still to step through one by one after a loop wrote into its
+  // own code at once, and as many the next time: so the cycle check sees them.
+  uint32_t hold, backoff;
+  uint32_t iters;     // iterations done in it
+  // Snapshot taken at a taken ']'.
+  int s_key, s_h0, s_h1;
+  uint32_t s_i, s_n, s_mods, s_power, s_lam;
+
+  __host__ __device__ __forceinline__ BffWarp(W warp, BffMem &mem, const uint8_t *table)
+      : w(warp), m(mem), optab(table) {}
+
+  __host__ __device__ __forceinline__ uint32_t word(const uint8_t *a, uint32_t l) const {
+    return reinterpret_cast<const uint32_t *>(a)[l];
+  }
+
+  // Ops, next commands, brackets and depths of all positions.
+  __host__ __device__ __forceinline__ void decode() {
+    if (dlo <= le && dhi >= ls) le = -1;
+    w.sync();
+    // Matches stay where no op between the two brackets changed.
+    w.each([&](uint32_t l) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint32_t r = m.M[32 * k + l];
+        const bool stays = r < kNone && clean(static_cast<int>(32 * k + l), static_cast<int>(r & 127));
+        m.M[32 * k + l] = static_cast<uint16_t>(stays ? r : kUnknown);
+      }
+    });
+    dlo = kPair;
+    dhi = -1;
+    const auto op0 = w.map([&](uint32_t l) { return uint32_t(optab[m.T[l]]); });
+    const auto op1 = w.map([&](uint32_t l) { return uint32_t(optab[m.T[32 + l]]); });
+    const auto op2 = w.map([&](uint32_t l) { return uint32_t(optab[m.T[64 + l]]); });
+    const auto op3 = w.map([&](uint32_t l) { return uint32_t(optab[m.T[96 + l]]); });
+    auto op = [&](int k, uint32_t l) {
+      return k == 0 ? op0(l) : k == 1 ? op1(l) : k == 2 ? op2(l) : op3(l);
+    };
+    uint32_t cmd[4], above[4];
+    int sum[4], total = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      cmd[k] = w.ballot([&](uint32_t l) { return op(k, l) < kNull; });
+      open[k] = w.ballot([&](uint32_t l) { return op(k, l) == kLoopStart; });
+      close[k] = w.ballot([&](uint32_t l) { return op(k, l) == kLoopEnd; });
+      sum[k] = total;
+      total += popc32(open[k]) - popc32(close[k]);
+    }
+    above[3] = kPair;
+#pragma unroll
+    for (int k = 2; k >= 0; k--) above[k] = cmd[k + 1] ? 32 * k + 32 + low32(cmd[k + 1]) : above[k + 1];
+    w.each([&](uint32_t l) {
+      const uint32_t upto = ~0u >> (31 - l);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        m.D[32 * k + l] =
+            static_cast<uint8_t>(sum[k] + popc32(open[k] & upto) - popc32(close[k] & upto));
+        const uint32_t x = cmd[k] & ~upto;
+        m.E[32 * k + l] =
+            static_cast<uint16_t>(op(k, l) | (x ? 32 * k + low32(x) : above[k]) << 8);
+      }
+    });
+    w.sync();
+  }
+
+  // Ops of positions lo..hi may have changed.
+  __host__ __device__ __forceinline__ void changed_op(int lo, int hi) {
+    dlo = lo < dlo ? lo : dlo;
+    dhi = hi > dhi ? hi : dhi;
+  }
+
+  // Writes v over o != v at position p.
+  __host__ __device__ __forceinline__ void write(int p, uint32_t o, uint32_t v) {
+    m.T[p] = static_cast<uint8_t>(v);
+    st.mods++;
+    if (optab[v] != optab[o]) changed_op(p, p);
+  }
+
+  // No op between a and b (in either order) changed since the decode.
+  __host__ __device__ __forceinline__ bool clean(int a, int b) const {
+    return dlo > (a > b ? a : b) || dhi < (a > b ? b : a);
+  }
+
+  // The match of the bracket at q (op c): position, | 128 when no brackets lie
+  // between; kNone when there is none; kUnknown when ops must be decoded again
+  // first.
+  __host__ __device__ __forceinline__ uint32_t match(int q, uint32_t c) {
+    uint32_t r = m.M[q];
+    if (r == kUnknown) r = search(q, c);
+    const bool stale = dlo <= dhi && (r == kNone || !clean(q, static_cast<int>(r & 127)));
+    return stale ? kUnknown : r;
+  }
+
+  // One set bit at or beyond which a search goes on: word k of the positions
+  // above q (fwd) or below it.
+  __host__ __device__ __forceinline__ static uint32_t beyond(int k, int q, bool fwd) {
+    const uint32_t upto = ~0u >> (31 - (q & 31));
+    return k == (q >> 5) ? (fwd ? ~upto : upto >> 1) : (k > (q >> 5)) == fwd ? ~0u : 0u;
+  }
+  // The first of the masked positions above q, or the last below it; -1.
+  __host__ __device__ __forceinline__ static int nearest(uint32_t x0, uint32_t x1, uint32_t x2,
+                                                         uint32_t x3, bool fwd) {
+    if (fwd) return x0 ? low32(x0) : x1 ? 32 + low32(x1) : x2 ? 64 + low32(x2) : x3 ? 96 + low32(x3) : -1;
+    return x3 ? 96 + high32(x3) : x2 ? 64 + high32(x2) : x1 ? 32 + high32(x1) : x0 ? high32(x0) : -1;
+  }
+  // match(), searched for and kept.
+  __host__ __device__ __forceinline__ uint32_t search(int q, uint32_t c) {
+    const bool fwd = c == kLoopStart;
+    uint32_t far[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) far[k] = beyond(k, q, fwd);
+    const int near = nearest((open[0] | close[0]) & far[0], (open[1] | close[1]) & far[1],
+                             (open[2] | close[2]) & far[2], (open[3] | close[3]) & far[3], fwd);
+    uint32_t r = kNone;
+    if (near >= 0) {
+      if ((m.E[near] & 15u) != c) {  // the next bracket is the match
+        r = static_cast<uint32_t>(near) | 128u;
+      } else {
+        // Forward: the first ']' that brings the depth below that at q; back:
+        // the last '[' that brings it one above.
+        const uint32_t want = (m.D[q] + (fwd ? 0xFFu : 1u)) & 0xFF;
+        uint32_t hit[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          hit[k] = far[k] & (fwd ? close[k] : open[k]) &
+                   w.ballot([&](uint32_t l) { return m.D[32 * k + l] == want; });
+        const int b = nearest(hit[0], hit[1], hit[2], hit[3], fwd);
+        if (b >= 0) r = static_cast<uint32_t>(b);
+      }
+    }
+    m.M[q] = static_cast<uint16_t>(r);
+    if (r != kNone) m.M[r & 127] = static_cast<uint16_t>(static_cast<uint32_t>(q) | (r & 128));
+    return r;
+  }
+
+  // At a taken ']', in the state named by key (where execution goes on).
+  __host__ __device__ __forceinline__ void visit(int key) {
+    if (key == s_key && st.h0 == s_h0 && (!used1 || st.h1 == s_h1) && st.i < kStepLimit &&
+        (st.mods == s_mods ||
+         !w.any([&](uint32_t l) { return word(m.T, l) != word(m.snap, l); }))) {
+      const uint32_t len = st.i - s_i;
+      const uint32_t k = (kStepLimit - st.i) / len;
+      st.i += k * len;
+      st.n += k * (st.n - s_n);
+      if (st.h1 != s_h1) {
+        st.h1 = (st.h1 + static_cast<int>(k) * (st.h1 - s_h1)) & (kPair - 1);
+        v1 = m.T[st.h1];
+      }
+    }
+    if (++s_lam == s_power) {
+      s_key = key;
+      s_h0 = st.h0;
+      s_h1 = st.h1;
+      s_i = st.i;
+      s_n = st.n;
+      s_mods = st.mods;
+      s_power <<= 1;
+      s_lam = 0;
+      used1 = false;
+      w.sync();
+      w.each([&](uint32_t l) {
+        reinterpret_cast<uint32_t *>(m.snap)[l] = word(m.T, l);
+      });
+      w.sync();
+    }
+  }
+
+  // Compiles the loop from '[' at s to ']' at e, with no brackets between and
+  // no op changed since the decode; false when it has too many micro-ops.
+  __host__ __device__ __forceinline__ bool compile(int s, int e) {
+    le = -1;
+    int k = 0, d0 = 0, d1 = 0, m0 = 0, m1 = 0;
+    uint32_t cmds = 1, last = kNoop, u = 0, first = 0;
+    copies = false;
+    for (int p = s;;) {
+      p = m.E[p] >> 8;
+      const uint32_t op = p < e ? m.E[p] & 15u : static_cast<uint32_t>(kLoopEnd);
+      if (op >= kDec0) {
+        cmds++;
+        if (op <= kInc0) d0 += op == kInc0 ? 1 : -1;
+        else d1 += op == kInc1 ? 1 : -1;
+        last = kNoop;
+        continue;
+      }
+      if (op != kLoopEnd) cmds++;
+      if (op == last) {  // a repeated copy changes nothing more; a run of '+' or '-' adds up
+        if (op <= kMinus) {
+          u += op == kPlus ? 1u << 24 : ~0u << 24;
+          m.P[k - 1] = u;
+        }
+        continue;
+      }
+      if (k == 8) return false;
+      m0 += d0;
+      m1 += d1;
+      const uint32_t act = op == kLoopEnd ? kTest : op == kCopy01 ? kTo1 : op == kCopy10 ? kTo0 : kAdd;
+      u = static_cast<uint32_t>((d0 & (kPair - 1)) | (d1 & (kPair - 1)) << 8) | act << 16 |
+          (op == kPlus ? 1u << 24 : op == kMinus ? ~0u << 24 : 0u);
+      m.P[k] = u;
+      if (k == 0) first = act;
+      k++;
+      if (op == kLoopEnd) break;
+      d0 = d1 = 0;
+      last = op;
+      copies |= act != kAdd;
+      if (kLogic == kLogicSelfmove && op == kCopy10) {
+        d1 = 1;
+        last = kNoop;
+      }
+    }
+    ls = s;
+    le = e;
+    net0 = m0;
+    net1 = m1;
+    lcmds = cmds;
+    const uint32_t moved = static_cast<uint32_t>(m0 | (copies ? m1 : 0)) | kPair;
+    period = static_cast<uint32_t>(kPair >> low32(moved));
+    kind = k == 1 || (k == 2 && first != kAdd)    ? kCopyOne
+           : k == 2 && m0 == 0 && (u & 0x7F) == 0 ? kCount
+                                                  : kGeneric;
+    return true;
+  }
+
+  // The loop changes nothing more and never ends: runs it to the step limit.
+  __host__ __device__ __forceinline__ int run_out() {
+    const uint32_t len = static_cast<uint32_t>(le - ls), k = (kStepLimit - st.i) / len;
+    st.i += k * len;
+    st.n += k * lcmds;
+    const int end = ls + 1 + static_cast<int>(kStepLimit - st.i);
+    for (int p = m.E[ls] >> 8; p < end; p = m.E[p] >> 8) st.n++;
+    st.i = kStepLimit;
+    return kEnd;
+  }
+
+  // The command at hand (the body's left-th that is no move) would write into
+  // the loop's code: leaves the loop, the heads moved, before it.
+  __host__ __device__ __forceinline__ int bail(int left) {
+    if (iters < 2) {
+      hold = backoff;
+      if (backoff < 64) backoff *= 2;
+    } else {
+      backoff = 4;
+    }
+    // Found as compile() counts them.
+    uint32_t last = kNoop;
+    int p = m.E[ls] >> 8;
+    for (; p < le; p = m.E[p] >> 8) {
+      const uint32_t op = m.E[p] & 15;
+      if (op < kDec0 && op != last && --left == 0) break;
+      last = op >= kDec0 || (kLogic == kLogicSelfmove && op == kCopy10)
+                 ? static_cast<uint32_t>(kNoop) : op;
+      st.n++;
+    }
+    st.i += static_cast<uint32_t>(p - 1 - ls);
+    return p - 1;
+  }
+
+  // Runs the compiled loop from its top until it ends, is left or reaches the
+  // step limit.  A whole iteration fits in the limit on entry.  This and the
+  // functions that run commands return the position after which execution
+  // goes on (raw steps through it counted), or kEnd.
+  __host__ __device__ __forceinline__ int loop() {
+    iters = 0;
+    used1 |= copies;
+    const uint32_t len = static_cast<uint32_t>(le - ls);
+    if (kind == kCopyOne) return loop_copy(len);
+    if (kind == kCount && (st.h0 < ls || st.h0 > le)) return loop_count(len);
+    return loop_generic(len);
+  }
+
+  // At most one copy.  Lane j is iteration j: it reads from src + j * ds,
+  // writes to dst + j * dd, and the ']' reads test + j * net0.  Iterations are
+  // cut where one would read what an earlier one of the same batch changed.
+  __host__ __device__ __forceinline__ int loop_copy(uint32_t len) {
+    const uint32_t u = m.P[0], act = (u >> 16) & 3;
+    const bool to1 = act == kTo1;
+    const int a0 = copies ? static_cast<int>(u & 127) : net0;
+    const int a1 = static_cast<int>((u >> 8) & 127);
+    const int ds = act == kTo0 ? net1 : net0, dd = to1 ? net1 : net0;
+    uint32_t most = kWarp;
+    if (copies) {
+      // Iterations that lie apart by so many read what the earlier one wrote.
+      const int x0 = st.h0 + a0, x1 = st.h1 + a1;
+      const int off_s = act == kTo0 ? x1 - x0 : x0 - x1;
+      const int off_t = st.h0 + net0 - (to1 ? x1 : x0);
+      if (dd == net0 && dd == ds && (dd == 1 || dd == -1)) {
+        const uint32_t js = static_cast<uint32_t>(-off_s * dd) & (kPair - 1);
+        const uint32_t jt = static_cast<uint32_t>(-off_t * dd) & (kPair - 1);
+        if (js - 1 < most - 1) most = js;
+        if (jt - 1 < most - 1) most = jt;
+      } else if (dd != 0) {
+        const uint32_t bad = w.ballot([&](uint32_t l) {
+          const int j = static_cast<int>(l);
+          bool b = ((dd * j) & (kPair - 1)) == 0;                      // the same byte written again
+          if (ds == dd) b |= ((off_s + ds * j) & (kPair - 1)) == 0;    // a written byte copied on
+          if (net0 == dd) b |= ((off_t + dd * j) & (kPair - 1)) == 0;  // a written byte tested later
+          if ((ds != dd && ds != 0) || (net0 != dd && net0 != 0)) b = true;
+          return b && j > 0;
+        });
+        if (bad) most = static_cast<uint32_t>(low32(bad));
+      }
+    }
+    uint32_t quiet = 0;
+    while (true) {
+      uint32_t room = kWarp;
+      if (st.i + kWarp * len > kStepLimit) room = (kStepLimit - st.i) / len;
+      const int t0 = st.h0 + net0, s0 = act == kTo0 ? st.h1 + a1 : st.h0 + a0;
+      const int w0 = to1 ? st.h1 + a1 : st.h0 + a0;
+      uint32_t cut = most < room ? most : room;
+      const auto at = w.map([&](uint32_t l) { return (w0 + dd * static_cast<int>(l)) & (kPair - 1); });
+      const auto x = w.map([&](uint32_t l) {
+        return uint32_t(m.T[(s0 + ds * static_cast<int>(l)) & (kPair - 1)]);
+      });
+      const auto y = w.map([&](uint32_t l) { return uint32_t(m.T[at(l)]); });
+      const auto z = w.map([&](uint32_t l) {
+        const int p = (t0 + net0 * static_cast<int>(l)) & (kPair - 1);
+        return copies && p == at(l) ? x(l) : uint32_t(m.T[p]);
+      });
+      uint32_t changed = copies ? w.ballot([&](uint32_t l) { return x(l) != y(l); }) : 0u;
+      if (copies && (changed != 0 || dd == 0)) {
+        if (dd == 0) {
+          // One byte written over and over: cut before an iteration that reads
+          // it; iteration j > 0 finds what j - 1 wrote.
+          if (ds != 0) {
+            const uint32_t self = w.ballot([&](uint32_t l) {
+              return l > 0 && ((s0 + ds * static_cast<int>(l) - w0) & (kPair - 1)) == 0;
+            });
+            if (self && static_cast<uint32_t>(low32(self)) < cut) cut = low32(self);
+          }
+          w.sync();
+          w.each([&](uint32_t l) { m.X[l] = static_cast<uint8_t>(x(l)); });
+          w.sync();
+          changed = (changed & 1) |
+                    w.ballot([&](uint32_t l) { return l > 0 && m.X[l - 1] != x(l); });
+        } else if (net0 == 0) {
+          // One byte tested throughout: cut after the iteration that writes it.
+          const uint32_t hits = w.ballot([&](uint32_t l) { return at(l) == (t0 & (kPair - 1)); });
+          if (hits && static_cast<uint32_t>(low32(hits)) + 1 < cut) cut = low32(hits) + 1;
+        }
+        const uint32_t code = changed == 0 ? 0u : changed & w.ballot([&](uint32_t l) {
+          return static_cast<uint32_t>(at(l) - ls) <= len;
+        });
+        if (code) {
+          // A change of the loop's code is one of its ops.
+          const uint32_t ops = code & w.ballot([&](uint32_t l) {
+            return optab[x(l)] != optab[dd == 0 && l > 0 ? m.X[l - 1] : y(l)];
+          });
+          const uint32_t first = ops ? static_cast<uint32_t>(low32(ops)) : kWarp;
+          if (first < cut) cut = first;
+          if (cut == 0) {
+            st.h0 = (st.h0 + a0) & (kPair - 1);
+            st.h1 = (st.h1 + a1) & (kPair - 1);
+            return bail(1);
+          }
+        }
+      }
+      uint32_t zero = w.ballot([&](uint32_t l) { return (z(l) & kNullMask) == 0; });
+      const uint32_t within = ~0u >> (32 - cut);
+      zero &= within;
+      if (zero) cut = low32(zero) + 1;
+      changed &= zero ? ~0u >> (32 - cut) : within;
+      if (changed) {
+        w.sync();
+        // (One byte: the last iteration's value stays.)
+        const uint32_t ops = w.ballot([&](uint32_t l) {
+          if (dd == 0 ? l + 1 != cut : !((changed >> l) & 1)) return false;
+          m.T[at(l)] = static_cast<uint8_t>(x(l));
+          return optab[x(l)] != optab[y(l)];
+        });
+        w.sync();
+        if (ops) {  // the range of the changed positions, which go from the first lane's by dd
+          const int a = (w0 + dd * low32(ops)) & (kPair - 1), b = a + dd * (high32(ops) - low32(ops));
+          if (b >= 0 && b < kPair) changed_op(a < b ? a : b, a < b ? b : a);
+          else changed_op(0, kPair - 1);
+        }
+        st.mods += popc32(changed);
+        quiet = cut - 1 - high32(changed);
+      } else {
+        quiet += cut;
+      }
+      st.h0 = (st.h0 + net0 * static_cast<int>(cut)) & (kPair - 1);
+      st.h1 = (st.h1 + net1 * static_cast<int>(cut)) & (kPair - 1);
+      st.i += cut * len;
+      st.n += cut * lcmds;
+      iters += cut;
+      if (zero) return le;
+      if (quiet >= period) return run_out();
+      if (st.i + len > kStepLimit) return ls;
+    }
+  }
+
+  // One run of '+' or '-' on the tested byte, outside the loop's code: the
+  // iterations until it is zero (or all that the step limit allows) at once.
+  __host__ __device__ __forceinline__ int loop_count(uint32_t len) {
+    const uint32_t d = m.P[0] >> 24;
+    const uint32_t o = m.T[st.h0];
+    const uint32_t room = (kStepLimit - st.i) / len;
+    uint32_t k = 0;
+    bool found = false;
+    while (k < room && k < 256 && !found) {  // the byte's values repeat after 256
+      const uint32_t zero = w.ballot([&](uint32_t l) {
+        return k + l < room && ((o + (k + l + 1) * d) & kNullMask) == 0;
+      });
+      found = zero != 0;
+      k += found ? low32(zero) + 1 : kWarp;
+    }
+    if (!found) k = room;
+    const uint32_t v = (o + k * d) & 0xFF;
+    if (v != o) write(st.h0, o, v);
+    st.i += k * len;
+    st.n += k * lcmds;
+    st.h1 = (st.h1 + static_cast<int>(k) * net1) & (kPair - 1);
+    return found ? le : ls;
+  }
+
+  // Whether micro-op u changes the op of a byte from o to v, or of one passed on
+  // the way of a run.
+  __host__ __device__ __forceinline__ bool code_changes(uint32_t u, uint32_t o, uint32_t v) const {
+    const bool down = u >> 31, copy = (u >> 16) & 1;
+    const uint32_t r = copy ? 1u : down ? 256 - (u >> 24) : u >> 24;
+    return r > kWarp || w.any([&](uint32_t l) {
+      const uint32_t x = copy ? v : down ? o - l - 1 : o + l + 1;
+      return l < r && optab[x & 0xFF] != optab[o];
+    });
+  }
+
+  // Micro-op by micro-op.  The cycle check (on a snapshot of its own) runs
+  // whenever the heads are back where they were after the first kSettle
+  // iterations.
+  __host__ __device__ __forceinline__ int loop_generic(uint32_t len) {
+    const uint32_t spacing = period < kSettle ? kSettle : period;
+    uint32_t quiet = 0, until = kSettle, since = 0, power = 0;
+    int lo = kPair, hi = -1, from;  // lo..hi: positions written
+    while (true) {
+      uint32_t u = m.P[0];
+      int k = 0;
+      do {
+        st.h0 = (st.h0 + static_cast<int>(u)) & (kPair - 1);
+        st.h1 = (st.h1 + static_cast<int>(u >> 8)) & (kPair - 1);
+        const uint32_t b0 = m.T[st.h0], b1 = m.T[st.h1];
+        const bool copy = (u >> 16) & 1, to1 = (u >> 17) & 1;
+        const uint32_t o = to1 ? b1 : b0;
+        const uint32_t v = copy ? (to1 ? b0 : b1) : (b0 + (u >> 24)) & 0xFF;
+        const int p = to1 ? st.h1 : st.h0;
+        const uint32_t was = u;
+        u = m.P[++k];
+        if (v != o) {
+          if (static_cast<uint32_t>(p - ls) <= len && code_changes(was, o, v)) {
+            if (lo <= hi) changed_op(lo, hi);
+            return bail(k);
+          }
+          m.T[p] = static_cast<uint8_t>(v);
+          st.mods++;
+          lo = p < lo ? p : lo;
+          hi = p > hi ? p : hi;
+          quiet = ~0u;
+        }
+      } while (((u >> 16) & 3) != kTest);
+      st.h0 = (st.h0 + static_cast<int>(u)) & (kPair - 1);
+      st.h1 = (st.h1 + static_cast<int>(u >> 8)) & (kPair - 1);
+      w.sync();
+      st.i += len;
+      st.n += lcmds;
+      from = le;
+      if ((m.T[st.h0] & kNullMask) == 0) break;
+      iters++;
+      if (++quiet >= period) {
+        from = run_out();
+        break;
+      }
+      if (--until == 0) {
+        until = spacing;
+        since += spacing;
+        if (power != 0 && !w.any([&](uint32_t l) { return word(m.T, l) != word(m.top, l); })) {
+          const uint32_t room = (kStepLimit - st.i) / len, skip = room - room % since;
+          st.i += skip * len;
+          st.n += skip * lcmds;
+          st.h1 = (st.h1 + static_cast<int>(skip) * net1) & (kPair - 1);
+        }
+        if (since >= power * spacing) {  // renewed after 1, 2, 4, ... checks
+          power = power ? 2 * power : 1;
+          since = 0;
+          w.each([&](uint32_t l) { reinterpret_cast<uint32_t *>(m.top)[l] = word(m.T, l); });
+        }
+      }
+      from = ls;
+      if (st.i + len > kStepLimit) break;
+    }
+    if (lo <= hi) changed_op(lo, hi);
+    return from;
+  }
+
+  // A bracket at q; back: a ']' was taken (and is no compiled loop's).  kRedo,
+  // with nothing done, when ops must be decoded again first.
+  __host__ __device__ __forceinline__ int bracket(uint32_t c, bool *back) {
+    const bool zero = (v0 & kNullMask) == 0, taken = zero == (c == kLoopStart);
+    const int q = st.q;
+    int from = q;
+    uint32_t mt = kNone;
+    if (kLogic == kLogicJump8) {
+      if (taken) from = c == kLoopStart ? q + 8 : q - 8;
+      *back = from < q;
+      if (from < 0 || from >= kPair) from = kEnd;
+    } else if (c == kLoopStart || taken) {
+      mt = match(q, c);
+      if (mt == kUnknown) return kRedo;
+      if (taken) from = mt == kNone ? kEnd : static_cast<int>(mt & 127);
+    }
+    st.n++;
+    st.i++;
+    if (kLogic == kLogicJump8) return from;
+    if ((mt & 128) != 0 && (c == kLoopEnd || !zero)) {
+      const int b = static_cast<int>(mt & 127), s = c == kLoopStart ? q : b,
+                e = c == kLoopStart ? b : q;
+      if (hold != 0) hold -= taken;
+      else if (((s == ls && e == le) || compile(s, e)) &&
+               st.i + static_cast<uint32_t>(e - s) <= kStepLimit)
+        return loop();
+    }
+    *back = taken && c == kLoopEnd;
+    return from;
+  }
+
+  // A command other than a bracket, at q.
+  __host__ __device__ __forceinline__ void command(uint32_t c) {
+    st.n++;
+    st.i++;
+    if (c >= kDec1) {
+      st.h1 = (st.h1 + (c == kInc1 ? 1 : -1)) & (kPair - 1);
+      v1 = m.T[st.h1];
+    } else if (c >= kDec0) {
+      st.h0 = (st.h0 + (c == kInc0 ? 1 : -1)) & (kPair - 1);
+      v0 = m.T[st.h0];
+    } else {
+      const bool to1 = c == kCopy01;
+      const uint32_t v =
+          (c == kPlus ? v0 + 1 : c == kMinus ? v0 - 1 : c == kCopy10 ? v1 : v0) & 0xFF;
+      const uint32_t o = to1 ? v1 : v0;
+      used1 |= c >= kCopy01;
+      if (v != o) {
+        write(to1 ? st.h1 : st.h0, o, v);
+        if (!to1 || st.h0 == st.h1) v0 = v;
+        if (to1 || st.h0 == st.h1) v1 = v;
+      }
+      if (kLogic == kLogicSelfmove && c == kCopy10) {
+        st.h1 = (st.h1 + 1) & (kPair - 1);
+        v1 = m.T[st.h1];
+      }
+    }
+  }
+
+  // Runs the program in m.T from state s (at a command) to its end; st.n and
+  // raw() are then the op and raw step counts.
+  __host__ __device__ __forceinline__ void run(const BffState &s) {
+    st = s;
+    used1 = true;
+    copies = false;
+    ls = le = s_key = -1;
+    net0 = net1 = 0;
+    lcmds = period = kind = iters = hold = 0;
+    backoff = 4;
+    s_h0 = s_h1 = 0;
+    s_i = s_n = s_mods = s_lam = 0;
+    s_power = 1;
+    dlo = 0;
+    dhi = kPair - 1;  // nothing is decoded yet
+    v0 = m.T[st.h0];
+    v1 = m.T[st.h1];
+    int from = kRedo, next = 0;
+    bool back = false;
+    while (true) {
+      // On to the command after `from` (or st.q once more).
+      if (from == kRedo || (dlo <= next && dhi > from)) {
+        decode();
+        if (from != kRedo) next = m.E[from] >> 8;
+      }
+      if (from != kRedo) {
+        st.i += static_cast<uint32_t>(next - from - 1);
+        st.q = next;
+        if (next >= kPair || st.i >= kStepLimit) return;
+        if (back) {
+          visit(next);
+          if (st.i >= kStepLimit) return;
+        }
+      }
+      const uint32_t en = m.E[st.q], c = en & 15;
+      back = false;
+      if (c > kLoopEnd) {
+        command(c);
+        from = st.q;
+        next = en >> 8;
+      } else {
+        w.sync();
+        from = bracket(c, &back);
+        if (from == kEnd) return;
+        if (from != kRedo) {
+          v0 = m.T[st.h0];
+          v1 = m.T[st.h1];
+          next = m.E[from] >> 8;
+        }
+      }
+    }
+  }
+
+  __host__ __device__ __forceinline__ uint32_t raw() const {
+    return st.i < kStepLimit ? st.i : kStepLimit;
+  }
+};
+
+// The one-shot machine.  Work per step is reduced without changing results:
 //  * a 128-bit mask marks command bytes; runs of no-op bytes are crossed in
 //    one step of the machine: the reference counts each as a step and a skip,
 //    so i and nskip advance by the run length (cut at the step limit; a run
@@ -14,53 +795,13 @@
 //  * '[' / ']' masks (built on the first loop command) let bracket matching
 //    walk only bracket positions;
 //  * masks are patched on writes that change a byte's op;
-//  * exact cycle fast-forward at backward jumps (cycle.cuh): the state is
-//    (pc, heads, tape).  Tape equality with the snapshot is checked on the
-//    positions written since the snapshot only: the first write to a
-//    position saves its snapshot value in a second per-lane area (the stack
-//    area, unused by BFF), so loops whose writes cancel are caught too.
-//    Head drift is allowed: a head that no command used as an address since
-//    the snapshot may differ from the snapshot's.  Control flow depends only
-//    on pc, the used heads and the tape, so the segment since the snapshot
-//    repeats with that head shifted by the same amount each time; k
-//    repetitions advance i by k*P, nskip by k times the segment's skips and
-//    the head by k times its shift (mod 128).
-//
-// Two ways to step, with the same results:
-//  * basic mode (step_basic; the one-shot bff_eval of the per-epoch kernels):
-//    the next command comes from the command mask, its op from the table;
-//  * fast mode (step_lane; the lanes of the pipelined kernel, which provide
-//    a next-command array, LaneNp): one 16-bit entry per position gives the
-//    next command position >= p and its op (entry = q << 4 | op, q = 128 when
-//    none), so a step's fetch and no-op run are one shared-memory load,
-//    issued one step ahead.  The bytes under the two heads are cached in
-//    registers (v0, v1).  Writes that change a byte's op rewrite the entries
-//    of the positions whose next command it is.
-#pragma once
-
-#include "cycle.cuh"
-#include "languages.cuh"
-
-namespace cubff {
-
-enum BffLogic { kLogicScan, kLogicJump8, kLogicSelfmove };
-
+//  * exact cycle fast-forward at backward jumps, as above; tape equality with
+//    the snapshot is checked on the positions written since (the first write
+//    to a position saves its snapshot value in a second per-lane area).
 template <bool kHeads, int kLogic, uint32_t kNullMask>
-struct BffMachine {
+struct BffBasic {
   int pc, h0, h1;
   uint32_t i, nskip, mods;
-  bool fast;          // fast mode: np holds the next-command entries
-  uint32_t v0, v1;    // fast mode: tape[h0], tape[h1]
-  uint32_t nxt;       // fast mode: np entry of pc, loaded one step ahead
-  // Fast mode, loop replay: a loop [ ... ] whose body has no brackets runs
-  // from its op list, one iteration per step, the no-op runs and the step
-  // count of an iteration accounted at its ']'.  Runs of one head move merge into one
-  // op (h +- r), and so do runs of '.' or ',' (a repeat copies a value onto
-  // itself); at most 8 ops of at most 16 commands each.
-  // rpk = S | E << 8 | m << 16 ('[' at S, ']' at E, m < 128 body commands),
-  // plus kScanLoop when the body only moves heads; 0 = not replaying.
-  uint32_t rpk;
-  uint64_t rcls;  // ops: 8 bits each (op | (count - 1) << 4), first in the low bits
   bool have_brk;
   bool used0, used1;  // heads used as addresses since the snapshot
   Mask128 cmd, opn, cls;
@@ -82,10 +823,6 @@ struct BffMachine {
       pc = 0;
     }
     i = nskip = mods = 0;
-    fast = false;
-    v0 = v1 = nxt = 0;
-    rpk = 0;
-    rcls = 0;
     used0 = used1 = false;
     touched = Mask128{0, 0};
     s_pc = -1;
@@ -172,726 +909,9 @@ struct BffMachine {
     }
   }
 
-  // Fast mode: builds the next-command entries and the bracket masks, loads
-  // the head caches and the entry of pc.
-  //
-  // With bracket scanning (all variants but bff8), pc only ever continues
-  // after a command (at q + 1) or starts at the initial pc, so only the
-  // entries at q + 1 of commands q are kept (the initial fetch is computed
-  // here).  bff8's jumps (pc +- 8) land anywhere: it keeps every entry.
-  __host__ __device__ __forceinline__ uint32_t entry_at(const LaneBytes t,
-                                                        const uint8_t *__restrict__ optab,
-                                                        int q) const {
-    return q < kPair ? (uint32_t(q) << 4) | optab[t.get(q)] : uint32_t(kPair) << 4;
-  }
-
-  __host__ __device__ __forceinline__ void enter_fast(const LaneBytes t, const LaneNp np,
-                                                      const uint8_t *__restrict__ optab) {
-    if (kLogic == kLogicJump8) {
-      uint32_t e = uint32_t(kPair) << 4;
-      np.set(kPair, e);
-      for (int p = kPair - 1; p >= 0; p--) {
-        if (mask_test(cmd, p)) e = (uint32_t(p) << 4) | optab[t.get(p)];
-        np.set(p, e);
-      }
-      nxt = np.get(pc);
-    } else {
-      // Commands from the top down: np[q + 1] = entry of the next command
-      // after q; the bracket masks on the way.
-      opn = Mask128{0, 0};
-      cls = Mask128{0, 0};
-      uint32_t e = uint32_t(kPair) << 4;
-      for (int half = 1; half >= 0; half--) {
-        uint64_t w = half ? cmd.hi : cmd.lo;
-        while (w) {
-          const int b = 63 - clz64(w);
-          w &= ~(1ull << b);
-          const int q = 64 * half + b;
-          const uint32_t c = optab[t.get(q)];
-          np.set(q + 1, e);
-          if (c == kLoopStart) mask_assign(opn, q, true);
-          if (c == kLoopEnd) mask_assign(cls, q, true);
-          e = (uint32_t(q) << 4) | c;
-        }
-      }
-      have_brk = true;
-      nxt = entry_at(t, optab, mask_next(cmd, pc));
-    }
-    v0 = t.get(h0);
-    v1 = t.get(h1);
-    fast = true;
-  }
-
-  // write() for fast mode: also rewrites the next-command entries of the
-  // positions after the previous command up to a when a's op changes.
-  // Returns 0 when no entry changed, else 1 + (a was a command): the
-  // prefetched entry may be stale.
-  __host__ __device__ __forceinline__ int write_fast(const LaneBytes t, const LaneBytes snapa,
-                                                      const LaneNp np,
-                                                      const uint8_t *__restrict__ optab, int a,
-                                                      uint32_t o, uint32_t v) {
-    if (v == o) return 0;
-    t.set(a, v);
-    mods++;
-    if (!mask_test(touched, a)) {
-      mask_assign(touched, a, true);
-      snapa.set(a, o);
-    }
-    const uint32_t co = optab[o], cn = optab[v];
-    if (co == cn) return 0;
-    const bool is = cn < kNull, was = co < kNull;
-    mask_assign(opn, a, cn == kLoopStart);
-    mask_assign(cls, a, cn == kLoopEnd);
-    if (!is && !was) return 0;
-    mask_assign(cmd, a, is);
-    if (kLogic == kLogicJump8) {
-      const uint32_t ent = is ? ((uint32_t(a) << 4) | cn) : np.get(a + 1);
-      const int lo = mask_prev(cmd, a - 1) + 1;
-      for (int p = a; p >= lo; p--) np.set(p, ent);
-    } else {
-      // The kept entries: a + 1 (when a becomes a command) and the one after
-      // the previous command, which now leads to a (or past it).
-      uint32_t ent;
-      if (is) {
-        ent = (uint32_t(a) << 4) | cn;
-        if (!was) np.set(a + 1, entry_at(t, optab, mask_next(cmd, a + 1)));
-      } else {
-        ent = np.get(a + 1);
-      }
-      const int pq = mask_prev(cmd, a - 1);
-      if (pq >= 0) np.set(pq + 1, ent);
-    }
-    return 1 + was;
-  }
-
-  __host__ __device__ __forceinline__ bool step_fast(const LaneBytes t, const LaneBytes snapa,
-                                                     const LaneNp np,
-                                                     const uint8_t *__restrict__ optab) {
-    const uint32_t e = nxt;
-    const int q = static_cast<int>(e >> 4);
-    const uint32_t run = static_cast<uint32_t>(q - pc);
-    if (run) {
-      if (i + run >= kStepLimit) {
-        nskip += kStepLimit - i;
-        i = kStepLimit;
-        return true;
-      }
-      i += run;
-      nskip += run;
-      pc = q;
-      if (pc >= kPair) return true;
-    }
-    const uint32_t c = e & 15;
-    int npc = pc + 1;
-    nxt = np.get(npc);  // npc <= kPair: the sentinel entry exists
-    bool back = false;
-    int pe = 0;  // a ']' taken backwards: its position
-    if (c >= kDec0) {
-      if (c <= kInc0) {
-        h0 = (h0 + (c == kInc0 ? 1 : -1)) & (kPair - 1);
-        v0 = t.get(h0);
-      } else {
-        h1 = (h1 + (c == kInc1 ? 1 : -1)) & (kPair - 1);
-        v1 = t.get(h1);
-      }
-    } else if (c >= kPlus) {
-      used0 = true;
-      const bool to1 = c == kCopy01;
-      if (c >= kCopy01) used1 = true;
-      const int a = to1 ? h1 : h0;
-      const uint32_t o = to1 ? v1 : v0;
-      const uint32_t v = (c == kPlus ? v0 + 1 : c == kMinus ? v0 - 1 : to1 ? v0 : v1) & 0xFF;
-      if (to1) v1 = v; else v0 = v;
-      if (h0 == h1) v0 = v1 = v;
-      if (write_fast(t, snapa, np, optab, a, o, v)) nxt = np.get(npc);
-      if (kLogic == kLogicSelfmove && c == kCopy10) {
-        h1 = (h1 + 1) & (kPair - 1);
-        v1 = t.get(h1);
-      }
-    } else if (c == kLoopStart) {
-      used0 = true;
-      if ((v0 & kNullMask) == 0) {
-        if (kLogic == kLogicJump8) {
-          pc += 8;
-        } else {
-          const Mask128 brk{opn.lo | cls.lo, opn.hi | cls.hi};
-          int depth = 1, p = pc + 1;
-          while (true) {
-            const int b = mask_next(brk, p);
-            if (b >= kPair) { pc = kPair; break; }
-            depth += mask_test(opn, b) ? 1 : -1;
-            if (depth == 0) { pc = b; break; }
-            p = b + 1;
-          }
-        }
-        npc = pc + 1;
-        if (npc <= kPair) nxt = np.get(npc);
-      }
-    } else {
-      used0 = true;
-      pe = pc;
-      if ((v0 & kNullMask) != 0) {
-        back = true;
-        if (kLogic == kLogicJump8) {
-          pc -= 8;
-        } else {
-          const Mask128 brk{opn.lo | cls.lo, opn.hi | cls.hi};
-          int depth = 1, p = pc - 1;
-          while (true) {
-            const int b = mask_prev(brk, p);
-            if (b < 0) { pc = -1; break; }
-            depth += mask_test(cls, b) ? 1 : -1;
-            if (depth == 0) { pc = b; break; }
-            p = b - 1;
-          }
-        }
-        npc = pc + 1;
-        if (npc >= 0) nxt = np.get(npc);
-      }
-    }
-    i++;
-    if (pc < 0) return true;
-    pc = npc;
-    if (pc >= kPair || i >= kStepLimit) return true;
-    if (back) {
-      const int g0 = h0, g1 = h1;
-      visit(t, snapa);
-      if (i >= kStepLimit) return true;
-      if (h0 != g0) v0 = t.get(h0);
-      if (h1 != g1) v1 = t.get(h1);
-      if (kLogic != kLogicJump8) enter_replay(np, pc - 1, pe);
-    }
-    return false;
-  }
-
-  // Bits a..b (inclusive) of one 64-bit mask word (none when a > b).
-  __host__ __device__ __forceinline__ static uint64_t word_bits(int a, int b) {
-    return a > b ? 0ull : (~0ull >> (63 - b)) & (~0ull << a);
-  }
-  // Positions strictly between s and e (0 <= s < e <= 127) of mask m.
-  __host__ __device__ __forceinline__ static Mask128 between(const Mask128 &m, int s, int e) {
-    const int lo_end = e - 1 < 63 ? e - 1 : 63;
-    const int hi_start = s + 1 > 64 ? s + 1 : 64;
-    return Mask128{m.lo & word_bits(s + 1, lo_end), m.hi & word_bits(hi_start - 64, e - 1 - 64)};
-  }
-
-  static constexpr uint32_t kScanLoop = 1u << 23;
-  static constexpr uint32_t kCountLoop = 1u << 24;
-  static constexpr uint32_t kFixedTest = 1u << 25;
-  // Copy sweeps (copy_sweep) never apply to bff_selfmove, whose copies move
-  // h1 (they are not a fixed-destination sweep): enter_replay does not flag
-  // them there.
-  static constexpr uint32_t kCopySweep = 1u << 26;
-  static constexpr int kReplayBatch = 8;  // replayed iterations per step call
-
-  // Ops that a run of may merge into one replay op: head moves, copies (a
-  // repeat copies a value onto itself) and '+' / '-' (a run adds its length
-  // to one byte; it runs merged only while that byte is outside the loop's
-  // code, so no op of the loop changes on the way).
-  __host__ __device__ __forceinline__ static bool mergeable(uint32_t c) {
-    return c >= kDec0 || c == kPlus || c == kMinus ||
-           (kLogic != kLogicSelfmove && (c == kCopy01 || c == kCopy10));
-  }
-
-  // After the ']' at e jumped back to the '[' at s: replay the loop when its
-  // body has no brackets and merges into at most 8 ops (the body's ops come
-  // from the next-command entries, which chain from s through the body to e).
-  __host__ __device__ __forceinline__ void enter_replay(const LaneNp np, int s, int e) {
-    const Mask128 body = between(cmd, s, e);
-    const Mask128 brk = between(Mask128{opn.lo | cls.lo, opn.hi | cls.hi}, s, e);
-    if (brk.lo | brk.hi) return;
-    const int m = popc64(body.lo) + popc64(body.hi);
-    // A body of head moves only: its net moves are all that matters.
-    {
-      int q = s, d0 = 0, d1 = 0;
-      bool moves = true;
-      for (int k = 0; k < m && moves; k++) {
-        const uint32_t en = np.get(q + 1);
-        q = static_cast<int>(en >> 4);
-        const uint32_t c = en & 15;
-        moves = c >= kDec0;
-        if (c == kInc0) d0++;
-        else if (c == kDec0) d0--;
-        else if (c == kInc1) d1++;
-        else if (c == kDec1) d1--;
-      }
-      if (moves) {
-        rcls = static_cast<uint64_t>(d0 & (kPair - 1)) | static_cast<uint64_t>(d1 & (kPair - 1)) << 8;
-        rpk = static_cast<uint32_t>(s) | (static_cast<uint32_t>(e) << 8) |
-              (static_cast<uint32_t>(m) << 16) | kScanLoop;
-        return;
-      }
-    }
-    // Otherwise up to 8 ops: a run of head moves becomes its net moves (ops
-    // of at most 16 per head), a run of one copy or of one of '+' / '-' one
-    // op.  The position of each op's first command is kept in the spare
-    // entries of np (np[kPair + 1 + op]) for leaving the replay mid-body.
-    uint64_t ops = 0;
-    int n = 0;              // ops so far
-    uint32_t last = 16;     // value op of the current run (16 = none)
-    uint32_t cnt = 0;
-    int md0 = 0, md1 = 0;   // net moves of the current run of moves
-    int mpos = -1;          // its first command (-1 = no run)
-    bool ok = true;
-    // Appends op c with count r (1..16) whose first command is at p.
-    auto emit = [&](uint32_t c, int r, int p) {
-      if (n == 8 || r > 16) {
-        ok = false;
-        return;
-      }
-      ops |= (static_cast<uint64_t>(c) | static_cast<uint64_t>(r - 1) << 4) << (8 * n);
-      np.set(kPair + 1 + n, static_cast<uint32_t>(p));
-      n++;
-    };
-    // A net move (mod 128, as the smallest |d| <= 64) in ops of at most 16.
-    auto emit_move = [&](int d, uint32_t inc, uint32_t dec) {
-      d &= kPair - 1;
-      if (d > kPair / 2) d -= kPair;
-      while (d != 0 && ok) {
-        const int r = d > 16 ? 16 : d < -16 ? -16 : d;
-        emit(r > 0 ? inc : dec, r > 0 ? r : -r, mpos);
-        d -= r;
-      }
-    };
-    auto flush_moves = [&]() {
-      if (mpos < 0) return;
-      emit_move(md0, kInc0, kDec0);
-      emit_move(md1, kInc1, kDec1);
-      md0 = md1 = 0;
-      mpos = -1;
-    };
-    int q = s;
-    for (int k = 0; k < m && ok; k++) {
-      const uint32_t en = np.get(q + 1);
-      q = static_cast<int>(en >> 4);
-      const uint32_t c = en & 15;
-      if (c >= kDec0) {
-        if (mpos < 0) mpos = q;
-        md0 += c == kInc0 ? 1 : c == kDec0 ? -1 : 0;
-        md1 += c == kInc1 ? 1 : c == kDec1 ? -1 : 0;
-        last = 16;
-        continue;
-      }
-      flush_moves();
-      if (c == last && mergeable(c) && cnt < 16) {
-        cnt++;
-        ops += 1ull << (8 * (n - 1) + 4);
-      } else {
-        emit(c, 1, q);
-        last = c;
-        cnt = 1;
-      }
-    }
-    flush_moves();
-    if (!ok) return;
-    const bool counter = n == 1 && ((ops & 15) == kPlus || (ops & 15) == kMinus);
-    // A body of head moves and '+' / '-' whose h0 moves cancel, none of whose
-    // '+' / '-' hits the byte under h0 at the ']': the ']' tests the same
-    // unchanged byte every iteration.
-    bool fixed = !counter;
-    int off = 0;
-    for (int o2 = 0; o2 < n && fixed; o2++) {
-      const uint32_t c = (ops >> (8 * o2)) & 15;
-      const int r = static_cast<int>((ops >> (8 * o2 + 4)) & 15) + 1;
-      if (c == kInc0) off += r;
-      else if (c == kDec0) off -= r;
-      else if (c == kPlus || c == kMinus) fixed = (off & (kPair - 1)) != 0;
-      else if (c != kInc1 && c != kDec1) fixed = false;
-    }
-    fixed = fixed && (off & (kPair - 1)) == 0;
-    // A body of head moves and at most two copies of one direction, all
-    // writing the same byte (the destination head is at the same offset at
-    // each copy and has no net move), whose source head sweeps.  A copy of
-    // the other direction right after a copy writes back the byte it just
-    // read: it changes nothing.
-    bool sweep = !counter && !fixed;
-    if (kLogic != kLogicSelfmove) {  // (bff_selfmove: see kCopySweep)
-      int o0 = 0, o1 = 0, wo = 0, nc = 0;
-      uint32_t dir = 16, prev = 16;
-      for (int o2 = 0; o2 < n && sweep; o2++) {
-        const uint32_t c = (ops >> (8 * o2)) & 15;
-        const int r = static_cast<int>((ops >> (8 * o2 + 4)) & 15) + 1;
-        if (c == kInc0) o0 += r;
-        else if (c == kDec0) o0 -= r;
-        else if (c == kInc1) o1 += r;
-        else if (c == kDec1) o1 -= r;
-        else if (c != kCopy01 && c != kCopy10) sweep = false;
-        else if (dir == 16 || c == dir) {
-          const int d = (c == kCopy01 ? o1 : o0) & (kPair - 1);
-          sweep = nc < 2 && (nc == 0 || d == wo);
-          dir = c;
-          wo = d;
-          nc++;
-        } else {
-          sweep = prev == dir;
-        }
-        prev = c;
-      }
-      sweep = sweep && nc > 0 && ((dir == kCopy01 ? o1 : o0) & (kPair - 1)) == 0 &&
-              ((dir == kCopy01 ? o0 : o1) & (kPair - 1)) != 0;
-    } else {
-      sweep = false;
-    }
-    rcls = ops;
-    rpk = static_cast<uint32_t>(s) | (static_cast<uint32_t>(e) << 8) |
-          (static_cast<uint32_t>(m) << 16) | (counter ? kCountLoop : 0u) |
-          (fixed ? kFixedTest : 0u) | (sweep ? kCopySweep : 0u);
-  }
-
-  // A loop of kFixedTest whose ']' was taken once takes it every time: it
-  // runs until the step limit.  Its bytes change by the same amounts every
-  // iteration (each '+' / '-' hits a byte at a fixed offset from h0), so all
-  // the whole iterations the limit allows are taken at once: each of those
-  // bytes gains k times its change per iteration, h1 drifts by k times its
-  // net move.  Returns 1 when the program ended, 0 when the loop was taken
-  // over, -1 when a byte it changes lies in the loop's code (those steps must
-  // stay exact, one by one).
-  __host__ __device__ __forceinline__ int fixed_loop(const LaneBytes t, const LaneBytes snapa,
-                                                     const LaneNp np,
-                                                     const uint8_t *__restrict__ optab, int s,
-                                                     int e, int m, uint32_t len) {
-    int off = 0;
-    for (uint64_t w = rcls; w; w >>= 8) {
-      const uint32_t c = w & 15;
-      const int r = static_cast<int>((w >> 4) & 15) + 1;
-      if (c == kInc0) off += r;
-      else if (c == kDec0) off -= r;
-      else if (c == kPlus || c == kMinus) {
-        const int a = (h0 + off) & (kPair - 1);
-        if (a >= s && a <= e) return -1;
-      }
-    }
-    const uint32_t k = (kStepLimit - i) / len;  // whole iterations left, >= 1
-    int d1 = 0;
-    off = 0;
-    for (uint64_t w = rcls; w; w >>= 8) {
-      const uint32_t c = w & 15;
-      const int r = static_cast<int>((w >> 4) & 15) + 1;
-      if (c == kInc0) off += r;
-      else if (c == kDec0) off -= r;
-      else if (c == kInc1) d1 += r;
-      else if (c == kDec1) d1 -= r;
-      else {
-        const int a = (h0 + off) & (kPair - 1);
-        const uint32_t o = t.get(a);
-        const uint32_t v = (o + k * static_cast<uint32_t>(c == kPlus ? r : -r)) & 0xFF;
-        write_fast(t, snapa, np, optab, a, o, v);
-      }
-    }
-    used0 = true;
-    h1 = (h1 + static_cast<int>(k) * d1) & (kPair - 1);
-    v0 = t.get(h0);
-    v1 = t.get(h1);
-    i += k * len;
-    nskip += k * (len - 1 - static_cast<uint32_t>(m));
-    pc = s + 1;
-    return i >= kStepLimit ? 1 : 0;
-  }
-
-  // A loop whose body is one run of '+' or '-' on the byte under h0 (outside
-  // the loop's code) counts that byte: each iteration adds d, and the ']'
-  // leaves once the byte is zero (under the null mask).  The iterations until
-  // then (all the step limit allows when it never is) are taken at once, the
-  // byte written once.  Returns 1 when the program ended, 0 otherwise.
-  __host__ __device__ __forceinline__ int count_loop(const LaneBytes t, const LaneBytes snapa,
-                                                     const LaneNp np,
-                                                     const uint8_t *__restrict__ optab, int s,
-                                                     int e, int m, uint32_t len) {
-    const int r = static_cast<int>((rcls >> 4) & 15) + 1;
-    const uint32_t d = static_cast<uint32_t>((rcls & 15) == kPlus ? r : -r);
-    const uint32_t lim = (kStepLimit - i) / len;  // whole iterations left, >= 1
-    const uint32_t kmax = lim < 256 ? lim : 256;  // the byte's values repeat after 256
-    uint32_t k = 1;
-    bool found = false;
-    for (; k <= kmax; k++) {
-      if (((v0 + k * d) & kNullMask) == 0) {
-        found = true;
-        break;
-      }
-    }
-    if (!found) k = lim;
-    const uint32_t v = (v0 + k * d) & 0xFF;
-    used0 = true;
-    write_fast(t, snapa, np, optab, h0, v0, v);
-    v0 = v;
-    if (h0 == h1) v1 = v;
-    i += k * len;
-    nskip += k * (len - 1 - static_cast<uint32_t>(m));
-    if (found) {  // the k-th ']' falls through
-      rpk = 0;
-      pc = e + 1;
-      if (pc >= kPair || i >= kStepLimit) return 1;
-      nxt = np.get(pc);
-      return 0;
-    }
-    pc = s + 1;
-    return i >= kStepLimit ? 1 : 0;
-  }
-
-  // A loop whose body only moves heads changes no byte, so its iterations
-  // differ only in the heads: each moves h0 by d0 and h1 by d1, and the ']'
-  // tests the byte under the new h0.  The iterations until that byte is a
-  // zero (all of them the step limit allows, when no position reachable by
-  // h0 holds one) are taken at once.  Returns 1 when the program ended, 0
-  // when the loop was taken over, -1 when it does not apply (d0 = 0 mod 128:
-  // the test never changes).
-  __host__ __device__ __forceinline__ int scan_loop(const LaneBytes t, const LaneNp np, int s,
-                                                    int e, int m, uint32_t len) {
-    const int d0 = static_cast<int>(rcls & (kPair - 1));         // net moves, mod 128
-    const int d1 = static_cast<int>((rcls >> 8) & (kPair - 1));
-    if ((d0 & (kPair - 1)) == 0) return -1;
-    const uint32_t lim = (kStepLimit - i) / len;  // whole iterations left, >= 1
-    const uint32_t kmax = lim < kPair ? lim : kPair;
-    uint32_t k = 1;
-    bool found = false;
-    for (; k <= kmax; k++) {
-      if ((t.get((h0 + static_cast<int>(k) * d0) & (kPair - 1)) & kNullMask) == 0) {
-        found = true;
-        break;
-      }
-    }
-    // No zero among the positions h0 reaches (all within kPair iterations):
-    // the loop runs until the step limit.
-    if (!found) k = lim;
-    h0 = (h0 + static_cast<int>(k) * d0) & (kPair - 1);
-    h1 = (h1 + static_cast<int>(k) * d1) & (kPair - 1);
-    v0 = t.get(h0);
-    v1 = t.get(h1);
-    i += k * len;
-    nskip += k * (len - 1 - static_cast<uint32_t>(m));
-    used0 = true;
-    if (found) {  // the k-th ']' falls through
-      rpk = 0;
-      pc = e + 1;
-      if (pc >= kPair || i >= kStepLimit) return 1;
-      nxt = np.get(pc);
-      return 0;
-    }
-    pc = s + 1;
-    return i >= kStepLimit ? 1 : 0;
-  }
-
-  // A loop of kCopySweep: every iteration writes one byte w with bytes that
-  // the sweeping source head reads.  As only w changes, the iterations are
-  // followed on positions alone: a copy reads the byte as it was, or w's
-  // value where it reads w (the value last copied), and the ']' tests the
-  // byte under h0 the same way.  From iteration 129 on, the positions and w's
-  // value repeat those of 128 iterations earlier (the heads move by the same
-  // amount mod 128 each iteration): 257 iterations without a zero test mean
-  // none ever comes, and whole periods of 128 are skipped.  w is then written
-  // once, with its final value.  Returns as scan_loop does; -1 (nothing done)
-  // when w lies in the loop's own code.
-  __host__ __device__ __forceinline__ int copy_sweep(const LaneBytes t, const LaneBytes snapa,
-                                                     const LaneNp np,
-                                                     const uint8_t *__restrict__ optab, int s,
-                                                     int e, int m, uint32_t len) {
-    int o0 = 0, o1 = 0, sa = 0, sb = 0, wo = 0, nc = 0;
-    uint32_t dir = 16;
-    for (uint64_t ops = rcls; ops != 0; ops >>= 8) {
-      const uint32_t c = ops & 15;
-      const int r = static_cast<int>((ops >> 4) & 15) + 1;
-      if (c == kInc0) o0 += r;
-      else if (c == kDec0) o0 -= r;
-      else if (c == kInc1) o1 += r;
-      else if (c == kDec1) o1 -= r;
-      else if (dir == 16 || c == dir) {  // (a copy of the other direction changes nothing)
-        dir = c;
-        if (nc == 0) sa = c == kCopy01 ? o0 : o1;
-        else sb = c == kCopy01 ? o0 : o1;
-        wo = c == kCopy01 ? o1 : o0;
-        nc++;
-      }
-    }
-    const bool to1 = dir == kCopy01;
-    const int w = ((to1 ? h1 : h0) + wo) & (kPair - 1);
-    if (w >= s && w <= e) return -1;
-    const int ds = to1 ? o0 : o1;  // the source head's net move
-    const uint32_t lim = (kStepLimit - i) / len;  // whole iterations left, >= 1
-    const uint32_t w_old = t.get(w);
-    uint32_t cur = w_old, k = 0;
-    bool found = false;
-    int pa = (to1 ? h0 : h1) + sa, pb = (to1 ? h0 : h1) + sb, pt = h0 + o0;
-    while (k < lim) {
-      if (k == 257) {
-        k += (lim - k) / kPair * kPair;
-        if (k >= lim) break;
-      }
-      const int a = pa & (kPair - 1);
-      if (a != w) cur = t.get(a);
-      if (nc == 2) {
-        const int b = pb & (kPair - 1);
-        if (b != w) cur = t.get(b);
-      }
-      const int tp = pt & (kPair - 1);
-      const uint32_t tv = tp == w ? cur : t.get(tp);
-      k++;
-      if ((tv & kNullMask) == 0) {
-        found = true;
-        break;
-      }
-      pa += ds;
-      pb += ds;
-      pt += o0;
-    }
-    h0 = (h0 + static_cast<int>(k) * o0) & (kPair - 1);
-    h1 = (h1 + static_cast<int>(k) * o1) & (kPair - 1);
-    i += k * len;
-    nskip += k * (len - 1 - static_cast<uint32_t>(m));
-    used0 = used1 = true;
-    write_fast(t, snapa, np, optab, w, w_old, cur);
-    v0 = t.get(h0);
-    v1 = t.get(h1);
-    if (found) {  // the k-th ']' falls through
-      rpk = 0;
-      pc = e + 1;
-      if (pc >= kPair || i >= kStepLimit) return 1;
-      nxt = np.get(pc);
-      return 0;
-    }
-    pc = s + 1;
-    return i >= kStepLimit ? 1 : 0;
-  }
-
-  // One step of a replayed loop: the next body command, or the closing ']'.
-  __host__ __device__ __forceinline__ bool step_replay(const LaneBytes t, const LaneBytes snapa,
-                                                       const LaneNp np,
-                                                       const uint8_t *__restrict__ optab) {
-    const int s = rpk & 0xFF, e = (rpk >> 8) & 0xFF, m = (rpk >> 16) & 0x7F;
-    const uint32_t len = static_cast<uint32_t>(e - s);  // raw steps of an iteration
-    if (i + len > kStepLimit) {
-      // Not a whole iteration left: continue step by step (no step taken here).
-      rpk = 0;
-      pc = s + 1;
-      nxt = np.get(pc);
-      return false;
-    }
-    if (rpk & kScanLoop) {
-      const int r = scan_loop(t, np, s, e, m, len);
-      if (r >= 0) return r == 1;
-    }
-    if ((rpk & kCountLoop) && (h0 < s || h0 > e)) return count_loop(t, snapa, np, optab, s, e, m, len) == 1;
-    if (rpk & kFixedTest) {
-      const int r = fixed_loop(t, snapa, np, optab, s, e, m, len);
-      if (r >= 0) return r == 1;
-    }
-    if (rpk & kCopySweep) {
-      const int r = copy_sweep(t, snapa, np, optab, s, e, m, len);
-      if (r >= 0) return r == 1;
-    }
-    // Up to kReplayBatch iterations.
-    for (int it = 0; it < kReplayBatch; it++) {
-      if (it > 0 && i + len > kStepLimit) {
-        rpk = 0;
-        pc = s + 1;
-        nxt = np.get(pc);
-        return false;
-      }
-      if (rpk & kScanLoop) {
-        // h0 returns to itself each iteration: the iteration is its net moves.
-        const int d1 = static_cast<int>((rcls >> 8) & (kPair - 1));
-        if (d1) {
-          h1 = (h1 + d1) & (kPair - 1);
-          v1 = t.get(h1);
-        }
-      }
-      // The body's ops.
-      int j = 0;
-      for (uint64_t ops = (rpk & kScanLoop) ? 0 : rcls; ops != 0; ops >>= 8, j++) {
-        const uint32_t c = ops & 15;
-        const int r = static_cast<int>((ops >> 4) & 15) + 1;  // commands merged into this op
-        if (c >= kDec0) {
-          if (c <= kInc0) {
-            h0 = (h0 + (c == kInc0 ? r : -r)) & (kPair - 1);
-            v0 = t.get(h0);
-          } else {
-            h1 = (h1 + (c == kInc1 ? r : -r)) & (kPair - 1);
-            v1 = t.get(h1);
-          }
-          continue;
-        }
-        if (r > 1 && c <= kMinus && h0 >= s && h0 <= e) {
-          // A run of '+' / '-' on a byte of the loop's own code: leave the
-          // replay before its first command (body command k) and step it.
-          const int p = static_cast<int>(np.get(kPair + 1 + j));
-          const Mask128 before = between(cmd, s, p);  // the body's commands before p
-          const int k = popc64(before.lo) + popc64(before.hi);
-          i += static_cast<uint32_t>(p - 1 - s);
-          nskip += static_cast<uint32_t>(p - 1 - s - k);
-          rpk = 0;
-          pc = p;
-          nxt = entry_at(t, optab, p);
-          return false;
-        }
-        used0 = true;
-        const bool to1 = c == kCopy01;
-        if (c >= kCopy01) used1 = true;
-        const int a = to1 ? h1 : h0;
-        const uint32_t o = to1 ? v1 : v0;
-        const uint32_t v = (c == kPlus ? v0 + r : c == kMinus ? v0 - r : to1 ? v0 : v1) & 0xFF;
-        if (to1) v1 = v; else v0 = v;
-        if (h0 == h1) v0 = v1 = v;
-        const int w = write_fast(t, snapa, np, optab, a, o, v);
-        if (kLogic == kLogicSelfmove && c == kCopy10) {
-          h1 = (h1 + 1) & (kPair - 1);
-          v1 = t.get(h1);
-        }
-        if (w && a >= s && a <= e) {
-          // The loop changed its own code: stop replaying after this command
-          // (the first of its op, at p; a repeat writes nothing).  The body's
-          // commands before p are counted as they were (a's bit as before the
-          // write).
-          const int p = static_cast<int>(np.get(kPair + 1 + j));
-          Mask128 before = between(cmd, s, p);
-          if (a > s && a < p) mask_assign(before, a, w == 2);
-          const int k = popc64(before.lo) + popc64(before.hi);  // commands before p
-          i += static_cast<uint32_t>(p - s);
-          nskip += static_cast<uint32_t>(p - s - (k + 1));
-          rpk = 0;
-          pc = p + 1;
-          nxt = np.get(pc);
-          return false;
-        }
-      }
-      // The ']' at e: the iteration's raw steps and no-ops, then its test.
-      i += len;
-      nskip += len - 1 - m;
-      used0 = true;
-      if ((v0 & kNullMask) == 0) {
-        rpk = 0;
-        pc = e + 1;
-        if (pc >= kPair || i >= kStepLimit) return true;
-        nxt = np.get(pc);
-        return false;
-      }
-      pc = s + 1;
-      if (i >= kStepLimit) return true;
-      // The cycle check runs on every kReplayBatch-th iteration only: states
-      // sampled at a fixed stride repeat when the loop does, and a repeat found
-      // on the samples is a repeat of the loop.
-      if (it == kReplayBatch - 1) {
-        const int g0 = h0, g1 = h1;
-        visit(t, snapa);
-        if (i >= kStepLimit) return true;
-        if (h0 != g0) v0 = t.get(h0);
-        if (h1 != g1) v1 = t.get(h1);
-      }
-    }
-    return false;
-  }
-
-  // Fast mode only (the pipelined kernel): the first step builds the
-  // next-command entries.
-  __host__ __device__ __forceinline__ bool step_lane(const LaneBytes t, const LaneBytes snapa,
-                                                     const LaneNp np,
-                                                     const uint8_t *__restrict__ optab) {
-    if (!fast) enter_fast(t, np, optab);
-    if (rpk) return step_replay(t, snapa, np, optab);
-    return step_fast(t, snapa, np, optab);
-  }
-
-  // Basic mode: a run of no-ops (if any) and then one command.  Returns true
+  // A run of no-ops (if any) and then one command.  Returns true
   // when the program has ended; the op count is then i - nskip.
-  __host__ __device__ __forceinline__ bool step_basic(const LaneBytes t, const LaneBytes snapa,
+  __host__ __device__ __forceinline__ bool step(const LaneBytes t, const LaneBytes snapa,
                                                       const uint8_t *__restrict__ optab) {
     const int q = mask_next(cmd, pc);
     const uint32_t run = static_cast<uint32_t>(q - pc);
@@ -994,9 +1014,9 @@ template <bool kHeads, int kLogic, uint32_t kNullMask>
 __host__ __device__ __forceinline__ uint32_t bff_eval(const LaneBytes t, const LaneBytes snapa,
                                                       const uint8_t *__restrict__ optab,
                                                       uint32_t *raw) {
-  BffMachine<kHeads, kLogic, kNullMask> m;
+  BffBasic<kHeads, kLogic, kNullMask> m;
   m.begin(t, bff_command_mask(t, optab));
-  while (!m.step_basic(t, snapa, optab)) {
+  while (!m.step(t, snapa, optab)) {
   }
   *raw = m.raw();
   return m.ops();

@@ -85,32 +85,33 @@ struct LaneBytes {
   }
 };
 
-// One thread's array of kNpEntries 16-bit entries (the BFF next-command
-// array, bff.cuh: kPair + 1 entries, then kNpSpare entries of loop-replay
-// state).  Entry p of thread tid sits at element p * 128 + tid of a block of
-// 128 threads: a warp's 32 lanes read 64 consecutive bytes for any common p.
-// Per block of 128 threads: kNpBytes.
-constexpr int kNpSpare = 8;
-constexpr int kNpEntries = kPair + 1 + kNpSpare;
-constexpr int kNpBytes = kNpEntries * 128 * 2;
+// The tapes of `stride` lanes of a warp as interleaved words: byte p of lane l
+// sits at (p / 4 * stride + l) * 4 + p % 4 of a block of stride * 128 bytes, so a
+// tape is staged and written back a word at a time.
+template <uint32_t stride>
+struct LaneWords {
+  uint8_t *s;     // the block, 4-byte aligned
+  uint32_t lane;
+  __device__ __forceinline__ uint32_t get(int p) const { return s[at(p)]; }
+  __device__ __forceinline__ void set(int p, uint32_t v) const {
+    s[at(p)] = static_cast<uint8_t>(v);
+  }
+  __device__ __forceinline__ uint32_t at(int p) const {
+    const uint32_t x = static_cast<uint32_t>(p) & (kPair - 1);
+    return ((x >> 2) * stride + lane) * 4 + (x & 3);
+  }
+  __device__ __forceinline__ uint32_t &word(uint32_t w) const {
+    return reinterpret_cast<uint32_t *>(s)[w * stride + lane];
+  }
+};
 
-// Entries are clamped to the last one (kNpEntries - 1) for the same reason:
-// the array never reaches past its thread's column.
+// A per-thread array that the interpreters' common interface passes along
+// (kNpBytes per 128 threads); none uses it any more.
+constexpr int kNpEntries = kPair + 1;
+constexpr int kNpBytes = kNpEntries * 128 * 2;
 struct LaneNp {
-  uint16_t *s;    // nullptr: no array (the interpreter stays in its basic mode)
-  uint32_t base;  // tid within the 128-thread block
-  __host__ __device__ __forceinline__ static uint32_t clamp(int p) {
-    const uint32_t q = static_cast<uint32_t>(p);
-    return q < kNpEntries - 1 ? q : kNpEntries - 1;
-  }
-  __host__ __device__ __forceinline__ uint32_t get(int p) const {
-    CUBFF_CHECK_POS(2, p, kNpEntries - 1);
-    return s[base + (clamp(p) << 7)];
-  }
-  __host__ __device__ __forceinline__ void set(int p, uint32_t v) const {
-    CUBFF_CHECK_POS(3, p, kNpEntries - 1);
-    s[base + (clamp(p) << 7)] = static_cast<uint16_t>(v);
-  }
+  uint16_t *s;
+  uint32_t base;
 };
 
 }  // namespace cubff

@@ -39,37 +39,76 @@ __host__ __device__ __forceinline__ uint32_t evaluate(const LaneBytes t, const L
   else return rsubleq4_eval(t, stk, raw);
 }
 
-// A resumable interpreter of language L behind one interface (used by the
-// lane-level pipeline): begin() on a staged tape, step() until it returns
-// true, then ops() / raw().  cmd_mask (BFF family only) marks command bytes.
+// The two machines that run a BFF program in turn: on a lane, then on a warp.
 template <int L>
+struct BffMachines {
+  static constexpr int kLogic = (L == kBff8 || L == kBff8Noheads)
+                                    ? kLogicJump8
+                                    : (L == kBffSelfmove ? kLogicSelfmove : kLogicScan);
+  static constexpr uint32_t kNullMask = L == kBffNoheads4bit ? 0x0Fu : 0xFFu;
+  using Lane = BffLane<(L == kBff || L == kBffPerm || L == kBff8 || L == kBffSelfmove), kLogic,
+                       kNullMask>;
+  template <class W>
+  using Warp = BffWarp<W, kLogic, kNullMask>;
+};
+
+// A resumable Forth or SUBLEQ interpreter of language L behind one interface:
+// begin() on a staged tape, step() until it returns true, then ops() / raw().
+template <int L, bool kBff = (L <= kBffSelfmove)>
 struct LaneMachine {
-  using Machine = std::conditional_t<
-      (L <= kBffSelfmove),
-      BffMachine<(L == kBff || L == kBffPerm || L == kBff8 || L == kBffSelfmove),
-                 (L == kBff8 || L == kBff8Noheads)
-                     ? kLogicJump8
-                     : (L == kBffSelfmove ? kLogicSelfmove : kLogicScan),
-                 (L == kBffNoheads4bit ? 0x0Fu : 0xFFu)>,
+  using Machine =
       std::conditional_t<LangTraits<L>::kForthFamily, ForthMachine<(L == kForthtrivialReset)>,
-                         SubleqMachine<(L == kRsubleq4)>>>;
+                         SubleqMachine<(L == kRsubleq4)>>;
   Machine m;
 
-  __host__ __device__ __forceinline__ void begin(const LaneBytes t, Mask128 cmd_mask) {
-    if constexpr (L <= kBffSelfmove) m.begin(t, cmd_mask);
-    else m.begin();
-  }
-  // np: the BFF next-command array (fast mode), ignored by the other families.
+  __host__ __device__ __forceinline__ void begin(const LaneBytes, Mask128) { m.begin(); }
   __host__ __device__ __forceinline__ bool step(const LaneBytes t, const LaneBytes stk,
-                                                const LaneNp np,
+                                                const LaneNp,
                                                 const uint8_t *__restrict__ optab) {
-    if constexpr (L <= kBffSelfmove) return m.step_lane(t, stk, np, optab);
-    else if constexpr (LangTraits<L>::kForthFamily) return m.step(t, stk, optab);
+    if constexpr (LangTraits<L>::kForthFamily) return m.step(t, stk, optab);
     else return m.step(t, stk);
   }
   __host__ __device__ __forceinline__ uint32_t ops() const { return m.ops(); }
   __host__ __device__ __forceinline__ uint32_t raw() const { return m.raw(); }
   __host__ __device__ __forceinline__ uint32_t mods() const { return m.mods; }
+};
+
+// The same interface over the BFF machines, on the host: a step of the lane's,
+// or all of the warp's.
+template <int L>
+struct LaneMachine<L, true> {
+  typename BffMachines<L>::Lane lane;
+  Mask128 cmd;
+  bool begun;
+  uint32_t n, i;
+
+  void begin(const LaneBytes, Mask128 cmd_mask) {
+    cmd = cmd_mask;
+    begun = false;
+    n = i = 0;
+  }
+  bool step(const LaneBytes t, const LaneBytes, const LaneNp, const uint8_t *optab) {
+    using Lane = typename BffMachines<L>::Lane;
+    if (!begun) lane.begin(t, cmd, optab);
+    else lane.step(t, optab);
+    begun = true;
+    if (lane.status == Lane::kJumps) lane.resolve(t, optab);
+    n = lane.st.n;
+    i = lane.st.i;
+    if (lane.status == Lane::kJumps) {
+      BffMem mem;
+      for (int p = 0; p < kPair; p++) mem.T[p] = static_cast<uint8_t>(t.get(p));
+      typename BffMachines<L>::template Warp<HostWarp> warp(HostWarp{}, mem, optab);
+      warp.run(lane.st);
+      for (int p = 0; p < kPair; p++) t.set(p, mem.T[p]);
+      n = warp.st.n;
+      i = warp.raw();
+      return true;
+    }
+    return lane.status == Lane::kEnds;
+  }
+  uint32_t ops() const { return n; }
+  uint32_t raw() const { return i; }
 };
 
 }  // namespace cubff

@@ -82,12 +82,15 @@ constexpr int kCountSlots = kPipeCountSlots;  // per-epoch counter slots (spread
 // other languages run in launches of their own, on other streams).
 //
 // No global access is consumed in the iteration that issues it where that
-// can be avoided: queue entries, shuffle indices and gathers land in
-// registers read back in a later iteration.  Lane states:
-//   idle -> slot (wait for the entry) -> index -> stage -> run -> notify -> idle
+// can be avoided: queue entries and shuffle indices land in registers read
+// back in a later iteration.  Lane states:
+//   idle -> slot (wait for the entry) -> index -> [stage ->] run [-> long]
+//        -> notify -> idle
 // and `exhausted` once a claim falls past the queue's last task.
 //
-// Launch-shape knobs (PipeTuning, chosen by the host):
+// How a warp runs its pairs depends on the language family (LaneServer,
+// BffServer).  Launch-shape knobs (PipeTuning, chosen by the host; the BFF
+// family runs a pair to its end and uses only the grid size):
 //  * steps_per_visit: interpreter steps a running lane takes per iteration of
 //    its warp after its first (an iteration lasts as long as its busiest
 //    lane, so a lane given more steps holds its warp-mates, and the pairs
@@ -117,16 +120,24 @@ __device__ __forceinline__ void st_release_u32(uint32_t *p, uint32_t v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-enum : uint32_t { kIdle, kSlot, kIndex, kStage, kRun, kNotify, kExhausted };
+enum : uint32_t { kIdle, kSlot, kIndex, kStage, kRun, kLong, kNotify, kExhausted };
 
-// Per-lane state that does not depend on the language.
+// Per-lane state of a held queue slot and its pair.
 struct Lane {
-  uint32_t state, slot, task, e, k, p1, p2, qv, poll_gap, poll_in, err, j1, j2, c1, c2, visits;
+  uint32_t state, slot, task, e, k, p1, p2, qv, poll_gap, poll_in, err, j1, j2, c1, c2;
   int si;  // soup index of the task
   uint64_t qp, t_wait;
   bool dirty, evaluated, has_next;
-  uint4 g[8];
-  uint4 mm;
+
+  __device__ __forceinline__ void begin() {
+    state = kIdle;
+    slot = task = e = k = p1 = p2 = qv = 0;
+    poll_gap = 1;
+    poll_in = err = j1 = j2 = c1 = c2 = 0;
+    si = 0;
+    qp = t_wait = 0;
+    dirty = evaluated = has_next = false;
+  }
 };
 
 // What a warp needs of the launch: the soup descriptors (in shared memory)
@@ -156,199 +167,157 @@ __device__ __forceinline__ int soup_of_slot(const PipeSoup *soups, int lo, int h
   return lo;
 }
 
-// One iteration of a warp serving language L.  Returns true if a lane made
-// progress.
-template <int L>
-__device__ __forceinline__ bool iterate(const PipeCtx &b, const PipeQueue &q, Lane &ln,
-                                        LaneMachine<L> &m, const LaneBytes t, const LaneBytes stk,
-                                        const LaneNp np, const uint8_t *__restrict__ optab,
-                                        const uint8_t *__restrict__ cmdflag, uint32_t lane,
-                                        uint32_t slot_ctr) {
-  constexpr bool kBffFam = (L <= kBffSelfmove);
+// Claims the next queue slots for the lanes of mask `idle` (warp-uniform,
+// non-zero).
+__device__ __forceinline__ void claim(const PipeCtx &b, const PipeQueue &q, Lane &ln,
+                                      uint32_t idle, uint32_t lane) {
   const uint32_t lt_mask = (1u << lane) - 1;
   const int s_lo = static_cast<int>(q.first_soup), s_hi = static_cast<int>(q.first_soup + q.n_soups);
-
-  // 1. Bulk claim of queue slots by idle lanes.
-  const uint32_t idle = __ballot_sync(0xffffffffu, ln.state == kIdle);
-  const uint32_t busy = __ballot_sync(0xffffffffu, ln.state != kIdle && ln.state != kExhausted);
-  const uint32_t lng = __ballot_sync(0xffffffffu, ln.state == kRun && ln.visits >= b.tune.long_visits);
-  if (idle && (busy == 0 || (lng == 0 && __popc(idle) >= b.tune.claim_min))) {
-    const int leader = __ffs(idle) - 1;
-    uint32_t base = 0;
-    if (lane == static_cast<uint32_t>(leader)) base = atomicAdd(q.ctl, __popc(idle));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (ln.state == kIdle) {
-      ln.slot = base + __popc(idle & lt_mask);
-      if (ln.slot >= q.total) {
-        ln.state = kExhausted;
-      } else if (ln.slot < q.initial) {  // a first-epoch pair: ready
-        ln.si = soup_of_slot(b.soups, s_lo, s_hi, ln.slot);
-        const PipeSoup &sp = b.soups[ln.si];
-        ln.task = sp.task_base + (ln.slot - sp.init_base);
-        ln.state = kIndex;
-        ln.qp = *reinterpret_cast<const unsigned long long *>(sp.perm + 2 * uint64_t(ln.slot - sp.init_base));
-      } else {
-        ln.state = kSlot;
-        ln.qv = ld_relaxed(q.queue + (ln.slot - q.initial));
-        ln.poll_gap = 1;
-        ln.poll_in = 0;
-        ln.t_wait = 0;
-      }
-    }
-  }
-  bool progressed = false;
-
-  if (ln.state == kSlot) {
-    // 2. Waiting for the claimed slot's entry (polled in an earlier iteration).
-    if (ln.qv != 0 && ln.qv - 1 >= q.total) {
-      // Only pushes of tasks of this launch fill the queue; any other value
-      // is reported (error 2) instead of being used as an index.
-      atomicExch(b.error, 2);
+  const int leader = __ffs(idle) - 1;
+  uint32_t base = 0;
+  if (lane == static_cast<uint32_t>(leader)) base = atomicAdd(q.ctl, __popc(idle));
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if ((idle >> lane) & 1) {
+    ln.slot = base + __popc(idle & lt_mask);
+    if (ln.slot >= q.total) {
       ln.state = kExhausted;
-    } else if (ln.qv != 0) {
-      ln.task = ln.qv - 1;
-      // Consumed: leave the entry zero for the next launch.
-      q.queue[ln.slot - q.initial] = 0;
-      ln.si = soup_of_task(b.soups, s_lo, s_hi, ln.task);
+    } else if (ln.slot < q.initial) {  // a first-epoch pair: ready
+      ln.si = soup_of_slot(b.soups, s_lo, s_hi, ln.slot);
       const PipeSoup &sp = b.soups[ln.si];
-      const uint32_t rel = ln.task - sp.task_base;
-      ln.e = rel / sp.npairs;
-      ln.k = rel - ln.e * sp.npairs;
-      ln.qp = *reinterpret_cast<const unsigned long long *>(sp.perm + uint64_t(ln.e) * sp.n +
-                                                            2 * uint64_t(ln.k));
+      ln.task = sp.task_base + (ln.slot - sp.init_base);
       ln.state = kIndex;
-      progressed = true;
-    } else if (ln.poll_in-- == 0) {
-      if (ln.err) {
-        ln.state = kExhausted;
-      } else {
-        const uint64_t now = globaltimer_ns();
-        if (ln.t_wait == 0) {
-          ln.t_wait = now;
-        } else if (now - ln.t_wait > b.wait_limit_ns) {
-          atomicExch(b.error, 1);
-          ln.state = kExhausted;
-        }
-      }
-      if (ln.state == kSlot) {
-        ln.qv = ld_relaxed(q.queue + (ln.slot - q.initial));
-        ln.err = ld_relaxed(reinterpret_cast<const uint32_t *>(b.error));
-        ln.poll_gap = ln.poll_gap < 16 ? ln.poll_gap * 2 : 16;
-        ln.poll_in = ln.poll_gap;
-      }
-    }
-  } else if (ln.state == kIndex) {
-    // 3. Shuffle indices landed: order after the producers, issue the gather,
-    //    the mutation mask and the next epoch's positions of both programs.
-    const PipeSoup &sp = b.soups[ln.si];
-    if (ln.slot < q.initial) {
-      ln.e = 0;
-      ln.k = ln.slot - sp.init_base;
-    }
-    ln.p1 = static_cast<uint32_t>(ln.qp);
-    ln.p2 = static_cast<uint32_t>(ln.qp >> 32);
-    fence_acq_rel_gpu();
-    // Both inputs have been counted: leave the counter zero for the next launch.
-    if (ln.e > 0) sp.readycnt[uint64_t(ln.e) * sp.npairs + ln.k] = 0;
-    const uint4 *g1 = reinterpret_cast<const uint4 *>(sp.soup + uint64_t(ln.p1) * kTape);
-    const uint4 *g2 = reinterpret_cast<const uint4 *>(sp.soup + uint64_t(ln.p2) * kTape);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      ln.g[i] = __ldcg(g1 + i);
-      ln.g[4 + i] = __ldcg(g2 + i);
-    }
-    ln.mm = __ldg(sp.mutmask + uint64_t(ln.e) * sp.npairs + ln.k);
-    ln.has_next = ln.e + 1 < sp.n_epochs;
-    if (ln.has_next) {
-      ln.j1 = __ldg(sp.inv + uint64_t(ln.e + 1) * sp.n + ln.p1);
-      ln.j2 = __ldg(sp.inv + uint64_t(ln.e + 1) * sp.n + ln.p2);
-    }
-    ln.state = kStage;
-    progressed = true;
-  } else if (ln.state == kStage) {
-    // 4. Stage the pair: bytes into shared memory, command mask, mutations.
-    const PipeSoup &sp = b.soups[ln.si];
-    Mask128 cmd{0, 0};
-#pragma unroll
-    for (int qd = 0; qd < 32; qd++) {
-      const uint32_t w = qd % 4 == 0 ? ln.g[qd / 4].x : qd % 4 == 1 ? ln.g[qd / 4].y
-                       : qd % 4 == 2 ? ln.g[qd / 4].z : ln.g[qd / 4].w;
-#pragma unroll
-      for (int bb = 0; bb < 4; bb++) t.set(4 * qd + bb, w >> (8 * bb));
-      if (kBffFam) {
-        const uint32_t f = cmdflag[w & 0xFF] | (cmdflag[(w >> 8) & 0xFF] << 8) |
-                           (cmdflag[(w >> 16) & 0xFF] << 16) | (cmdflag[w >> 24] << 24);
-        const uint64_t nib = (f * 0x01020408u) >> 24;
-        if (qd < 16) cmd.lo |= nib << (4 * qd);
-        else cmd.hi |= nib << (4 * (qd - 16));
-      }
-    }
-    ln.dirty = (ln.mm.x | ln.mm.y | ln.mm.z | ln.mm.w) != 0;
-    if (ln.dirty) {
-      const uint64_t key0 = (sp.n * seed_from(sp.s0, sp.e0 + ln.e) + ln.k) * kPair;
-      const uint32_t mw[4] = {ln.mm.x, ln.mm.y, ln.mm.z, ln.mm.w};
-#pragma unroll
-      for (int qd = 0; qd < 4; qd++) {
-        uint32_t bits = mw[qd];
-        while (bits) {
-          const int i = qd * 32 + __ffs(bits) - 1;
-          bits &= bits - 1;
-          const uint32_t v = static_cast<uint32_t>(splitmix64(key0 + i)) & 0xFFu;
-          t.set(i, v);
-          if (kBffFam) mask_assign(cmd, i, cmdflag[v] != 0);
-        }
-      }
-    }
-    const uint64_t num_indices = sp.num_indices ? sp.num_indices[ln.e] : sp.npairs;
-    ln.evaluated = ln.k < num_indices;
-    m.begin(t, cmd);
-    ln.visits = 0;
-    ln.state = kRun;
-    progressed = true;
-  } else if (ln.state == kRun) {
-    // 5. A few interpreter steps; on the end, write back and notify.
-    progressed = true;
-    bool fin = !ln.evaluated;
-    const uint32_t steps = ln.visits ? b.tune.steps_per_visit : b.tune.first_visit_steps;
-    for (uint32_t r = 0; r < steps && !fin; r++) fin = m.step(t, stk, np, optab);
-    ln.visits++;
-    if (fin) {
-      const PipeSoup &sp = b.soups[ln.si];
-      if (ln.dirty || (ln.evaluated && m.mods() != 0)) {
-        uint32_t w[32];
-#pragma unroll
-        for (int qd = 0; qd < 32; qd++)
-          w[qd] = t.get(4 * qd) | (t.get(4 * qd + 1) << 8) | (t.get(4 * qd + 2) << 16) |
-                  (t.get(4 * qd + 3) << 24);
-        // First half, then second half (common_language.h:188-191).
-        uint4 *o1 = reinterpret_cast<uint4 *>(sp.soup + uint64_t(ln.p1) * kTape);
-        uint4 *o2 = reinterpret_cast<uint4 *>(sp.soup + uint64_t(ln.p2) * kTape);
-#pragma unroll
-        for (int qd = 0; qd < 4; qd++)
-          o1[qd] = make_uint4(w[4 * qd], w[4 * qd + 1], w[4 * qd + 2], w[4 * qd + 3]);
-#pragma unroll
-        for (int qd = 0; qd < 4; qd++)
-          o2[qd] = make_uint4(w[16 + 4 * qd], w[16 + 4 * qd + 1], w[16 + 4 * qd + 2],
-                              w[16 + 4 * qd + 3]);
-      }
-      if (ln.evaluated) {
-        unsigned long long *c = sp.ops + (uint64_t(ln.e) * kCountSlots + slot_ctr) * 2;
-        if (m.ops()) atomicAdd(c, static_cast<unsigned long long>(m.ops()));
-        if (m.raw()) atomicAdd(c + 1, static_cast<unsigned long long>(m.raw()));
-      }
-      if (ln.has_next) {
-        // The acq_rel increments order the stores above before them, and make
-        // the earlier producer's stores visible to whoever pushes.
-        uint32_t *rc = sp.readycnt + uint64_t(ln.e + 1) * sp.npairs;
-        ln.c1 = atom_add_acq_rel(rc + (ln.j1 >> 1), 1);
-        ln.c2 = atom_add_acq_rel(rc + (ln.j2 >> 1), 1);
-        ln.state = kNotify;
-      } else {
-        ln.state = kIdle;
-      }
+      ln.qp = *reinterpret_cast<const unsigned long long *>(sp.perm + 2 * uint64_t(ln.slot - sp.init_base));
+    } else {
+      ln.state = kSlot;
+      ln.qv = ld_relaxed(q.queue + (ln.slot - q.initial));
+      ln.poll_gap = 1;
+      ln.poll_in = 0;
+      ln.t_wait = 0;
     }
   }
-  // 6. Push the consumers whose second input this pair was.
+}
+
+// A lane in kSlot: its slot's entry, loaded in an earlier iteration, is taken
+// up or loaded again.  Returns true when it was there.
+__device__ __forceinline__ bool poll_slot(const PipeCtx &b, const PipeQueue &q, Lane &ln) {
+  const int s_lo = static_cast<int>(q.first_soup), s_hi = static_cast<int>(q.first_soup + q.n_soups);
+  bool progressed = false;
+  if (ln.qv != 0 && ln.qv - 1 >= q.total) {
+    // Only pushes of tasks of this launch fill the queue; any other value
+    // is reported (error 2) instead of being used as an index.
+    atomicExch(b.error, 2);
+    ln.state = kExhausted;
+  } else if (ln.qv != 0) {
+    ln.task = ln.qv - 1;
+    // Consumed: leave the entry zero for the next launch.
+    q.queue[ln.slot - q.initial] = 0;
+    ln.si = soup_of_task(b.soups, s_lo, s_hi, ln.task);
+    const PipeSoup &sp = b.soups[ln.si];
+    const uint32_t rel = ln.task - sp.task_base;
+    ln.e = rel / sp.npairs;
+    ln.k = rel - ln.e * sp.npairs;
+    ln.qp = *reinterpret_cast<const unsigned long long *>(sp.perm + uint64_t(ln.e) * sp.n +
+                                                          2 * uint64_t(ln.k));
+    ln.state = kIndex;
+    progressed = true;
+  } else if (ln.poll_in-- == 0) {
+    if (ln.err) {
+      ln.state = kExhausted;
+    } else {
+      const uint64_t now = globaltimer_ns();
+      if (ln.t_wait == 0) {
+        ln.t_wait = now;
+      } else if (now - ln.t_wait > b.wait_limit_ns) {
+        atomicExch(b.error, 1);
+        ln.state = kExhausted;
+      }
+    }
+    if (ln.state == kSlot) {
+      ln.qv = ld_relaxed(q.queue + (ln.slot - q.initial));
+      ln.err = ld_relaxed(reinterpret_cast<const uint32_t *>(b.error));
+      ln.poll_gap = ln.poll_gap < 16 ? ln.poll_gap * 2 : 16;
+      ln.poll_in = ln.poll_gap;
+    }
+  }
+  return progressed;
+}
+
+// A lane in kIndex: its shuffle indices have landed.  Orders its reads after
+// the producers' writes and loads the next epoch's positions of both programs.
+__device__ __forceinline__ void take_index(const PipeSoup &sp, const PipeQueue &q, Lane &ln) {
+  if (ln.slot < q.initial) {
+    ln.e = 0;
+    ln.k = ln.slot - sp.init_base;
+  }
+  ln.p1 = static_cast<uint32_t>(ln.qp);
+  ln.p2 = static_cast<uint32_t>(ln.qp >> 32);
+  fence_acq_rel_gpu();
+  // Both inputs have been counted: leave the counter zero for the next launch.
+  if (ln.e > 0) sp.readycnt[uint64_t(ln.e) * sp.npairs + ln.k] = 0;
+  ln.has_next = ln.e + 1 < sp.n_epochs;
+  if (ln.has_next) {
+    ln.j1 = __ldg(sp.inv + uint64_t(ln.e + 1) * sp.n + ln.p1);
+    ln.j2 = __ldg(sp.inv + uint64_t(ln.e + 1) * sp.n + ln.p2);
+  }
+}
+
+// The mutations of a pair (common_language.h:172-180), whose positions mm
+// marks: set(i, byte) for each.
+template <class F>
+__device__ __forceinline__ void mutate_bits(const PipeSoup &sp, const Lane &ln, uint4 mm, F set) {
+  const uint64_t key0 = (sp.n * seed_from(sp.s0, sp.e0 + ln.e) + ln.k) * kPair;
+  const uint32_t mw[4] = {mm.x, mm.y, mm.z, mm.w};
+#pragma unroll
+  for (int qd = 0; qd < 4; qd++) {
+    uint32_t bits = mw[qd];
+    while (bits) {
+      const int i = qd * 32 + __ffs(bits) - 1;
+      bits &= bits - 1;
+      set(i, static_cast<uint32_t>(splitmix64(key0 + i)) & 0xFFu);
+    }
+  }
+}
+
+// Writes back the 32 words of a lane's pair: first half, then second half
+// (common_language.h:188-191).
+template <class F>
+__device__ __forceinline__ void store_pair(const PipeSoup &sp, const Lane &ln, F word) {
+  uint4 *o1 = reinterpret_cast<uint4 *>(sp.soup + uint64_t(ln.p1) * kTape);
+  uint4 *o2 = reinterpret_cast<uint4 *>(sp.soup + uint64_t(ln.p2) * kTape);
+#pragma unroll
+  for (int qd = 0; qd < 4; qd++)
+    o1[qd] = make_uint4(word(4 * qd), word(4 * qd + 1), word(4 * qd + 2), word(4 * qd + 3));
+#pragma unroll
+  for (int qd = 0; qd < 4; qd++)
+    o2[qd] = make_uint4(word(16 + 4 * qd), word(17 + 4 * qd), word(18 + 4 * qd),
+                        word(19 + 4 * qd));
+}
+
+// A finished pair whose bytes have been written: adds its counts and notifies
+// the consumers of its two programs.
+__device__ __forceinline__ void finish(const PipeSoup &sp, Lane &ln, uint32_t slot_ctr,
+                                       uint32_t ops, uint32_t raw) {
+  if (ln.evaluated) {
+    unsigned long long *c = sp.ops + (uint64_t(ln.e) * kCountSlots + slot_ctr) * 2;
+    if (ops) atomicAdd(c, static_cast<unsigned long long>(ops));
+    if (raw) atomicAdd(c + 1, static_cast<unsigned long long>(raw));
+  }
+  if (ln.has_next) {
+    // The acq_rel increments order the stores above before them, and make
+    // the earlier producer's stores visible to whoever pushes.
+    uint32_t *rc = sp.readycnt + uint64_t(ln.e + 1) * sp.npairs;
+    ln.c1 = atom_add_acq_rel(rc + (ln.j1 >> 1), 1);
+    ln.c2 = atom_add_acq_rel(rc + (ln.j2 >> 1), 1);
+    ln.state = kNotify;
+  } else {
+    ln.state = kIdle;
+  }
+}
+
+// Pushes the consumers whose second input was a pair of a lane in kNotify.
+__device__ __forceinline__ void push_ready(const PipeCtx &b, const PipeQueue &q, Lane &ln,
+                                           uint32_t lane) {
+  const uint32_t lt_mask = (1u << lane) - 1;
   const bool same = (ln.j2 >> 1) == (ln.j1 >> 1);
   const bool push1 = ln.state == kNotify && (ln.c1 == 1 || (same && ln.c2 == 1));
   const bool push2 = ln.state == kNotify && !same && ln.c2 == 1;
@@ -367,63 +336,276 @@ __device__ __forceinline__ bool iterate(const PipeCtx &b, const PipeQueue &q, La
                      next + (ln.j2 >> 1) + 1);
   }
   if (ln.state == kNotify) ln.state = kIdle;
-  return progressed;
 }
 
-// A warp serves queue q until every lane has claimed past its last task.
+// The Forth and SUBLEQ languages: one pair per lane.  iterate() is one
+// iteration of the warp; it returns true if the lane made progress.
 template <int L>
-__device__ __forceinline__ void serve(const PipeCtx &b, const PipeQueue &q,
-                                      const uint8_t *__restrict__ optab,
-                                      const uint8_t *__restrict__ cmdflag, const LaneBytes t,
-                                      const LaneBytes stk, const LaneNp np, uint32_t lane,
-                                      uint32_t slot_ctr) {
-  Lane ln;
-  ln.state = kIdle;
-  ln.slot = ln.task = ln.e = ln.k = ln.p1 = ln.p2 = ln.qv = 0;
-  ln.poll_gap = 1;
-  ln.poll_in = ln.err = ln.j1 = ln.j2 = ln.c1 = ln.c2 = ln.visits = 0;
-  ln.si = 0;
-  ln.qp = ln.t_wait = 0;
-  ln.dirty = ln.evaluated = ln.has_next = false;
-  ln.mm = make_uint4(0, 0, 0, 0);
+struct LaneServer {
   LaneMachine<L> m;
-  while (true) {
-    const bool progressed = iterate<L>(b, q, ln, m, t, stk, np, optab, cmdflag, lane, slot_ctr);
-    if (__all_sync(0xffffffffu, ln.state == kExhausted)) return;
-    if (!__any_sync(0xffffffffu, progressed)) __nanosleep(200);
-  }
-}
+  uint32_t visits;
+  uint4 g[8];
+  uint4 mm;
+  LaneBytes t, stk;
+  const uint8_t *optab;
 
-// Shared memory of a pipelined launch: the tape and second areas, the BFF
-// next-command arrays (BFF family only), the op and command tables, then the
-// soup descriptors.
+  static constexpr uint32_t kWidth = 32;                     // lanes that hold pairs
+  static constexpr size_t kWarpBytes = 2 * kGroupBytes / 4;  // of shared memory
+
+  __device__ __forceinline__ LaneServer(uint8_t *smem, const uint8_t *tables, uint32_t tid)
+      : visits(0), t{smem, lane_base(tid)}, stk{smem + kGroups * kGroupBytes, lane_base(tid)},
+        optab(tables) {
+    mm = make_uint4(0, 0, 0, 0);
+  }
+
+  __device__ __forceinline__ bool iterate(const PipeCtx &b, const PipeQueue &q, Lane &ln,
+                                          uint32_t lane, uint32_t slot_ctr) {
+    // 1. Bulk claim of queue slots by idle lanes.
+    const uint32_t idle = __ballot_sync(0xffffffffu, ln.state == kIdle);
+    const uint32_t busy = __ballot_sync(0xffffffffu, ln.state != kIdle && ln.state != kExhausted);
+    const uint32_t lng = __ballot_sync(0xffffffffu, ln.state == kRun && visits >= b.tune.long_visits);
+    if (idle && (busy == 0 || (lng == 0 && __popc(idle) >= b.tune.claim_min)))
+      claim(b, q, ln, idle, lane);
+    bool progressed = false;
+
+    if (ln.state == kSlot) {
+      // 2. Waiting for the claimed slot's entry (polled in an earlier iteration).
+      progressed = poll_slot(b, q, ln);
+    } else if (ln.state == kIndex) {
+      // 3. Shuffle indices landed: order after the producers, issue the gather,
+      //    the mutation mask and the next epoch's positions of both programs.
+      const PipeSoup &sp = b.soups[ln.si];
+      take_index(sp, q, ln);
+      const uint4 *g1 = reinterpret_cast<const uint4 *>(sp.soup + uint64_t(ln.p1) * kTape);
+      const uint4 *g2 = reinterpret_cast<const uint4 *>(sp.soup + uint64_t(ln.p2) * kTape);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        g[i] = __ldcg(g1 + i);
+        g[4 + i] = __ldcg(g2 + i);
+      }
+      mm = __ldg(sp.mutmask + uint64_t(ln.e) * sp.npairs + ln.k);
+      ln.state = kStage;
+      progressed = true;
+    } else if (ln.state == kStage) {
+      // 4. Stage the pair: bytes into shared memory, mutations.
+      const PipeSoup &sp = b.soups[ln.si];
+#pragma unroll
+      for (int qd = 0; qd < 32; qd++) {
+        const uint32_t w = qd % 4 == 0 ? g[qd / 4].x : qd % 4 == 1 ? g[qd / 4].y
+                         : qd % 4 == 2 ? g[qd / 4].z : g[qd / 4].w;
+#pragma unroll
+        for (int bb = 0; bb < 4; bb++) t.set(4 * qd + bb, w >> (8 * bb));
+      }
+      ln.dirty = (mm.x | mm.y | mm.z | mm.w) != 0;
+      if (ln.dirty)
+        mutate_bits(sp, ln, mm, [&](int i, uint32_t v) { t.set(i, v); });
+      const uint64_t num_indices = sp.num_indices ? sp.num_indices[ln.e] : sp.npairs;
+      ln.evaluated = ln.k < num_indices;
+      m.begin(t, Mask128{0, 0});
+      visits = 0;
+      ln.state = kRun;
+      progressed = true;
+    } else if (ln.state == kRun) {
+      // 5. A few interpreter steps; on the end, write back and notify.
+      progressed = true;
+      bool fin = !ln.evaluated;
+      const uint32_t steps = visits ? b.tune.steps_per_visit : b.tune.first_visit_steps;
+      for (uint32_t r = 0; r < steps && !fin; r++) fin = m.step(t, stk, LaneNp{nullptr, 0}, optab);
+      visits++;
+      if (fin) {
+        const PipeSoup &sp = b.soups[ln.si];
+        if (ln.dirty || (ln.evaluated && m.mods() != 0)) {
+          uint32_t w[32];
+#pragma unroll
+          for (int qd = 0; qd < 32; qd++)
+            w[qd] = t.get(4 * qd) | (t.get(4 * qd + 1) << 8) | (t.get(4 * qd + 2) << 16) |
+                    (t.get(4 * qd + 3) << 24);
+          store_pair(sp, ln, [&](int qd) { return w[qd]; });
+        }
+        finish(sp, ln, slot_ctr, m.ops(), m.raw());
+      }
+    }
+    // 6. Push the consumers whose second input this pair was.
+    push_ready(b, q, ln, lane);
+    return progressed;
+  }
+};
+
+// The BFF family.  The lanes of a warp run the forward part of a pair each
+// (BffLane): most random programs end there, and those pairs are written back
+// and their consumers notified at once.  The pairs that jump are kept (kLong)
+// and run one after the other on the whole warp (BffWarp), one per iteration,
+// so that slots held by other lanes are still polled in between.  So that
+// pairs wait behind few others, a warp holds 8 and there are many warps: a soup
+// of 2^17 bff programs taken over by self-replicators takes 35.4 ms for 16
+// epochs with 8 (32 lanes: 76.9, 16: 44.6), one of 1022 bff_noheads programs
+// 2.1 ms for 64 (4.3, 3.0); only the 20 first epochs of a random soup of 2^17
+// are a little faster with 32 (3.07 ms, 8: 3.27).
 template <int L>
-__host__ __device__ constexpr size_t pipeline_np_bytes() {
-  return L <= kBffSelfmove ? size_t(kNpBytes) : 0;
+struct BffServer {
+  using LaneM = typename BffMachines<L>::Lane;
+  using WarpM = typename BffMachines<L>::template Warp<DeviceWarp>;
+  static constexpr uint32_t kWidth = 8;  // lanes that hold pairs
+  static constexpr size_t kTapes = kWidth * kPair, kWarpBytes = kTapes + sizeof(BffMem);
+  LaneM m;
+  LaneWords<kWidth> t;
+  BffMem &mem;
+  const uint8_t *optab, *cmdflag;
+
+  __device__ __forceinline__ BffServer(uint8_t *smem, const uint8_t *tables, uint32_t tid)
+      : t{smem + (tid >> 5) * kWarpBytes, tid & 31},
+        mem(*reinterpret_cast<BffMem *>(smem + (tid >> 5) * kWarpBytes + kTapes)),
+        optab(tables), cmdflag(tables + 256) {
+    m.status = LaneM::kEnds;
+  }
+
+  // Stages the pair of a lane in kIndex: bytes into shared memory, command
+  // mask, mutations.
+  __device__ __forceinline__ void stage(const PipeSoup &sp, Lane &ln) {
+    const uint4 *g1 = reinterpret_cast<const uint4 *>(sp.soup + uint64_t(ln.p1) * kTape);
+    const uint4 *g2 = reinterpret_cast<const uint4 *>(sp.soup + uint64_t(ln.p2) * kTape);
+    uint4 g[8];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      g[i] = __ldcg(g1 + i);
+      g[4 + i] = __ldcg(g2 + i);
+    }
+    const uint4 mm = __ldg(sp.mutmask + uint64_t(ln.e) * sp.npairs + ln.k);
+    Mask128 cmd{0, 0};
+#pragma unroll
+    for (int qd = 0; qd < 32; qd++) {
+      const uint32_t w = qd % 4 == 0 ? g[qd / 4].x : qd % 4 == 1 ? g[qd / 4].y
+                       : qd % 4 == 2 ? g[qd / 4].z : g[qd / 4].w;
+      t.word(qd) = w;
+      const uint32_t f = cmdflag[w & 0xFF] | (cmdflag[(w >> 8) & 0xFF] << 8) |
+                         (cmdflag[(w >> 16) & 0xFF] << 16) | (cmdflag[w >> 24] << 24);
+      const uint64_t nib = (f * 0x01020408u) >> 24;
+      if (qd < 16) cmd.lo |= nib << (4 * qd);
+      else cmd.hi |= nib << (4 * (qd - 16));
+    }
+    ln.dirty = (mm.x | mm.y | mm.z | mm.w) != 0;
+    if (ln.dirty) {
+      mutate_bits(sp, ln, mm, [&](int i, uint32_t v) {
+        t.set(i, v);
+        mask_assign(cmd, i, cmdflag[v] != 0);
+      });
+    }
+    const uint64_t num_indices = sp.num_indices ? sp.num_indices[ln.e] : sp.npairs;
+    ln.evaluated = ln.k < num_indices;
+    m.begin(t, cmd, optab);
+    if (!ln.evaluated) m.status = LaneM::kEnds;
+  }
+
+  // Runs the pair of lane `src` on the whole warp, writes it back and finishes
+  // it.
+  __device__ __forceinline__ void run_long(const PipeCtx &b, Lane &ln, uint32_t src,
+                                           uint32_t lane, uint32_t slot_ctr) {
+    constexpr uint32_t kAll = 0xffffffffu;
+    BffState st;
+    st.q = __shfl_sync(kAll, m.st.q, src);
+    st.h0 = __shfl_sync(kAll, m.st.h0, src);
+    st.h1 = __shfl_sync(kAll, m.st.h1, src);
+    st.i = __shfl_sync(kAll, m.st.i, src);
+    st.n = __shfl_sync(kAll, m.st.n, src);
+    st.mods = __shfl_sync(kAll, m.st.mods, src);
+    __syncwarp();  // the lane's tape
+    uint32_t *T = reinterpret_cast<uint32_t *>(mem.T);
+    T[lane] = reinterpret_cast<const uint32_t *>(t.s)[lane * kWidth + src];
+    __syncwarp();
+    WarpM wm(DeviceWarp{lane}, mem, optab);
+    wm.run(st);
+    __syncwarp();
+    const PipeSoup &sp = b.soups[__shfl_sync(kAll, ln.si, src)];
+    if (wm.st.mods != 0 || __shfl_sync(kAll, ln.dirty, src)) {
+      const uint32_t p1 = __shfl_sync(kAll, ln.p1, src), p2 = __shfl_sync(kAll, ln.p2, src);
+      // First half, then second half (common_language.h:188-191): of a
+      // program paired with itself the second half stays.
+      if (lane >= 16 || p1 != p2)
+        reinterpret_cast<uint32_t *>(sp.soup + uint64_t(lane < 16 ? p1 : p2) * kTape)[lane & 15] =
+            T[lane];
+    }
+    __syncwarp();  // the warp's stores before the lane's notifications
+    if (lane == src) finish(sp, ln, slot_ctr, wm.st.n, wm.raw());
+  }
+
+  __device__ __forceinline__ bool iterate(const PipeCtx &b, const PipeQueue &q, Lane &ln,
+                                          uint32_t lane, uint32_t slot_ctr) {
+    // 1. The next long pair, or a bulk claim of queue slots by idle lanes.
+    const uint32_t lng = __ballot_sync(0xffffffffu, ln.state == kLong);
+    if (lng) {
+      run_long(b, ln, static_cast<uint32_t>(__ffs(lng) - 1), lane, slot_ctr);
+    } else {
+      const uint32_t idle = __ballot_sync(0xffffffffu, ln.state == kIdle);
+      const uint32_t busy = __ballot_sync(0xffffffffu, ln.state != kIdle && ln.state != kExhausted);
+      if (idle && busy == 0) claim(b, q, ln, idle, lane);
+    }
+    bool progressed = lng != 0;
+
+    if (ln.state == kSlot) {
+      // 2. Waiting for the claimed slot's entry (polled in an earlier iteration).
+      progressed |= poll_slot(b, q, ln);
+    } else if (ln.state == kIndex) {
+      // 3. Shuffle indices landed: gather and stage the pair.
+      const PipeSoup &sp = b.soups[ln.si];
+      take_index(sp, q, ln);
+      stage(sp, ln);
+      ln.state = kRun;
+      progressed = true;
+    }
+    // 4. The forward parts of the pairs just staged, all lanes together.
+    while (true) {
+      const bool go = ln.state == kRun && m.status == LaneM::kRuns;
+      if (!__any_sync(0xffffffffu, go)) break;
+      if (go) m.step(t, optab);
+    }
+    // 5. Pairs that ended: write back and notify.
+    if (ln.state == kRun) {
+      if (m.status == LaneM::kJumps) m.resolve(t, optab);
+      if (m.status == LaneM::kJumps) {
+        ln.state = kLong;
+      } else {
+        const PipeSoup &sp = b.soups[ln.si];
+        if (ln.dirty || (ln.evaluated && m.st.mods != 0))
+          store_pair(sp, ln, [&](int qd) { return t.word(qd); });
+        finish(sp, ln, slot_ctr, m.st.n, m.st.i);
+      }
+    }
+    // 6. Push the consumers whose second input this pair was.
+    push_ready(b, q, ln, lane);
+    return progressed;
+  }
+};
+
+template <int L>
+using Server = std::conditional_t<(L <= kBffSelfmove), BffServer<L>, LaneServer<L>>;
+
+// Shared memory of a pipelined launch: the servers' (tapes and so on), the op
+// and command tables, then the soup descriptors.
+template <int L>
+__host__ __device__ constexpr size_t server_bytes() {
+  return (kThreads / 32) * Server<L>::kWarpBytes;
 }
 
 template <int L>
 size_t pipeline_smem_bytes(int n_soups) {
-  return 2 * kGroups * kGroupBytes + pipeline_np_bytes<L>() + 512 +
-         size_t(n_soups) * sizeof(PipeSoup);
+  return server_bytes<L>() + 512 + size_t(n_soups) * sizeof(PipeSoup);
 }
 
-// The persistent kernel of a pipelined launch over soups of language L.  The
-// BFF family's larger shared-memory footprint allows 3 blocks per SM, the
-// others 4; the register budget follows.
+// The persistent kernel of a pipelined launch over soups of language L.
+// Blocks per SM set the register budget: the BFF machines take 96 without
+// spills that matter (6 blocks, 80 registers: 39.9 ms instead of 35.1 on the
+// self-replicators above), the lanes' shared memory allows the others 4.
 template <int L>
-__global__ void __launch_bounds__(kThreads, (L <= kBffSelfmove) ? 3 : 4)
+__global__ void __launch_bounds__(kThreads, (L <= kBffSelfmove) ? 5 : 4)
     pipeline_kernel(const __grid_constant__ PipeBatch pb) {
   extern __shared__ __align__(16) uint8_t smem[];
-  uint16_t *npa = reinterpret_cast<uint16_t *>(smem + 2 * kGroups * kGroupBytes);
-  uint8_t *optab = smem + 2 * kGroups * kGroupBytes + pipeline_np_bytes<L>();
-  uint8_t *cmdflag = optab + 256;
-  PipeSoup *soups = reinterpret_cast<PipeSoup *>(optab + 512);
+  uint8_t *tables = smem + server_bytes<L>();
+  PipeSoup *soups = reinterpret_cast<PipeSoup *>(tables + 512);
   const uint32_t tid = threadIdx.x, lane = tid & 31;
   if (LangTraits<L>::kNeedsTable) {
     for (uint32_t c = tid; c < 256; c += kThreads) {
-      optab[c] = op_of(L, c);
-      cmdflag[c] = op_of(L, c) < kNull;
+      tables[c] = op_of(L, c);
+      tables[256 + c] = op_of(L, c) < kNull;
     }
   }
   {
@@ -433,13 +615,19 @@ __global__ void __launch_bounds__(kThreads, (L <= kBffSelfmove) ? 3 : 4)
     for (uint32_t i = tid; i < words; i += kThreads) dst[i] = src[i];
   }
   __syncthreads();  // tables and descriptors are read-only from here on
-  const LaneBytes t{smem, lane_base(tid)};
-  const LaneBytes stk{smem + kGroups * kGroupBytes, lane_base(tid)};
   const uint32_t warp = blockIdx.x * (kThreads / 32) + (tid >> 5);
-  const LaneNp np{L <= kBffSelfmove ? npa : nullptr, tid};
   const PipeCtx b{soups, pb.error, pb.wait_limit_ns, pb.tune};
   const PipeQueue q = pb.queue;
-  serve<L>(b, q, optab, cmdflag, t, stk, np, lane, warp % kCountSlots);
+  Server<L> server(smem, tables, tid);
+  Lane ln;
+  ln.begin();
+  if (lane >= Server<L>::kWidth) ln.state = kExhausted;
+  // A warp serves the queue until every lane has claimed past its last task.
+  while (true) {
+    const bool progressed = server.iterate(b, q, ln, lane, warp % kCountSlots);
+    if (__all_sync(0xffffffffu, ln.state == kExhausted)) return;
+    if (!__any_sync(0xffffffffu, progressed)) __nanosleep(200);
+  }
 }
 
 template <int L>
@@ -466,7 +654,8 @@ int launch_pipeline_t(const PipeBatch &b, uint64_t total_pairs, uint32_t lanes_p
   // pairs in flight.
   uint64_t want = (total_pairs * uint64_t(lanes_per_pair64 ? lanes_per_pair64 : 32)) / 64;
   want = std::max<uint64_t>(want, kThreads);
-  const uint64_t blocks = (want + kThreads - 1) / kThreads;
+  const uint64_t per_block = kThreads / 32 * Server<L>::kWidth;
+  const uint64_t blocks = (want + per_block - 1) / per_block;
   const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(blocks, resident));
   pipeline_kernel<L><<<grid, kThreads, smem, stream>>>(b);
   CUBFF_CUDA_TRY(cudaGetLastError());
