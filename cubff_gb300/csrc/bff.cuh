@@ -73,7 +73,7 @@ struct BffLane {
   // One command that does not jump (fewer than kPair run, so the step limit is
   // never reached).
   template <class Tape>
-  __host__ __device__ __forceinline__ void step(const Tape t,
+  __host__ __device__ __forceinline__ void step(const Tape t, const Tape,
                                                 const uint8_t *__restrict__ optab) {
     st.h0 = (st.h0 + (c == kInc0) - (c == kDec0)) & (kPair - 1);
     st.h1 = (st.h1 + (c == kInc1 || (kLogic == kLogicSelfmove && c == kCopy10)) - (c == kDec1)) &
@@ -108,6 +108,11 @@ struct BffLane {
     st.i++;
     status = kEnds;
   }
+
+  __host__ __device__ __forceinline__ const BffState &state() const { return st; }
+  __host__ __device__ __forceinline__ uint32_t ops() const { return st.n; }
+  __host__ __device__ __forceinline__ uint32_t raw() const { return st.i; }
+  __host__ __device__ __forceinline__ uint32_t mods() const { return st.mods; }
 };
 
 // Shared memory of one warp's BffWarp.
@@ -782,6 +787,8 @@ struct BffWarp {
     }
   }
 
+  __host__ __device__ __forceinline__ uint32_t ops() const { return st.n; }
+  __host__ __device__ __forceinline__ uint32_t mods() const { return st.mods; }
   __host__ __device__ __forceinline__ uint32_t raw() const {
     return st.i < kStepLimit ? st.i : kStepLimit;
   }

@@ -3,25 +3,24 @@
 //
 // Semantics: Stack (forth.inc.h:236-249), EvaluateOne (forth.inc.h:250-373),
 // Evaluate (forth.inc.h:379-397); forthtrivial_reset's Reset / ResetIf and its
-// Write1 / Copy0 (forthtrivial_reset.cu:58-72, :157-166, :215-223).  The
-// stack (128 bytes) lives in shared memory in the same bank-per-lane layout as
-// the tape, its top two entries in registers (ForthMachine).
+// Write1 / Copy0 (forthtrivial_reset.cu:58-72, :157-166, :215-223).  The top
+// two entries of the 128-byte stack are kept in registers.
 //
-// Exact cycle fast-forward at backward jumps (Brent's schedule, as in
-// cycle.cuh): the state is (pos, stack pointer, stack contents, tape).  The
-// stack below the stack pointer is compared byte for byte with the
-// snapshot's (kept packed in a register, so only for stacks of at most 8);
-// the tape through a count of value-changing writes (a write that stores the
-// byte already there changes nothing).  Stack slots at or above the stack
-// pointer are not part of the state: a push overwrites them before any read.
+// Three machines with the same results:
+//  * ForthFirst, one pair per lane, for a program's first steps (most random
+//    programs end in them);
+//  * ForthWarp, one pair per warp, which takes over from there;
+//  * ForthMachine, the one-shot one of the per-epoch kernels (forth_eval):
+//    ForthLane with a cycle check.
 #pragma once
 
-#include "cycle.cuh"
+#include "coop.cuh"
 #include "languages.cuh"
 
 namespace cubff {
 
-static __host__ __device__ __noinline__ void forth_reset(const LaneBytes t, int pos) {
+template <class Tape>
+static __host__ __device__ __noinline__ void forth_reset(const Tape t, int pos) {
   uint64_t seed = 0;
   for (int i = 0; i < kPair; i++) seed = splitmix64(seed ^ t.get(i));
   for (int i = 0; i < kTape; i++)
@@ -30,106 +29,116 @@ static __host__ __device__ __noinline__ void forth_reset(const LaneBytes t, int 
                                               static_cast<uint64_t>(i))));
 }
 
-// The top two stack entries live in registers (r0 = stack[sp - 1], r1 =
-// stack[sp - 2]); shared memory holds stack[0 .. sp - 2).  Most ops then
-// touch no memory for their stack traffic: a push spills the entry it
+// A tape that all lanes of a warp access alike, or a stack.
+struct SharedBytes {
+  uint8_t *s;
+  __host__ __device__ __forceinline__ uint32_t get(int p) const { return s[p & (kPair - 1)]; }
+  __host__ __device__ __forceinline__ void set(int p, uint32_t v) const {
+    s[p & (kPair - 1)] = static_cast<uint8_t>(v);
+  }
+};
+// Positions written in each half of a tape: [lo, hi] (none: lo > hi).
+struct Written {
+  int lo0, hi0, lo1, hi1;
+  __host__ __device__ __forceinline__ bool none() const { return hi0 < 0 && hi1 < 0; }
+  __host__ __device__ __forceinline__ void clear() {
+    lo0 = lo1 = kPair;
+    hi0 = hi1 = -1;
+  }
+  __host__ __device__ __forceinline__ void add(int p) {
+    if (p < kTape) {
+      lo0 = p < lo0 ? p : lo0;
+      hi0 = p > hi0 ? p : hi0;
+    } else {
+      lo1 = p < lo1 ? p : lo1;
+      hi1 = p > hi1 ? p : hi1;
+    }
+  }
+  __host__ __device__ __forceinline__ bool meets(int lo, int hi) const {
+    return (lo0 <= hi && hi0 >= lo) || (lo1 <= hi && hi1 >= lo);
+  }
+};
+// A shared tape that notes what is written.
+struct TrackedBytes {
+  uint8_t *s;
+  Written &written;
+  __host__ __device__ __forceinline__ uint32_t get(int p) const { return s[p & (kPair - 1)]; }
+  __host__ __device__ __forceinline__ void set(int p, uint32_t v) const {
+    s[p & (kPair - 1)] = static_cast<uint8_t>(v);
+    written.add(p);
+  }
+};
+template <class Tape>
+__host__ __device__ __forceinline__ void reset_tape(const Tape t, int pos) {
+  forth_reset(t, pos);
+}
+__host__ __device__ __forceinline__ void reset_tape(const TrackedBytes t, int pos) {
+  forth_reset(SharedBytes{t.s}, pos);
+  t.written.lo0 = 0;
+  t.written.hi0 = kTape - 1;
+}
+
+// Where a program stands.  The top two stack entries live in registers (r0 =
+// stack[sp - 1], r1 = stack[sp - 2]); memory holds stack[0 .. sp - 2).  Most
+// ops then touch no memory for their stack traffic: a push spills the entry it
 // pushes down, a pop refills the second entry, neither on the step's own
-// dependency chain.
-template <bool kWithReset>
-struct ForthMachine {
+// dependency chain.  Stack slots at or above sp hold anything; they are never
+// read before a push overwrites them.
+struct ForthState {
   int pos, sp;
   bool overflow;
   uint32_t r0, r1;         // stack[sp - 1], stack[sp - 2] (when they exist)
-  uint32_t i, nops, mods;  // mods: value-changing tape writes
-  // Brent-schedule snapshot taken at a backward jump.
-  int s_pos, s_sp;
-  uint32_t s_mods, s_i, s_nops, s_power, s_lam;
-  uint32_t s_top;          // stack[s_sp - 1] | stack[s_sp - 2] << 8 (0 where absent)
-  uint64_t s_mem;          // stack[0 .. s_sp - 2) packed, byte j at bits 8j (s_sp <= 8)
+  uint32_t i, nops, mods;  // raw steps, no-ops, value-changing tape writes
 
-  // Stack slots at or above sp hold bytes left by an earlier pair; they are
-  // never read before a push overwrites them.
   __host__ __device__ __forceinline__ void begin() {
     pos = sp = 0;
     overflow = false;
     r0 = r1 = 0;
     i = nops = mods = 0;
-    s_pos = -1;
-    s_sp = 0;
-    s_mods = s_i = s_nops = 0;
-    s_power = 1;
-    s_lam = 0;
-    s_top = 0;
-    s_mem = 0;
   }
+};
 
-  __host__ __device__ __forceinline__ void push(const LaneBytes stk, uint32_t v) {
-    if (sp != kPair) {
-      if (sp >= 2) stk.set(sp - 2, r1);
-      r1 = r0;
-      r0 = v & 0xFF;
-      sp++;
+template <bool kWithReset>
+struct ForthLane {
+  ForthState st;
+
+  template <class Tape>
+  __host__ __device__ __forceinline__ void push(const Tape stk, uint32_t v) {
+    if (st.sp != kPair) {
+      if (st.sp >= 2) stk.set(st.sp - 2, st.r1);
+      st.r1 = st.r0;
+      st.r0 = v & 0xFF;
+      st.sp++;
     } else {
-      overflow = true;
+      st.overflow = true;
     }
   }
 
-  // stack[0 .. sp - 2), the entries below the registers, packed.
-  __host__ __device__ __forceinline__ uint64_t pack_mem(const LaneBytes stk) const {
-    uint64_t w = 0;
-    for (int j = 0; j < sp - 2; j++) w |= static_cast<uint64_t>(stk.get(j)) << (8 * j);
-    return w;
-  }
-
-  // At a step boundary right after a backward jump: when the state equals
-  // the snapshot's, execution since the snapshot is periodic and whole periods
-  // are skipped (i += k * P, nops += k * the period's no-ops); the snapshot is
-  // renewed after 1, 2, 4, ... visits.  The two entries in registers are
-  // compared first: a loop's counter usually sits on top, so most visits end
-  // there without reading the stack in memory.
-  __host__ __device__ __forceinline__ void visit(const LaneBytes stk) {
-    const uint32_t top = (sp >= 1 ? r0 : 0u) | ((sp >= 2 ? r1 : 0u) << 8);
-    if (pos == s_pos && sp == s_sp && mods == s_mods && top == s_top &&
-        (sp <= 2 || pack_mem(stk) == s_mem)) {
-      const uint32_t period = i - s_i;
-      const uint32_t k = (kStepLimit - i) / period;
-      i += k * period;
-      nops += k * (nops - s_nops);
-    }
-    if (++s_lam == s_power) {
-      s_pos = sp <= 8 ? pos : -1;  // larger stacks: no snapshot
-      s_sp = sp;
-      s_mods = mods;
-      s_i = i;
-      s_nops = nops;
-      s_top = top;
-      s_mem = (sp > 2 && sp <= 8) ? pack_mem(stk) : 0;
-      s_power <<= 1;
-      s_lam = 0;
-    }
-  }
-  __host__ __device__ __forceinline__ uint32_t pop(const LaneBytes stk) {
-    if (sp == 0) return 0u;
-    const uint32_t v = r0;
-    sp--;
-    r0 = r1;
-    if (sp >= 2) r1 = stk.get(sp - 2);
+  template <class Tape>
+  __host__ __device__ __forceinline__ uint32_t pop(const Tape stk) {
+    if (st.sp == 0) return 0u;
+    const uint32_t v = st.r0;
+    st.sp--;
+    st.r0 = st.r1;
+    if (st.sp >= 2) st.r1 = stk.get(st.sp - 2);
     return v;
   }
-  __host__ __device__ __forceinline__ void write(const LaneBytes t, int a, uint32_t v) {
+  template <class Tape>
+  __host__ __device__ __forceinline__ void write(const Tape t, int a, uint32_t v) {
     v &= 0xFF;
     if (t.get(a) != v) {
       t.set(a, v);
-      mods++;
+      st.mods++;
     }
   }
 
-  // One step; returns true when the program has ended (ops = i - nops).
-  __host__ __device__ __forceinline__ bool step(const LaneBytes t, const LaneBytes stk,
-                                                const uint8_t *__restrict__ optab) {
-    const uint32_t c = t.get(pos);
-    bool back = false;
-    switch (optab[c]) {
+  // The step at st.pos, whose byte is c, of op `op` (back: it jumped
+  // backwards); returns true when the program has ended.
+  template <class Tape, class Stack>
+  __host__ __device__ __forceinline__ bool execute(const Tape t, const Stack stk, uint32_t op,
+                                                   uint32_t c, bool &back) {
+    back = false;
+    switch (op) {
       case kRead0: { const int a = pop(stk) % kTape; push(stk, t.get(a)); break; }
       case kRead1: { const int a = pop(stk) % kTape; push(stk, t.get(kTape + a)); break; }
       case kRead: { const int a = pop(stk) % kPair; push(stk, t.get(a)); break; }
@@ -149,8 +158,8 @@ struct ForthMachine {
         const uint32_t v = pop(stk);
         const int a = pop(stk) % kTape;
         if (kWithReset && t.get(kTape + a) == 0x13) {
-          forth_reset(t, pos);
-          mods++;
+          reset_tape(t, st.pos);
+          st.mods++;
         } else {
           write(t, kTape + a, v);
         }
@@ -166,7 +175,7 @@ struct ForthMachine {
       }
       case kIf0: {
         const uint32_t v = pop(stk);
-        if (v) pos++;
+        if (v) st.pos++;
         push(stk, v);
         break;
       }
@@ -178,8 +187,8 @@ struct ForthMachine {
       case kCopy0: {
         const int a = pop(stk) % kTape;
         if (kWithReset && t.get(kTape + a) == 0x13) {
-          forth_reset(t, pos);
-          mods++;
+          reset_tape(t, st.pos);
+          st.mods++;
         } else {
           write(t, kTape + a, t.get(a));
         }
@@ -195,25 +204,501 @@ struct ForthMachine {
       case kXor: push(stk, pop(stk) ^ 64); break;
       case kJmp: {
         const int a = (c & 63) + 1;
-        pos += (c & 64) ? -a : a;
-        pos--;
+        st.pos += (c & 64) ? -a : a;
+        st.pos--;
         back = (c & 64) != 0;
         break;
       }
-      default: nops++;
+      default: st.nops++;
     }
-    pos++;
-    i++;
-    if (pos >= kPair || pos < 0 || overflow || i >= kStepLimit) return true;
+    st.pos++;
+    st.i++;
+    if (st.pos >= kPair || st.pos < 0 || st.overflow || st.i >= kStepLimit) return true;
+    return false;
+  }
+  template <class Tape, class Stack>
+  __host__ __device__ __forceinline__ bool step(const Tape t, const Stack stk,
+                                                const uint8_t *__restrict__ optab, bool &back) {
+    const uint32_t c = t.get(st.pos);
+    return execute(t, stk, optab[c], c, back);
+  }
+};
+
+// The first steps of a program on one lane.
+template <bool kWithReset>
+struct ForthFirst {
+  // Most random programs end within 24 steps (90 % of those of a soup of 2^15
+  // forth programs after 256 epochs).
+  static constexpr uint32_t kSteps = 24;
+  enum Status : uint32_t { kRuns, kEnds, kJumps };
+  ForthLane<kWithReset> ln;
+  uint32_t status;
+
+  template <class Tape>
+  __host__ __device__ __forceinline__ void begin(const Tape, Mask128, const uint8_t *) {
+    ln.st.begin();
+    status = kRuns;
+  }
+  template <class Tape>
+  __host__ __device__ __forceinline__ void step(const Tape t, const Tape stk,
+                                                const uint8_t *__restrict__ optab) {
+    bool back;
+    status = ln.step(t, stk, optab, back) ? kEnds : ln.st.i >= kSteps ? kJumps : kRuns;
+  }
+  template <class Tape>
+  __host__ __device__ __forceinline__ void resolve(const Tape, const uint8_t *) {}
+  __host__ __device__ __forceinline__ const ForthState &state() const { return ln.st; }
+  __host__ __device__ __forceinline__ uint32_t ops() const { return ln.st.i - ln.st.nops; }
+  __host__ __device__ __forceinline__ uint32_t raw() const { return ln.st.i; }
+  __host__ __device__ __forceinline__ uint32_t mods() const { return ln.st.mods; }
+};
+
+// Shared memory of one warp's ForthWarp.
+struct alignas(16) ForthMem {
+  uint8_t T[kPair];      // the pair tape
+  uint8_t stk[kPair];    // the stack
+  uint8_t snap[kPair];   // their snapshots
+  uint8_t ssnap[kPair];
+  uint32_t E[kPair];     // where a run of jumps and no-ops leads (ForthWarp)
+  uint16_t R[kPair];     // lowest | highest << 8 of the positions it depends on
+};
+
+// One pair on a whole warp.
+//
+// What bounds it: the chain of dependent instructions of one program (~5
+// cycles each), and most steps of the programs that run long are jumps (44 %)
+// and no-ops (22 %), which change nothing but the position.  So all 128
+// positions are decoded at once into where the run of jumps and no-ops from
+// there leads: E[p] = q | steps << 8 | no-ops << 16 | code << 24, with q the
+// first position that holds another op (code: the op, or kConstant | value) or
+// kPair where the run leaves the tape.  The lanes find it by pointer doubling:
+// a run of up to 2^r steps is resolved after r rounds, and one not resolved
+// after 7 goes in circles (its entry then leads 128 steps ahead).  Writes only
+// widen the ranges of positions changed since; an entry is used when no
+// position it depends on (R) lies in them, else all are decoded again; a
+// program that changes its own code all the time is stepped through plainly.
+//
+// Exact cycle fast-forward where a run leads backwards, on Brent's schedule
+// (cycle.cuh): the state is (position, stack, tape); the two registers are
+// compared first, then stack and tape with their snapshots, four bytes per
+// lane.  Less will do for a segment without an if0 or a tape write ("blind"):
+// nothing it does depends on a value but other values, so back at the same
+// position and depth it repeats to the step limit whatever is on the stack;
+// and one that leaves the stack deeper by d without having met its bottom
+// repeats, d deeper each time, until the stack overflows.
+template <class W, bool kWithReset>
+struct ForthWarp {
+  static constexpr uint32_t kConstant = 64, kOut = 62, kPending = 63;  // codes
+  static constexpr uint32_t kPlainSteps = 64;
+
+  const W w;
+  ForthMem &m;
+  const uint8_t *const optab;
+  ForthLane<kWithReset> ln;
+  Written written;       // since the decode
+  uint32_t since;        // ops executed since the decode
+  // Snapshot.
+  int s_key, s_sp;
+  uint32_t s_r0, s_r1, s_i, s_nops, s_mods, s_power, s_lam;
+  // Since the snapshot: no if0 or tape write; a pop found the stack empty; the
+  // deepest stack.
+  bool blind, bottom;
+  int deepest;
+
+  __host__ __device__ __forceinline__ ForthWarp(W warp, ForthMem &mem, const uint8_t *table)
+      : w(warp), m(mem), optab(table) {}
+
+  __host__ __device__ __forceinline__ uint32_t word(const uint8_t *a, uint32_t l) const {
+    return reinterpret_cast<const uint32_t *>(a)[l];
+  }
+
+  __host__ __device__ __forceinline__ void decode() {
+    written.clear();
+    since = 0;
+    w.sync();
+    w.each([&](uint32_t l) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int p = static_cast<int>(32 * k + l);
+        const uint32_t b = m.T[p], op = optab[b];
+        int q = p;
+        uint32_t e = (op == kConst ? kConstant | (b & 63) : op) << 24;
+        if (op == kFNoop || op == kJmp) {
+          const int a = static_cast<int>(b & 63) + 1;
+          q = op == kFNoop ? p + 1 : (b & 64) ? p - a : p + a;
+          const bool out = q < 0 || q >= kPair;
+          e = (out ? kOut : kPending) << 24 | (op == kFNoop ? 1u << 16 : 0u) | 1u << 8;
+          if (out) q = kPair;
+        }
+        m.E[p] = e | static_cast<uint32_t>(q);
+        m.R[p] = static_cast<uint16_t>(p | p << 8);
+      }
+    });
+    w.sync();
+    for (int round = 0; round < 7; round++) {
+      struct Entries {
+        uint32_t e[4], r[4];
+      };
+      const auto next = w.map([&](uint32_t l) {
+        Entries x;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const uint32_t e = m.E[32 * k + l], r = m.R[32 * k + l];
+          x.e[k] = e;
+          x.r[k] = r;
+          if ((e >> 24) == kPending) {
+            const uint32_t f = m.E[e & 0xFF], g = m.R[e & 0xFF];
+            x.e[k] = f + (e & 0x00FFFF00u);
+            const uint32_t lo = (r & 0xFF) < (g & 0xFF) ? r & 0xFF : g & 0xFF;
+            const uint32_t hi = (r >> 8) > (g >> 8) ? r >> 8 : g >> 8;
+            x.r[k] = lo | hi << 8;
+          }
+        }
+        return x;
+      });
+      w.sync();
+      const bool more = w.any([&](uint32_t l) {
+        bool pending = false;
+        const Entries x = next(l);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          m.E[32 * k + l] = x.e[k];
+          m.R[32 * k + l] = static_cast<uint16_t>(x.r[k]);
+          pending |= (x.e[k] >> 24) == kPending;
+        }
+        return pending;
+      });
+      w.sync();
+      if (!more) break;
+    }
+  }
+
+  // At position `key`, which a run led back to.
+  __host__ __device__ __forceinline__ void visit(int key) {
+    ForthState &st = ln.st;
+    if (key == s_key && st.i < kStepLimit) {
+      const int deeper = st.sp - s_sp;
+      uint32_t most = 0;  // segments that may be skipped
+      if (blind) {
+        if (deeper == 0) most = kStepLimit;
+        else if (deeper > 0 && !bottom && st.sp + deepest - s_sp + deeper <= kPair)
+          most = static_cast<uint32_t>((kPair - (deepest - s_sp) - st.sp) / deeper);
+      } else if (deeper == 0 && (st.sp < 1 || st.r0 == s_r0) && (st.sp < 2 || st.r1 == s_r1)) {
+        const bool differs = w.any([&](uint32_t l) {
+          const int b = st.sp - 2 - 4 * static_cast<int>(l);  // entries in memory
+          const uint32_t use = b >= 4 ? ~0u : b <= 0 ? 0u : ~0u >> (32 - 8 * b);
+          return ((word(m.stk, l) ^ word(m.ssnap, l)) & use) != 0 ||
+                 (st.mods != s_mods && word(m.T, l) != word(m.snap, l));
+        });
+        if (!differs) most = kStepLimit;
+      }
+      if (most != 0) {
+        const uint32_t len = st.i - s_i, room = (kStepLimit - st.i) / len;
+        const uint32_t k = most < room ? most : room;
+        st.i += k * len;
+        st.nops += k * (st.nops - s_nops);
+        st.sp += static_cast<int>(k) * deeper;
+        deepest += static_cast<int>(k) * deeper;
+      }
+    }
+    if (++s_lam == s_power) {
+      s_key = key;
+      s_sp = st.sp;
+      s_r0 = st.r0;
+      s_r1 = st.r1;
+      s_i = st.i;
+      s_nops = st.nops;
+      s_mods = st.mods;
+      s_power <<= 1;
+      s_lam = 0;
+      blind = true;
+      bottom = false;
+      deepest = st.sp;
+      w.each([&](uint32_t l) {
+        reinterpret_cast<uint32_t *>(m.snap)[l] = word(m.T, l);
+        reinterpret_cast<uint32_t *>(m.ssnap)[l] = word(m.stk, l);
+      });
+    }
+  }
+
+  // The jumps and no-ops from position p up to the step limit, which comes
+  // before anything else.
+  __host__ __device__ __forceinline__ void run_out(int p) {
+    ForthState &st = ln.st;
+    while (st.i < kStepLimit) {
+      const uint32_t b = m.T[p & (kPair - 1)];
+      if (optab[b] == kFNoop) {
+        st.nops++;
+        p++;
+      } else {
+        p += (b & 64) ? -static_cast<int>(b & 63) - 1 : static_cast<int>(b & 63) + 1;
+      }
+      st.i++;
+    }
+  }
+
+  // Writes v at position a.
+  __host__ __device__ __forceinline__ void write(int a, uint32_t v) {
+    blind = false;
+    if (m.T[a] != v) {
+      m.T[a] = static_cast<uint8_t>(v);
+      ln.st.mods++;
+      written.add(a);
+    }
+  }
+  // The second register after a pop.
+  __host__ __device__ __forceinline__ void refill() {
+    if (ln.st.sp >= 2) ln.st.r1 = m.stk[ln.st.sp - 2];
+  }
+  __host__ __device__ __forceinline__ void drop() {
+    ForthState &st = ln.st;
+    bottom |= st.sp == 0;
+    if (st.sp == 0) return;
+    st.sp--;
+    st.r0 = st.r1;
+    refill();
+  }
+  __host__ __device__ __forceinline__ void push(uint32_t v) {
+    ForthState &st = ln.st;
+    if (st.sp == kPair) {
+      st.overflow = true;
+      return;
+    }
+    if (st.sp >= 2) m.stk[st.sp - 2] = static_cast<uint8_t>(st.r1);
+    st.r1 = st.r0;
+    st.r0 = v;
+    st.sp++;
+    deepest = st.sp > deepest ? st.sp : deepest;
+  }
+  // The top entry, 0 when there is none, which it then becomes.
+  __host__ __device__ __forceinline__ uint32_t top() {
+    ForthState &st = ln.st;
+    if (st.sp == 0) {
+      bottom = true;
+      st.sp = 1;
+      st.r0 = 0;
+    }
+    return st.r0;
+  }
+  // Pops two entries: v on top of a.
+  __host__ __device__ __forceinline__ void pop2(uint32_t &v, uint32_t &a) {
+    ForthState &st = ln.st;
+    bottom |= st.sp < 2;
+    v = st.sp >= 1 ? st.r0 : 0u;
+    a = st.sp >= 2 ? st.r1 : 0u;
+    if (st.sp >= 3) st.r0 = m.stk[st.sp - 3];
+    st.sp = st.sp >= 2 ? st.sp - 2 : 0;
+    refill();
+  }
+
+  // The op `code` at st.pos, as ForthLane::execute.
+  __host__ __device__ __forceinline__ void operate(uint32_t code) {
+    ForthState &st = ln.st;
+    st.pos++;
+    st.i++;
+    if (code >= kConstant) {
+      push(code & 63);
+      return;
+    }
+    switch (code) {
+      case kInc: st.r0 = (top() + 1) & 0xFF; break;
+      case kDec: st.r0 = (top() - 1) & 0xFF; break;
+      case kXor: st.r0 = top() ^ 64; break;
+      case kRead0: st.r0 = m.T[top() % kTape]; break;
+      case kRead1: st.r0 = m.T[kTape + top() % kTape]; break;
+      case kRead: st.r0 = m.T[top() % kPair]; break;
+      case kIf0:
+        blind = false;
+        st.pos += top() != 0;
+        break;
+      case kDrop: drop(); break;
+      case kDup: {
+        const uint32_t v = top();
+        push(v);
+        break;
+      }
+      case kAdd:
+      case kSub: {
+        const uint32_t a = top(), b = st.sp >= 2 ? st.r1 : 0u;
+        bottom |= st.sp < 2;
+        if (st.sp >= 2) {
+          st.sp--;
+          refill();
+        }
+        st.r0 = (code == kAdd ? a + b : a - b) & 0xFF;
+        break;
+      }
+      case kSwap: {
+        const uint32_t a = top();
+        st.r0 = st.sp >= 2 ? st.r1 : 0u;
+        st.r1 = a;
+        bottom |= st.sp < 2;
+        if (st.sp < 2) st.sp = 2;
+        break;
+      }
+      case kWrite0:
+      case kWrite1:
+      case kWrite: {
+        uint32_t v, a;
+        pop2(v, a);
+        const int p = code == kWrite ? a % kPair : code == kWrite1 ? kTape + a % kTape : a % kTape;
+        if (kWithReset && code == kWrite1 && m.T[p] == 0x13) reset();
+        else write(p, v);
+        break;
+      }
+      case kCopy: {
+        uint32_t to, from;
+        pop2(to, from);
+        write(to % kPair, m.T[from % kPair]);
+        break;
+      }
+      default: {  // kCopy0, kCopy1
+        const int a = (st.sp >= 1 ? st.r0 : 0u) % kTape;
+        drop();
+        const int to = code == kCopy0 ? kTape + a : a;
+        if (kWithReset && code == kCopy0 && m.T[to] == 0x13) reset();
+        else write(to, m.T[to ^ kTape]);
+        break;
+      }
+    }
+  }
+  __host__ __device__ __forceinline__ void reset() {
+    forth_reset(SharedBytes{m.T}, ln.st.pos - 1);
+    ln.st.mods++;
+    blind = false;
+    written.lo0 = 0;
+    written.hi0 = kTape - 1;
+  }
+
+  // Runs the program in m.T, with the stack in m.stk, from state s to its end.
+  __host__ __device__ __forceinline__ void run(const ForthState &s) {
+    ln.st = s;
+    ForthState &st = ln.st;
+    s_key = -1;
+    s_sp = 0;
+    s_r0 = s_r1 = s_i = s_nops = s_mods = s_lam = 0;
+    s_power = 1;
+    blind = bottom = false;
+    deepest = 0;
+    decode();
+    uint32_t plain = 0;  // steps to take one by one
+    int last = -1;
+    while (true) {
+      w.sync();
+      if (plain != 0) {
+        const TrackedBytes t{m.T, written};
+        bool back;
+        blind = false;  // (not tracked here)
+        if (ln.step(t, SharedBytes{m.stk}, optab, back)) return;
+        if (back) {
+          visit(st.pos);
+          if (st.i >= kStepLimit) return;
+        }
+        if (--plain == 0) decode();
+        continue;
+      }
+      const uint32_t e = m.E[st.pos], r = m.R[st.pos];
+      if (!written.none() && written.meets(static_cast<int>(r & 0xFF), static_cast<int>(r >> 8))) {
+        if (since < 8) plain = kPlainSteps;
+        else decode();
+        continue;
+      }
+      const uint32_t steps = (e >> 8) & 0xFF, code = e >> 24;
+      if (st.i + steps >= kStepLimit) {
+        run_out(st.pos);
+        return;
+      }
+      st.i += steps;
+      st.nops += (e >> 16) & 0xFF;
+      st.pos = static_cast<int>(e & 0xFF);
+      if (code == kOut) return;
+      if (code == kPending) continue;  // in circles, 128 steps at a time
+      if (st.pos <= last) {
+        visit(st.pos);
+        if (st.i >= kStepLimit) return;
+      }
+      last = st.pos;
+      since++;
+      operate(code);
+      if (st.pos >= kPair || st.overflow || st.i >= kStepLimit) return;
+    }
+  }
+
+  __host__ __device__ __forceinline__ uint32_t ops() const { return ln.st.i - ln.st.nops; }
+  __host__ __device__ __forceinline__ uint32_t raw() const { return ln.st.i; }
+  __host__ __device__ __forceinline__ uint32_t mods() const { return ln.st.mods; }
+};
+
+// The one-shot machine: ForthLane with exact cycle fast-forward at backward
+// jumps (Brent's schedule, cycle.cuh).  The state is (pos, stack pointer, stack
+// contents, tape).  The stack below the stack pointer is compared byte for
+// byte with the snapshot's (kept packed in a register, so only for stacks of
+// at most 8); the tape through a count of value-changing writes.
+template <bool kWithReset>
+struct ForthMachine : ForthLane<kWithReset> {
+  using ForthLane<kWithReset>::st;
+  // Brent-schedule snapshot taken at a backward jump.
+  int s_pos, s_sp;
+  uint32_t s_mods, s_i, s_nops, s_power, s_lam;
+  uint32_t s_top;          // stack[s_sp - 1] | stack[s_sp - 2] << 8 (0 where absent)
+  uint64_t s_mem;          // stack[0 .. s_sp - 2) packed, byte j at bits 8j (s_sp <= 8)
+
+  __host__ __device__ __forceinline__ void begin() {
+    st.begin();
+    s_pos = -1;
+    s_sp = 0;
+    s_mods = s_i = s_nops = 0;
+    s_power = 1;
+    s_lam = 0;
+    s_top = 0;
+    s_mem = 0;
+  }
+
+  // stack[0 .. sp - 2), the entries below the registers, packed.
+  __host__ __device__ __forceinline__ uint64_t pack_mem(const LaneBytes stk) const {
+    uint64_t w = 0;
+    for (int j = 0; j < st.sp - 2; j++) w |= static_cast<uint64_t>(stk.get(j)) << (8 * j);
+    return w;
+  }
+
+  // At a step boundary right after a backward jump: when the state equals
+  // the snapshot's, execution since the snapshot is periodic and whole periods
+  // are skipped (i += k * P, nops += k * the period's no-ops); the snapshot is
+  // renewed after 1, 2, 4, ... visits.  The two entries in registers are
+  // compared first: a loop's counter usually sits on top, so most visits end
+  // there without reading the stack in memory.
+  __host__ __device__ __forceinline__ void visit(const LaneBytes stk) {
+    const uint32_t top = (st.sp >= 1 ? st.r0 : 0u) | ((st.sp >= 2 ? st.r1 : 0u) << 8);
+    if (st.pos == s_pos && st.sp == s_sp && st.mods == s_mods && top == s_top &&
+        (st.sp <= 2 || pack_mem(stk) == s_mem)) {
+      const uint32_t period = st.i - s_i;
+      const uint32_t k = (kStepLimit - st.i) / period;
+      st.i += k * period;
+      st.nops += k * (st.nops - s_nops);
+    }
+    if (++s_lam == s_power) {
+      s_pos = st.sp <= 8 ? st.pos : -1;  // larger stacks: no snapshot
+      s_sp = st.sp;
+      s_mods = st.mods;
+      s_i = st.i;
+      s_nops = st.nops;
+      s_top = top;
+      s_mem = (st.sp > 2 && st.sp <= 8) ? pack_mem(stk) : 0;
+      s_power <<= 1;
+      s_lam = 0;
+    }
+  }
+  // One step; returns true when the program has ended.
+  __host__ __device__ __forceinline__ bool step(const LaneBytes t, const LaneBytes stk,
+                                                const uint8_t *__restrict__ optab) {
+    bool back;
+    if (ForthLane<kWithReset>::step(t, stk, optab, back)) return true;
     if (back) {
       visit(stk);
-      if (i >= kStepLimit) return true;
+      if (st.i >= kStepLimit) return true;
     }
     return false;
   }
-
-  __host__ __device__ __forceinline__ uint32_t ops() const { return i - nops; }
-  __host__ __device__ __forceinline__ uint32_t raw() const { return i; }
 };
 
 template <bool kWithReset>
@@ -224,8 +709,8 @@ __host__ __device__ __forceinline__ uint32_t forth_eval(const LaneBytes t, const
   m.begin();
   while (!m.step(t, stk, optab)) {
   }
-  *raw = m.raw();
-  return m.ops();
+  *raw = m.st.i;
+  return m.st.i - m.st.nops;
 }
 
 }  // namespace cubff

@@ -39,45 +39,52 @@ __host__ __device__ __forceinline__ uint32_t evaluate(const LaneBytes t, const L
   else return rsubleq4_eval(t, stk, raw);
 }
 
-// The two machines that run a BFF program in turn: on a lane, then on a warp.
-template <int L>
-struct BffMachines {
+// The two machines that run a BFF or Forth program in turn: on a lane, then on
+// a warp (with that warp's shared memory, and whether a program has a stack).
+template <int L, bool kBff = (L <= kBffSelfmove)>
+struct Stages {
   static constexpr int kLogic = (L == kBff8 || L == kBff8Noheads)
                                     ? kLogicJump8
                                     : (L == kBffSelfmove ? kLogicSelfmove : kLogicScan);
   static constexpr uint32_t kNullMask = L == kBffNoheads4bit ? 0x0Fu : 0xFFu;
-  using Lane = BffLane<(L == kBff || L == kBffPerm || L == kBff8 || L == kBffSelfmove), kLogic,
-                       kNullMask>;
+  using Lane = BffLane<(L == cubff::kBff || L == kBffPerm || L == kBff8 || L == kBffSelfmove),
+                       kLogic, kNullMask>;
   template <class W>
   using Warp = BffWarp<W, kLogic, kNullMask>;
+  using Mem = BffMem;
+  static constexpr bool kStack = false;
+};
+template <int L>
+struct Stages<L, false> {
+  using Lane = ForthFirst<(L == kForthtrivialReset)>;
+  template <class W>
+  using Warp = ForthWarp<W, (L == kForthtrivialReset)>;
+  using Mem = ForthMem;
+  static constexpr bool kStack = true;
 };
 
-// A resumable Forth or SUBLEQ interpreter of language L behind one interface:
-// begin() on a staged tape, step() until it returns true, then ops() / raw().
-template <int L, bool kBff = (L <= kBffSelfmove)>
+// A resumable SUBLEQ interpreter of language L behind one interface: begin()
+// on a staged tape, step() until it returns true, then ops() / raw().
+template <int L, bool kStaged = (L <= kForthtrivialReset)>
 struct LaneMachine {
-  using Machine =
-      std::conditional_t<LangTraits<L>::kForthFamily, ForthMachine<(L == kForthtrivialReset)>,
-                         SubleqMachine<(L == kRsubleq4)>>;
-  Machine m;
+  SubleqMachine<(L == kRsubleq4)> m;
 
   __host__ __device__ __forceinline__ void begin(const LaneBytes, Mask128) { m.begin(); }
   __host__ __device__ __forceinline__ bool step(const LaneBytes t, const LaneBytes stk,
-                                                const LaneNp,
-                                                const uint8_t *__restrict__ optab) {
-    if constexpr (LangTraits<L>::kForthFamily) return m.step(t, stk, optab);
-    else return m.step(t, stk);
+                                                const LaneNp, const uint8_t *) {
+    return m.step(t, stk);
   }
   __host__ __device__ __forceinline__ uint32_t ops() const { return m.ops(); }
   __host__ __device__ __forceinline__ uint32_t raw() const { return m.raw(); }
   __host__ __device__ __forceinline__ uint32_t mods() const { return m.mods; }
 };
 
-// The same interface over the BFF machines, on the host: a step of the lane's,
-// or all of the warp's.
+// The same interface over the two stages, on the host: a step of the lane's, or
+// all of the warp's.
 template <int L>
 struct LaneMachine<L, true> {
-  typename BffMachines<L>::Lane lane;
+  using Lane = typename Stages<L>::Lane;
+  Lane lane;
   Mask128 cmd;
   bool begun;
   uint32_t n, i;
@@ -87,21 +94,23 @@ struct LaneMachine<L, true> {
     begun = false;
     n = i = 0;
   }
-  bool step(const LaneBytes t, const LaneBytes, const LaneNp, const uint8_t *optab) {
-    using Lane = typename BffMachines<L>::Lane;
+  bool step(const LaneBytes t, const LaneBytes stk, const LaneNp, const uint8_t *optab) {
     if (!begun) lane.begin(t, cmd, optab);
-    else lane.step(t, optab);
+    else lane.step(t, stk, optab);
     begun = true;
     if (lane.status == Lane::kJumps) lane.resolve(t, optab);
-    n = lane.st.n;
-    i = lane.st.i;
+    n = lane.ops();
+    i = lane.raw();
     if (lane.status == Lane::kJumps) {
-      BffMem mem;
-      for (int p = 0; p < kPair; p++) mem.T[p] = static_cast<uint8_t>(t.get(p));
-      typename BffMachines<L>::template Warp<HostWarp> warp(HostWarp{}, mem, optab);
-      warp.run(lane.st);
+      typename Stages<L>::Mem mem;
+      for (int p = 0; p < kPair; p++) {
+        mem.T[p] = static_cast<uint8_t>(t.get(p));
+        if constexpr (Stages<L>::kStack) mem.stk[p] = static_cast<uint8_t>(stk.get(p));
+      }
+      typename Stages<L>::template Warp<HostWarp> warp(HostWarp{}, mem, optab);
+      warp.run(lane.state());
       for (int p = 0; p < kPair; p++) t.set(p, mem.T[p]);
-      n = warp.st.n;
+      n = warp.ops();
       i = warp.raw();
       return true;
     }

@@ -89,7 +89,7 @@ constexpr int kCountSlots = kPipeCountSlots;  // per-epoch counter slots (spread
 // and `exhausted` once a claim falls past the queue's last task.
 //
 // How a warp runs its pairs depends on the language family (LaneServer,
-// BffServer).  Launch-shape knobs (PipeTuning, chosen by the host; the BFF
+// StagedServer).  Launch-shape knobs (PipeTuning, chosen by the host; the BFF
 // family runs a pair to its end and uses only the grid size):
 //  * steps_per_visit: interpreter steps a running lane takes per iteration of
 //    its warp after its first (an iteration lasts as long as its busiest
@@ -338,7 +338,7 @@ __device__ __forceinline__ void push_ready(const PipeCtx &b, const PipeQueue &q,
   if (ln.state == kNotify) ln.state = kIdle;
 }
 
-// The Forth and SUBLEQ languages: one pair per lane.  iterate() is one
+// The SUBLEQ languages: one pair per lane.  iterate() is one
 // iteration of the warp; it returns true if the lane made progress.
 template <int L>
 struct LaneServer {
@@ -431,30 +431,57 @@ struct LaneServer {
   }
 };
 
-// The BFF family.  The lanes of a warp run the forward part of a pair each
-// (BffLane): most random programs end there, and those pairs are written back
-// and their consumers notified at once.  The pairs that jump are kept (kLong)
-// and run one after the other on the whole warp (BffWarp), one per iteration,
-// so that slots held by other lanes are still polled in between.  So that
+// The BFF and Forth families.  The lanes of a warp run the first part of a
+// pair each (BFF: up to the first jump; Forth: a few steps): most random
+// programs end there, and those pairs are written back and their consumers
+// notified at once.  The pairs that go on are kept (kLong) and run one after the
+// other on the whole warp, one per iteration, so that slots held by other lanes are still polled in between.  So that
 // pairs wait behind few others, a warp holds 8 and there are many warps: a soup
 // of 2^17 bff programs taken over by self-replicators takes 35.4 ms for 16
 // epochs with 8 (32 lanes: 76.9, 16: 44.6), one of 1022 bff_noheads programs
 // 2.1 ms for 64 (4.3, 3.0); only the 20 first epochs of a random soup of 2^17
 // are a little faster with 32 (3.07 ms, 8: 3.27).
+__device__ __forceinline__ BffState broadcast(const BffState &s, uint32_t src) {
+  constexpr uint32_t kAll = 0xffffffffu;
+  BffState r;
+  r.q = __shfl_sync(kAll, s.q, src);
+  r.h0 = __shfl_sync(kAll, s.h0, src);
+  r.h1 = __shfl_sync(kAll, s.h1, src);
+  r.i = __shfl_sync(kAll, s.i, src);
+  r.n = __shfl_sync(kAll, s.n, src);
+  r.mods = __shfl_sync(kAll, s.mods, src);
+  return r;
+}
+__device__ __forceinline__ ForthState broadcast(const ForthState &s, uint32_t src) {
+  constexpr uint32_t kAll = 0xffffffffu;
+  ForthState r;
+  r.begin();
+  r.pos = __shfl_sync(kAll, s.pos, src);
+  r.sp = __shfl_sync(kAll, s.sp, src);
+  r.r0 = __shfl_sync(kAll, s.r0, src);
+  r.r1 = __shfl_sync(kAll, s.r1, src);
+  r.i = __shfl_sync(kAll, s.i, src);
+  r.nops = __shfl_sync(kAll, s.nops, src);
+  r.mods = __shfl_sync(kAll, s.mods, src);
+  return r;
+}
+
 template <int L>
-struct BffServer {
-  using LaneM = typename BffMachines<L>::Lane;
-  using WarpM = typename BffMachines<L>::template Warp<DeviceWarp>;
+struct StagedServer {
+  using LaneM = typename Stages<L>::Lane;
+  using WarpM = typename Stages<L>::template Warp<DeviceWarp>;
+  using Mem = typename Stages<L>::Mem;
   static constexpr uint32_t kWidth = 8;  // lanes that hold pairs
-  static constexpr size_t kTapes = kWidth * kPair, kWarpBytes = kTapes + sizeof(BffMem);
+  static constexpr size_t kTapes = kWidth * kPair, kStacks = Stages<L>::kStack ? kTapes : 0,
+                          kWarpBytes = kTapes + kStacks + sizeof(Mem);
   LaneM m;
-  LaneWords<kWidth> t;
-  BffMem &mem;
+  LaneWords<kWidth> t, stk;
+  Mem &mem;
   const uint8_t *optab, *cmdflag;
 
-  __device__ __forceinline__ BffServer(uint8_t *smem, const uint8_t *tables, uint32_t tid)
-      : t{smem + (tid >> 5) * kWarpBytes, tid & 31},
-        mem(*reinterpret_cast<BffMem *>(smem + (tid >> 5) * kWarpBytes + kTapes)),
+  __device__ __forceinline__ StagedServer(uint8_t *smem, const uint8_t *tables, uint32_t tid)
+      : t{smem + (tid >> 5) * kWarpBytes, tid & 31}, stk{t.s + kStacks, tid & 31},
+        mem(*reinterpret_cast<Mem *>(smem + (tid >> 5) * kWarpBytes + kTapes + kStacks)),
         optab(tables), cmdflag(tables + 256) {
     m.status = LaneM::kEnds;
   }
@@ -477,6 +504,7 @@ struct BffServer {
       const uint32_t w = qd % 4 == 0 ? g[qd / 4].x : qd % 4 == 1 ? g[qd / 4].y
                        : qd % 4 == 2 ? g[qd / 4].z : g[qd / 4].w;
       t.word(qd) = w;
+      if (L > kBffSelfmove) continue;
       const uint32_t f = cmdflag[w & 0xFF] | (cmdflag[(w >> 8) & 0xFF] << 8) |
                          (cmdflag[(w >> 16) & 0xFF] << 16) | (cmdflag[w >> 24] << 24);
       const uint64_t nib = (f * 0x01020408u) >> 24;
@@ -487,7 +515,7 @@ struct BffServer {
     if (ln.dirty) {
       mutate_bits(sp, ln, mm, [&](int i, uint32_t v) {
         t.set(i, v);
-        mask_assign(cmd, i, cmdflag[v] != 0);
+        if (L <= kBffSelfmove) mask_assign(cmd, i, cmdflag[v] != 0);
       });
     }
     const uint64_t num_indices = sp.num_indices ? sp.num_indices[ln.e] : sp.npairs;
@@ -501,22 +529,19 @@ struct BffServer {
   __device__ __forceinline__ void run_long(const PipeCtx &b, Lane &ln, uint32_t src,
                                            uint32_t lane, uint32_t slot_ctr) {
     constexpr uint32_t kAll = 0xffffffffu;
-    BffState st;
-    st.q = __shfl_sync(kAll, m.st.q, src);
-    st.h0 = __shfl_sync(kAll, m.st.h0, src);
-    st.h1 = __shfl_sync(kAll, m.st.h1, src);
-    st.i = __shfl_sync(kAll, m.st.i, src);
-    st.n = __shfl_sync(kAll, m.st.n, src);
-    st.mods = __shfl_sync(kAll, m.st.mods, src);
+    const auto st = broadcast(m.state(), src);
     __syncwarp();  // the lane's tape
     uint32_t *T = reinterpret_cast<uint32_t *>(mem.T);
     T[lane] = reinterpret_cast<const uint32_t *>(t.s)[lane * kWidth + src];
+    if constexpr (Stages<L>::kStack)
+      reinterpret_cast<uint32_t *>(mem.stk)[lane] =
+          reinterpret_cast<const uint32_t *>(stk.s)[lane * kWidth + src];
     __syncwarp();
     WarpM wm(DeviceWarp{lane}, mem, optab);
     wm.run(st);
     __syncwarp();
     const PipeSoup &sp = b.soups[__shfl_sync(kAll, ln.si, src)];
-    if (wm.st.mods != 0 || __shfl_sync(kAll, ln.dirty, src)) {
+    if (wm.mods() != 0 || __shfl_sync(kAll, ln.dirty, src)) {
       const uint32_t p1 = __shfl_sync(kAll, ln.p1, src), p2 = __shfl_sync(kAll, ln.p2, src);
       // First half, then second half (common_language.h:188-191): of a
       // program paired with itself the second half stays.
@@ -525,7 +550,7 @@ struct BffServer {
             T[lane];
     }
     __syncwarp();  // the warp's stores before the lane's notifications
-    if (lane == src) finish(sp, ln, slot_ctr, wm.st.n, wm.raw());
+    if (lane == src) finish(sp, ln, slot_ctr, wm.ops(), wm.raw());
   }
 
   __device__ __forceinline__ bool iterate(const PipeCtx &b, const PipeQueue &q, Lane &ln,
@@ -556,7 +581,7 @@ struct BffServer {
     while (true) {
       const bool go = ln.state == kRun && m.status == LaneM::kRuns;
       if (!__any_sync(0xffffffffu, go)) break;
-      if (go) m.step(t, optab);
+      if (go) m.step(t, stk, optab);
     }
     // 5. Pairs that ended: write back and notify.
     if (ln.state == kRun) {
@@ -565,9 +590,9 @@ struct BffServer {
         ln.state = kLong;
       } else {
         const PipeSoup &sp = b.soups[ln.si];
-        if (ln.dirty || (ln.evaluated && m.st.mods != 0))
+        if (ln.dirty || (ln.evaluated && m.mods() != 0))
           store_pair(sp, ln, [&](int qd) { return t.word(qd); });
-        finish(sp, ln, slot_ctr, m.st.n, m.st.i);
+        finish(sp, ln, slot_ctr, m.ops(), m.raw());
       }
     }
     // 6. Push the consumers whose second input this pair was.
@@ -577,7 +602,7 @@ struct BffServer {
 };
 
 template <int L>
-using Server = std::conditional_t<(L <= kBffSelfmove), BffServer<L>, LaneServer<L>>;
+using Server = std::conditional_t<(L <= kForthtrivialReset), StagedServer<L>, LaneServer<L>>;
 
 // Shared memory of a pipelined launch: the servers' (tapes and so on), the op
 // and command tables, then the soup descriptors.
@@ -596,7 +621,7 @@ size_t pipeline_smem_bytes(int n_soups) {
 // spills that matter (6 blocks, 80 registers: 39.9 ms instead of 35.1 on the
 // self-replicators above), the lanes' shared memory allows the others 4.
 template <int L>
-__global__ void __launch_bounds__(kThreads, (L <= kBffSelfmove) ? 5 : 4)
+__global__ void __launch_bounds__(kThreads, (L <= kForthtrivialReset) ? 5 : 4)
     pipeline_kernel(const __grid_constant__ PipeBatch pb) {
   extern __shared__ __align__(16) uint8_t smem[];
   uint8_t *tables = smem + server_bytes<L>();
