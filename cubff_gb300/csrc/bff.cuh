@@ -6,11 +6,10 @@
 // bff_selfmove (bff_selfmove.cu:47-98).  The op of a byte comes from the
 // language's table (optab, BffOp values).
 //
-// Three machines with the same results:
+// Two machines that a program runs on in turn:
 //  * BffLane, one pair per lane: runs a program until it ends or first jumps
 //    (most random programs never do);
-//  * BffWarp, one pair per warp, which takes over from there;
-//  * BffBasic, the one-shot one of the per-epoch kernels (bff_eval).
+//  * BffWarp, one pair per warp, which takes over from there.
 #pragma once
 
 #include "coop.cuh"
@@ -734,8 +733,23 @@ struct BffWarp {
     }
   }
 
-  // Runs the program in m.T from state s (at a command) to its end; st.n and
-  // raw() are then the op and raw step counts.
+  // The state at the start of the program in m.T: at its first command.
+  __host__ __device__ __forceinline__ BffState start(bool heads) const {
+    const int pc = heads ? 2 : 0;
+    int q = kPair;
+#pragma unroll
+    for (int k = 3; k >= 0; k--) {
+      const uint32_t cmd = w.ballot([&](uint32_t l) {
+        return static_cast<int>(32 * k + l) >= pc && optab[m.T[32 * k + l]] < kNull;
+      });
+      if (cmd) q = 32 * k + low32(cmd);
+    }
+    return {q, heads ? m.T[0] & (kPair - 1) : 0, heads ? m.T[1] & (kPair - 1) : 0,
+            static_cast<uint32_t>(q - pc), 0, 0};
+  }
+
+  // Runs the program in m.T from state s (at a command) to its end; ops() and
+  // raw() are then its op and raw step counts.
   __host__ __device__ __forceinline__ void run(const BffState &s) {
     st = s;
     used1 = true;
@@ -751,6 +765,7 @@ struct BffWarp {
     dhi = kPair - 1;  // nothing is decoded yet
     v0 = m.T[st.h0];
     v1 = m.T[st.h1];
+    if (st.q >= kPair) return;
     int from = kRedo, next = 0;
     bool back = false;
     while (true) {
@@ -793,240 +808,5 @@ struct BffWarp {
     return st.i < kStepLimit ? st.i : kStepLimit;
   }
 };
-
-// The one-shot machine.  Work per step is reduced without changing results:
-//  * a 128-bit mask marks command bytes; runs of no-op bytes are crossed in
-//    one step of the machine: the reference counts each as a step and a skip,
-//    so i and nskip advance by the run length (cut at the step limit; a run
-//    reaching the tape end ends the program);
-//  * '[' / ']' masks (built on the first loop command) let bracket matching
-//    walk only bracket positions;
-//  * masks are patched on writes that change a byte's op;
-//  * exact cycle fast-forward at backward jumps, as above; tape equality with
-//    the snapshot is checked on the positions written since (the first write
-//    to a position saves its snapshot value in a second per-lane area).
-template <bool kHeads, int kLogic, uint32_t kNullMask>
-struct BffBasic {
-  int pc, h0, h1;
-  uint32_t i, nskip, mods;
-  bool have_brk;
-  bool used0, used1;  // heads used as addresses since the snapshot
-  Mask128 cmd, opn, cls;
-  Mask128 touched;    // positions written since the snapshot
-  // Brent-schedule snapshot taken at a backward jump.
-  int s_pc, s_h0, s_h1;
-  uint32_t s_mods, s_i, s_skip, s_power, s_lam;
-
-  // cmd_mask: bit p set iff tape byte p is a command (op < kNull).
-  __host__ __device__ __forceinline__ void begin(const LaneBytes t, Mask128 cmd_mask) {
-    cmd = cmd_mask;
-    have_brk = false;
-    if (kHeads) {
-      h0 = t.get(0) & (kPair - 1);
-      h1 = t.get(1) & (kPair - 1);
-      pc = 2;
-    } else {
-      h0 = h1 = 0;  // 2 * kSingleTapeSize, masked to 0 at the first step
-      pc = 0;
-    }
-    i = nskip = mods = 0;
-    used0 = used1 = false;
-    touched = Mask128{0, 0};
-    s_pc = -1;
-    s_h0 = s_h1 = 0;
-    s_mods = s_i = s_skip = 0;
-    s_power = 1;
-    s_lam = 0;
-  }
-
-  // True when every position written since the snapshot holds its snapshot
-  // value again (saved in snapa by the first write).
-  __host__ __device__ __forceinline__ bool tape_back(const LaneBytes t, const LaneBytes snapa) const {
-    if (mods == s_mods) return true;
-    uint64_t lo = touched.lo, hi = touched.hi;
-    while (lo) {
-      const int p = ffs64(lo) - 1;
-      lo &= lo - 1;
-      if (t.get(p) != snapa.get(p)) return false;
-    }
-    while (hi) {
-      const int p = 63 + ffs64(hi);
-      hi &= hi - 1;
-      if (t.get(p) != snapa.get(p)) return false;
-    }
-    return true;
-  }
-
-  // At a step boundary right after a backward jump.
-  __host__ __device__ __forceinline__ void visit(const LaneBytes t, const LaneBytes snapa) {
-    if (pc == s_pc && (!used0 || h0 == s_h0) && (!used1 || h1 == s_h1) && tape_back(t, snapa)) {
-      const uint32_t period = i - s_i;
-      const uint32_t k = (kStepLimit - i) / period;
-      i += k * period;
-      nskip += k * (nskip - s_skip);
-      h0 = (h0 + static_cast<int>(k) * (h0 - s_h0)) & (kPair - 1);
-      h1 = (h1 + static_cast<int>(k) * (h1 - s_h1)) & (kPair - 1);
-    }
-    if (++s_lam == s_power) {
-      s_pc = pc;
-      s_h0 = h0;
-      s_h1 = h1;
-      s_mods = mods;
-      s_i = i;
-      s_skip = nskip;
-      s_power <<= 1;
-      s_lam = 0;
-      used0 = used1 = false;
-      touched = Mask128{0, 0};
-    }
-  }
-
-  __host__ __device__ __forceinline__ void build_brackets(const LaneBytes t,
-                                                          const uint8_t *__restrict__ optab) {
-    opn = Mask128{0, 0};
-    cls = Mask128{0, 0};
-    for (int p = 0; p < kPair; p++) {
-      if (!mask_test(cmd, p)) continue;
-      const uint32_t c = optab[t.get(p)];
-      if (c == kLoopStart) mask_assign(opn, p, true);
-      if (c == kLoopEnd) mask_assign(cls, p, true);
-    }
-    have_brk = true;
-  }
-
-  // Writes tape[a] = v (old value o); patches the masks when the op changes.
-  __host__ __device__ __forceinline__ void write(const LaneBytes t, const LaneBytes snapa,
-                                                 const uint8_t *__restrict__ optab, int a,
-                                                 uint32_t o, uint32_t v) {
-    v &= 0xFF;
-    if (v == o) return;
-    t.set(a, v);
-    mods++;
-    if (!mask_test(touched, a)) {
-      mask_assign(touched, a, true);
-      snapa.set(a, o);
-    }
-    const uint32_t co = optab[o], cn = optab[v];
-    if (co != cn) {
-      mask_assign(cmd, a, cn < kNull);
-      if (have_brk) {
-        mask_assign(opn, a, cn == kLoopStart);
-        mask_assign(cls, a, cn == kLoopEnd);
-      }
-    }
-  }
-
-  // A run of no-ops (if any) and then one command.  Returns true
-  // when the program has ended; the op count is then i - nskip.
-  __host__ __device__ __forceinline__ bool step(const LaneBytes t, const LaneBytes snapa,
-                                                      const uint8_t *__restrict__ optab) {
-    const int q = mask_next(cmd, pc);
-    const uint32_t run = static_cast<uint32_t>(q - pc);
-    if (run) {
-      if (i + run >= kStepLimit) {
-        nskip += kStepLimit - i;
-        i = kStepLimit;
-        return true;
-      }
-      i += run;
-      nskip += run;
-      pc = q;
-      if (pc >= kPair) return true;
-    }
-    const uint32_t c = optab[t.get(pc)];
-    bool back = false;
-    switch (c) {
-      case kDec0: h0 = (h0 - 1) & (kPair - 1); break;
-      case kInc0: h0 = (h0 + 1) & (kPair - 1); break;
-      case kDec1: h1 = (h1 - 1) & (kPair - 1); break;
-      case kInc1: h1 = (h1 + 1) & (kPair - 1); break;
-      case kPlus: { used0 = true; const uint32_t o = t.get(h0); write(t, snapa, optab, h0, o, o + 1); break; }
-      case kMinus: { used0 = true; const uint32_t o = t.get(h0); write(t, snapa, optab, h0, o, o - 1); break; }
-      case kCopy01:
-        used0 = used1 = true;
-        write(t, snapa, optab, h1, t.get(h1), t.get(h0));
-        break;
-      case kCopy10:
-        used0 = used1 = true;
-        write(t, snapa, optab, h0, t.get(h0), t.get(h1));
-        if (kLogic == kLogicSelfmove) h1 = (h1 + 1) & (kPair - 1);
-        break;
-      case kLoopStart:
-        used0 = true;
-        if ((t.get(h0) & kNullMask) == 0) {
-          if (kLogic == kLogicJump8) {
-            pc += 8;
-          } else {
-            if (!have_brk) build_brackets(t, optab);
-            const Mask128 brk{opn.lo | cls.lo, opn.hi | cls.hi};
-            int depth = 1, p = pc + 1;
-            while (true) {
-              const int b = mask_next(brk, p);
-              if (b >= kPair) { pc = kPair; break; }
-              depth += mask_test(opn, b) ? 1 : -1;
-              if (depth == 0) { pc = b; break; }
-              p = b + 1;
-            }
-          }
-        }
-        break;
-      case kLoopEnd:
-        used0 = true;
-        if ((t.get(h0) & kNullMask) != 0) {
-          back = true;
-          if (kLogic == kLogicJump8) {
-            pc -= 8;
-          } else {
-            if (!have_brk) build_brackets(t, optab);
-            const Mask128 brk{opn.lo | cls.lo, opn.hi | cls.hi};
-            int depth = 1, p = pc - 1;
-            while (true) {
-              const int b = mask_prev(brk, p);
-              if (b < 0) { pc = -1; break; }
-              depth += mask_test(cls, b) ? 1 : -1;
-              if (depth == 0) { pc = b; break; }
-              p = b - 1;
-            }
-          }
-        }
-        break;
-      default:  // only command bytes reach here
-        break;
-    }
-    i++;
-    if (pc < 0) return true;
-    pc++;
-    if (pc >= kPair || i >= kStepLimit) return true;
-    if (back) {
-      visit(t, snapa);
-      if (i >= kStepLimit) return true;
-    }
-    return false;
-  }
-
-  __host__ __device__ __forceinline__ uint32_t ops() const { return i - nskip; }
-  __host__ __device__ __forceinline__ uint32_t raw() const { return i; }
-};
-
-// Command mask of a staged tape (bit p set iff optab[tape[p]] < kNull).
-__host__ __device__ __forceinline__ Mask128 bff_command_mask(const LaneBytes t,
-                                                             const uint8_t *__restrict__ optab) {
-  Mask128 m{0, 0};
-  for (int p = 0; p < kPair; p++) mask_assign(m, p, optab[t.get(p)] < kNull);
-  return m;
-}
-
-// snapa: a second per-lane 128-byte area (snapshot values for the cycle check).
-template <bool kHeads, int kLogic, uint32_t kNullMask>
-__host__ __device__ __forceinline__ uint32_t bff_eval(const LaneBytes t, const LaneBytes snapa,
-                                                      const uint8_t *__restrict__ optab,
-                                                      uint32_t *raw) {
-  BffBasic<kHeads, kLogic, kNullMask> m;
-  m.begin(t, bff_command_mask(t, optab));
-  while (!m.step(t, snapa, optab)) {
-  }
-  *raw = m.raw();
-  return m.ops();
-}
 
 }  // namespace cubff

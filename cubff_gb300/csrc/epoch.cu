@@ -1,15 +1,10 @@
 // epoch.cu — the fused epoch kernel (gather -> mutate -> run -> split -> count)
-// and the soup-init and self-replication kernels, for all 13 languages.
+// and the soup-init, self-replication and histogram kernels, for all 13
+// languages.
 //
-// One thread owns one pair.  Its two 64-byte programs are read from HBM with
-// 16-byte loads, the 128 per-byte mutation draws of the reference
-// (common_language.h:172-180) are applied in registers, and the 128-byte pair
-// tape is staged in shared memory in the bank-per-lane layout of common.cuh, so
-// the interpreter's data-dependent byte accesses never bank-conflict.  The
-// op count is reduced per warp (redux) and added with one atomic per warp, as
-// IncreaseInsnCount does (common_language.h:56-63).
+// The op count is reduced per warp (redux) and added with one atomic per warp,
+// as IncreaseInsnCount does (common_language.h:56-63).
 #include <algorithm>
-#include <atomic>
 #include "internal.h"
 #include "epoch_body.cuh"
 
@@ -38,59 +33,128 @@ __global__ void init_kernel(uint8_t *soup, uint64_t n, uint64_t key, int zero_in
 }
 
 // CheckSelfRep (common_language.h:203-277): per program, 13 noise partners
-// x (1 + 4) generations, then the byte-stability vote.  One thread per
-// program, its working tape in the shared-memory layout, its 13 final tapes
-// in thread-local memory.
+// x (1 + 4) generations, then the byte-stability vote.
+constexpr int kIters = 13, kGens = 4;
+
+// Byte j of noise partner `it`.
+__device__ __forceinline__ uint32_t noise(uint64_t local_seed, int it, uint32_t j) {
+  return static_cast<uint32_t>(
+             splitmix64(local_seed ^ splitmix64(uint64_t(it + 1) * kTape + j))) & 0xFF;
+}
+
+// Whether position i of the 13 final tapes counts for the program.
+__device__ __forceinline__ bool stable(const uint8_t (*fin)[kPair], const uint8_t *prog, int i) {
+  for (int x = 0; x < kIters; x++) {
+    if (i < kTape && fin[x][i] != prog[i]) continue;
+    uint32_t cnt = 1;
+    for (int y = x + 1; y < kIters; y++) cnt += fin[x][i] == fin[y][i];
+    if (cnt > kIters / 4) return true;
+  }
+  return false;
+}
+
+// SUBLEQ: one thread per program, its working tape in the shared-memory
+// layout, its 13 final tapes in thread-local memory.
 template <int L>
 __global__ void __launch_bounds__(kThreads) selfrep_kernel(const uint8_t *soup,
                                                            uint64_t epoch_key,
                                                            uint64_t n, uint64_t count,
                                                            uint64_t *result) {
   extern __shared__ __align__(16) uint8_t smem[];
-  uint8_t *optab = smem + 2 * kGroups * kGroupBytes;
   const uint32_t tid = threadIdx.x;
-  if (LangTraits<L>::kNeedsTable)
-    for (uint32_t c = tid; c < 256; c += kThreads) optab[c] = op_of(L, c);
-  __syncthreads();
   const uint64_t index = uint64_t(blockIdx.x) * kThreads + tid;
   if (index >= count) return;
   const LaneBytes t{smem, lane_base(tid)};
   const LaneBytes stk{smem + kGroups * kGroupBytes, lane_base(tid)};
-  constexpr int kIters = 13, kGens = 4;
   uint8_t fin[kIters][kPair];
   const uint8_t *prog = soup + index * kTape;
   const uint64_t local_seed = splitmix64(n * epoch_key + index);
   for (int it = 0; it < kIters; it++) {
-    for (int j = 0; j < kTape; j++) {
-      t.set(j, prog[j]);
-      t.set(kTape + j, static_cast<uint32_t>(
-                           splitmix64(local_seed ^ splitmix64(uint64_t(it + 1) * kTape + j))));
-    }
-    uint32_t raw;
-    evaluate<L>(t, stk, optab, &raw);
-    for (int g = 0; g < kGens; g++) {
+    for (int g = 0; g <= kGens; g++) {
       for (int j = 0; j < kTape; j++) {
-        t.set(j, t.get(kTape + j));
-        t.set(kTape + j, static_cast<uint32_t>(splitmix64(
-                             local_seed ^ splitmix64(uint64_t(it + 1) * kTape + j))));
+        t.set(j, g == 0 ? prog[j] : t.get(kTape + j));
+        t.set(kTape + j, noise(local_seed, it, j));
       }
-      evaluate<L>(t, stk, optab, &raw);
+      uint32_t raw;
+      evaluate<L>(t, stk, nullptr, &raw);
     }
     for (int j = 0; j < kPair; j++) fin[it][j] = static_cast<uint8_t>(t.get(j));
   }
   uint64_t res[2] = {0, 0};
-  for (int i = 0; i < kPair; i++) {
-    for (int x = 0; x < kIters; x++) {
-      if (i < kTape && fin[x][i] != prog[i]) continue;
-      uint32_t cnt = 1;
-      for (int y = x + 1; y < kIters; y++) cnt += fin[x][i] == fin[y][i];
-      if (cnt > kIters / 4) {
-        res[i / kTape]++;
-        break;
-      }
-    }
-  }
+  for (int i = 0; i < kPair; i++) res[i / kTape] += stable(fin, prog, i);
   result[index] = res[0] < res[1] ? res[0] : res[1];
+}
+
+// The staged languages.  The 13 chains of 5 evaluations of a program are
+// independent, and a chain of a self-replicator takes a whole warp some 0.2 ms;
+// so a block takes kScored programs, its warps claim their chains one by one and
+// keep the final tapes in shared memory, and all threads vote, one position
+// each.  (One thread per program, 65 evaluations in a row, had a warp wait for
+// the slowest of its 32 programs 65 times: 103 ms for a soup of 2^14 bff
+// programs with self-replicators about; now 35.)
+constexpr int kScored = 4;
+
+template <int L>
+struct ScoreMem {
+  typename Stages<L>::Mem warps[kThreads / 32];
+  uint8_t fin[kScored][kIters][kPair];
+  uint8_t prog[kScored][kTape];
+  uint32_t votes[kScored][2];
+  uint32_t claimed;
+  uint8_t tables[512];
+};
+
+template <int L>
+__global__ void __launch_bounds__(kThreads, 5) staged_selfrep_kernel(const uint8_t *soup,
+                                                                     uint64_t epoch_key,
+                                                                     uint64_t n, uint64_t count,
+                                                                     uint64_t *result) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  ScoreMem<L> &sm = *reinterpret_cast<ScoreMem<L> *>(smem);
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  const uint64_t first = uint64_t(blockIdx.x) * kScored;
+  const uint32_t programs = static_cast<uint32_t>(count - first < kScored ? count - first : kScored);
+  fill_tables<L>(sm.tables);
+  for (uint32_t b = tid; b < programs * kTape; b += kThreads)
+    sm.prog[0][b] = soup[first * kTape + b];
+  if (tid < 2 * kScored) sm.votes[0][tid] = 0;
+  if (tid == 0) sm.claimed = 0;
+  __syncthreads();
+  typename Stages<L>::Mem &mem = sm.warps[tid >> 5];
+  while (true) {
+    uint32_t chain = 0;
+    if (lane == 0) chain = atomicAdd(&sm.claimed, 1u);
+    chain = __shfl_sync(0xffffffffu, chain, 0);
+    if (chain >= programs * kIters) break;
+    const uint32_t p = chain / kIters, it = chain % kIters;
+    const uint64_t local_seed = splitmix64(n * epoch_key + first + p);
+    const uint32_t n0 = noise(local_seed, it, lane), n1 = noise(local_seed, it, 32 + lane);
+    for (int g = 0; g <= kGens; g++) {
+      const uint8_t *from = g == 0 ? sm.prog[p] : mem.T + kTape;
+      const uint8_t b0 = from[lane], b1 = from[32 + lane];
+      __syncwarp();
+      mem.T[lane] = b0;
+      mem.T[32 + lane] = b1;
+      mem.T[kTape + lane] = static_cast<uint8_t>(n0);
+      mem.T[kTape + 32 + lane] = static_cast<uint8_t>(n1);
+      __syncwarp();
+      typename Stages<L>::template Warp<DeviceWarp> wm(DeviceWarp{lane}, mem, sm.tables);
+      wm.run(wm.start(L == kBff || L == kBffPerm || L == kBff8 || L == kBffSelfmove));
+      __syncwarp();
+    }
+    reinterpret_cast<uint32_t *>(sm.fin[p][it])[lane] =
+        reinterpret_cast<const uint32_t *>(mem.T)[lane];
+    __syncwarp();
+  }
+  __syncthreads();
+  for (uint32_t p = 0; p < programs; p++)
+    if (stable(sm.fin[p], sm.prog[p], static_cast<int>(tid)))
+      atomicAdd(&sm.votes[p][tid / kTape], 1u);
+  __syncthreads();
+  if (tid < programs) {
+    const uint32_t a = sm.votes[tid][0], b = sm.votes[tid][1];
+    result[first + tid] = a < b ? a : b;
+  }
 }
 
 template <int L>
@@ -98,15 +162,14 @@ int launch_epoch_t(const EpochArgs &a, cudaStream_t stream) {
   const uint64_t npairs = a.n / 2;
   if (npairs == 0) return CUBFF_OK;
   const size_t smem = epoch_smem_bytes<L>();
-  static std::atomic<bool> attr_set{false};  // per process; setting it twice is harmless
-  if (!attr_set.load()) {
-    CUBFF_CUDA_TRY(cudaFuncSetAttribute(epoch_kernel<L>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(smem)));
-    attr_set.store(true);
+  if constexpr (LangTraits<L>::kStaged) {
+    const uint64_t per_block = kThreads / 32 * StagedMem<L>::kWidth;
+    staged_epoch_kernel<L><<<static_cast<unsigned>((npairs + per_block - 1) / per_block), kThreads,
+                             smem, stream>>>(a);
+  } else {
+    epoch_kernel<L><<<static_cast<unsigned>((npairs + kThreads - 1) / kThreads), kThreads, smem,
+                      stream>>>(a);
   }
-  const uint64_t grid = (npairs + kThreads - 1) / kThreads;
-  epoch_kernel<L><<<static_cast<unsigned>(grid), kThreads, smem, stream>>>(a);
   CUBFF_CUDA_TRY(cudaGetLastError());
   return CUBFF_OK;
 }
@@ -115,10 +178,13 @@ template <int L>
 int launch_selfrep_t(const uint8_t *soup, uint64_t epoch_key, uint64_t n,
                      uint64_t count, uint64_t *result, cudaStream_t stream) {
   if (count == 0) return CUBFF_OK;
-  const size_t smem = epoch_smem_bytes<L>();
-  const uint64_t grid = (count + kThreads - 1) / kThreads;
-  selfrep_kernel<L><<<static_cast<unsigned>(grid), kThreads, smem, stream>>>(
-      soup, epoch_key, n, count, result);
+  if constexpr (LangTraits<L>::kStaged) {
+    staged_selfrep_kernel<L><<<static_cast<unsigned>((count + kScored - 1) / kScored), kThreads,
+                               sizeof(ScoreMem<L>), stream>>>(soup, epoch_key, n, count, result);
+  } else {
+    selfrep_kernel<L><<<static_cast<unsigned>((count + kThreads - 1) / kThreads), kThreads,
+                        epoch_smem_bytes<L>(), stream>>>(soup, epoch_key, n, count, result);
+  }
   CUBFF_CUDA_TRY(cudaGetLastError());
   return CUBFF_OK;
 }

@@ -1,23 +1,23 @@
-// epoch_body.cuh — the per-CTA body of one epoch of one soup
-// (MutateAndRunPrograms, common_language.h:157-193), shared by the
-// single-soup kernel and the batched multi-soup kernel.
+// epoch_body.cuh — the kernels of one epoch of one soup
+// (MutateAndRunPrograms, common_language.h:157-193).
 #pragma once
 
 #include "internal.h"
-#include "interp.cuh"
+#include "staged.cuh"
 
 namespace cubff {
 
 constexpr int kThreads = 128;  // one group of four warps
 constexpr int kGroups = kThreads / 128;
 
-// Shared memory per CTA: two per-lane 128-byte areas per thread (the tape, and
-// the Forth stack or the BFF/SUBLEQ cycle-check snapshot), then the op table.
+// Shared memory per CTA.  SUBLEQ: two per-lane 128-byte areas per thread (the
+// tape and the cycle check's snapshot); the staged languages: their warps', then
+// the op and command tables.
 template <int L>
 constexpr size_t epoch_smem_bytes() {
-  return 2 * kGroups * kGroupBytes + 256;
+  if constexpr (LangTraits<L>::kStaged) return kThreads / 32 * sizeof(StagedMem<L>) + 512;
+  else return 2 * kGroups * kGroupBytes;
 }
-constexpr size_t kMaxEpochSmem = 2 * kGroups * kGroupBytes + 256;
 
 __device__ __forceinline__ void load_pair(const uint8_t *soup, uint32_t p1, uint32_t p2,
                                           uint32_t w[32]) {
@@ -46,38 +46,36 @@ __device__ __forceinline__ void mutate(uint64_t key0, uint32_t prob, uint32_t w[
   }
 }
 
-// One CTA's share (pairs [block*kThreads, (block+1)*kThreads)) of one epoch of
-// one soup.  smem holds epoch_smem_bytes<L>() bytes.  Ends with the CTA's
-// threads converged and smem free for reuse after a __syncthreads().
-template <int L>
-__device__ __forceinline__ void epoch_cta(const EpochArgs &a, uint64_t block, uint8_t *smem) {
-  uint8_t *optab = smem + 2 * kGroups * kGroupBytes;
-  const uint32_t tid = threadIdx.x;
-  if (LangTraits<L>::kNeedsTable)
-    for (uint32_t c = tid; c < 256; c += kThreads) optab[c] = op_of(L, c);
+__device__ __forceinline__ void add_counts(const EpochArgs &a, uint32_t ops, uint32_t raw) {
+  const uint32_t wops = __reduce_add_sync(0xffffffffu, ops);
+  const uint32_t wraw = __reduce_add_sync(0xffffffffu, raw);
+  if ((threadIdx.x & 31) == 0) {
+    if (wops) atomicAdd(a.ops, static_cast<unsigned long long>(wops));
+    if (a.raw && wraw) atomicAdd(a.raw, static_cast<unsigned long long>(wraw));
+  }
+}
 
+// SUBLEQ: one pair per thread.
+template <int L>
+__global__ void __launch_bounds__(kThreads) epoch_kernel(EpochArgs a) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const uint32_t tid = threadIdx.x;
   const uint64_t npairs = a.n / 2;
-  const uint64_t k = block * kThreads + tid;
+  const uint64_t k = uint64_t(blockIdx.x) * kThreads + tid;
   const bool active = k < npairs;
   const LaneBytes t{smem, lane_base(tid)};
-  const LaneBytes stk{smem + kGroups * kGroupBytes, lane_base(tid)};
+  const LaneBytes snap{smem + kGroups * kGroupBytes, lane_base(tid)};
 
-  uint32_t p1 = 0, p2 = 0;
-  uint32_t w[32];
+  uint32_t ops = 0, raw = 0;
   if (active) {
-    p1 = a.perm[2 * k];
-    p2 = a.perm[2 * k + 1];
+    const uint32_t p1 = a.perm[2 * k], p2 = a.perm[2 * k + 1];
+    uint32_t w[32];
     load_pair(a.soup, p1, p2, w);
     mutate((a.n * a.epoch_key + k) * kPair, a.mutation_prob, w);
 #pragma unroll
     for (int i = 0; i < kPair; i++) t.set(i, w[i >> 2] >> ((i & 3) * 8));
-  }
-  __syncthreads();  // op table visible
-
-  uint32_t ops = 0, raw = 0;
-  const uint64_t num_indices = a.d_num_indices ? *a.d_num_indices : a.num_indices;
-  if (active) {
-    if (k < num_indices) ops = evaluate<L>(t, stk, optab, &raw);
+    const uint64_t num_indices = a.d_num_indices ? *a.d_num_indices : a.num_indices;
+    if (k < num_indices) ops = evaluate<L>(t, snap, nullptr, &raw);
 #pragma unroll
     for (int q = 0; q < 32; q++) {
       w[q] = t.get(4 * q) | (t.get(4 * q + 1) << 8) | (t.get(4 * q + 2) << 16) |
@@ -95,18 +93,103 @@ __device__ __forceinline__ void epoch_cta(const EpochArgs &a, uint64_t block, ui
       g2[q] = make_uint4(w[16 + 4 * q], w[16 + 4 * q + 1], w[16 + 4 * q + 2],
                          w[16 + 4 * q + 3]);
   }
-  const uint32_t wops = __reduce_add_sync(0xffffffffu, ops);
-  const uint32_t wraw = __reduce_add_sync(0xffffffffu, raw);
-  if ((tid & 31) == 0) {
-    if (wops) atomicAdd(a.ops, static_cast<unsigned long long>(wops));
-    if (a.raw && wraw) atomicAdd(a.raw, static_cast<unsigned long long>(wraw));
-  }
+  add_counts(a, ops, raw);
 }
 
+// The staged languages.  A warp takes kWidth consecutive pairs: all lanes load
+// and mutate them together (a pair's 128 mutation draws are four per lane),
+// its first lanes run the first part of one each, and the pairs that go on run
+// on the whole warp one after the other.  The launch lasts as long as its
+// longest pairs, so a warp holds few.
 template <int L>
-__global__ void __launch_bounds__(kThreads) epoch_kernel(EpochArgs a) {
+__global__ void __launch_bounds__(kThreads, 5) staged_epoch_kernel(EpochArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
-  epoch_cta<L>(a, blockIdx.x, smem);
+  using LaneM = typename Stages<L>::Lane;
+  constexpr uint32_t kWidth = StagedMem<L>::kWidth;
+  uint8_t *tables = smem + kThreads / 32 * sizeof(StagedMem<L>);
+  const uint8_t *optab = tables, *cmdflag = tables + 256;
+  fill_tables<L>(tables);
+  __syncthreads();
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t npairs = a.n / 2;
+  const uint64_t k0 = (uint64_t(blockIdx.x) * (kThreads / 32) + warp) * kWidth;
+  if (k0 >= npairs) return;
+  const uint32_t count = static_cast<uint32_t>(npairs - k0 < kWidth ? npairs - k0 : kWidth);
+  StagedMem<L> &mem = reinterpret_cast<StagedMem<L> *>(smem)[warp];
+  const LaneWords<kWidth> t = mem.tape(lane), stk = mem.stack(lane);
+  uint32_t *soup = reinterpret_cast<uint32_t *>(a.soup);
+
+  // Lane l holds word l of each pair: program `mine` of it, word l % 16.
+  uint32_t mine[kWidth];
+#pragma unroll
+  for (uint32_t j = 0; j < kWidth; j++)
+    mine[j] = j < count ? a.perm[2 * (k0 + j) + (lane >> 4)] : 0;
+#pragma unroll
+  for (uint32_t j = 0; j < kWidth; j++)
+    if (j < count) mem.tapes[lane * kWidth + j] = soup[uint64_t(mine[j]) * 16 + (lane & 15)];
+  __syncwarp();
+  // Mutations (common_language.h:172-180).
+  if (a.mutation_prob != 0) {
+    for (uint32_t j = 0; j < count; j++) {
+      const uint64_t key = (a.n * a.epoch_key + k0 + j) * kPair + lane;
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const uint64_t r = splitmix64(key + 32 * q);
+        if (static_cast<uint32_t>(r >> 8) % (1u << 30) < a.mutation_prob)
+          mem.tape(j).set(32 * q + lane, static_cast<uint32_t>(r));
+      }
+    }
+    __syncwarp();
+  }
+  const uint64_t num_indices = a.d_num_indices ? *a.d_num_indices : a.num_indices;
+  LaneM m;
+  m.status = LaneM::kEnds;
+  Mask128 cmd{0, 0};
+  if (L <= kBffSelfmove) {
+    for (uint32_t j = 0; j < count; j++) {
+      const LaneWords<kWidth> tj = mem.tape(j);
+      uint32_t w[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        w[q] = __ballot_sync(0xffffffffu, cmdflag[tj.get(32 * q + lane)] != 0);
+      if (lane == j)
+        cmd = Mask128{w[0] | static_cast<uint64_t>(w[1]) << 32, w[2] | static_cast<uint64_t>(w[3]) << 32};
+    }
+  }
+  const bool evaluated = lane < count && k0 + lane < num_indices;
+  if (evaluated) m.begin(t, cmd, optab);
+  while (true) {
+    const bool go = evaluated && m.status == LaneM::kRuns;
+    if (!__any_sync(0xffffffffu, go)) break;
+    if (go) m.step(t, stk, optab);
+  }
+  uint32_t ops = 0, raw = 0;
+  if (evaluated && m.status == LaneM::kJumps) m.resolve(t, optab);
+  uint32_t longs = __ballot_sync(0xffffffffu, evaluated && m.status == LaneM::kJumps);
+  if (evaluated && m.status == LaneM::kEnds) {
+    ops = m.ops();
+    raw = m.raw();
+  }
+  while (longs) {
+    const uint32_t src = static_cast<uint32_t>(__ffs(longs) - 1);
+    longs &= longs - 1;
+    const Counts c = run_on_warp(mem, m, src, lane, optab);
+    mem.tapes[lane * kWidth + src] = reinterpret_cast<const uint32_t *>(mem.warp.T)[lane];
+    if (lane == src) {
+      ops = c.ops;
+      raw = c.raw;
+    }
+  }
+  __syncwarp();
+  // First half, then second half (common_language.h:188-191): of a program
+  // paired with itself the second half stays.
+#pragma unroll
+  for (uint32_t j = 0; j < kWidth; j++) {
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, mine[j], 16);
+    if (j < count && (lane >= 16 || mine[j] != other))
+      soup[uint64_t(mine[j]) * 16 + (lane & 15)] = mem.tapes[lane * kWidth + j];
+  }
+  add_counts(a, ops, raw);
 }
 
 }  // namespace cubff

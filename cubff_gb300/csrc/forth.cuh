@@ -6,12 +6,10 @@
 // Write1 / Copy0 (forthtrivial_reset.cu:58-72, :157-166, :215-223).  The top
 // two entries of the 128-byte stack are kept in registers.
 //
-// Three machines with the same results:
+// Two machines that a program runs on in turn:
 //  * ForthFirst, one pair per lane, for a program's first steps (most random
 //    programs end in them);
-//  * ForthWarp, one pair per warp, which takes over from there;
-//  * ForthMachine, the one-shot one of the per-epoch kernels (forth_eval):
-//    ForthLane with a cycle check.
+//  * ForthWarp, one pair per warp, which takes over from there.
 #pragma once
 
 #include "coop.cuh"
@@ -570,6 +568,13 @@ struct ForthWarp {
     written.hi0 = kTape - 1;
   }
 
+  // The state at the start of a program.
+  __host__ __device__ __forceinline__ ForthState start(bool) const {
+    ForthState s;
+    s.begin();
+    return s;
+  }
+
   // Runs the program in m.T, with the stack in m.stk, from state s to its end.
   __host__ __device__ __forceinline__ void run(const ForthState &s) {
     ln.st = s;
@@ -628,89 +633,5 @@ struct ForthWarp {
   __host__ __device__ __forceinline__ uint32_t raw() const { return ln.st.i; }
   __host__ __device__ __forceinline__ uint32_t mods() const { return ln.st.mods; }
 };
-
-// The one-shot machine: ForthLane with exact cycle fast-forward at backward
-// jumps (Brent's schedule, cycle.cuh).  The state is (pos, stack pointer, stack
-// contents, tape).  The stack below the stack pointer is compared byte for
-// byte with the snapshot's (kept packed in a register, so only for stacks of
-// at most 8); the tape through a count of value-changing writes.
-template <bool kWithReset>
-struct ForthMachine : ForthLane<kWithReset> {
-  using ForthLane<kWithReset>::st;
-  // Brent-schedule snapshot taken at a backward jump.
-  int s_pos, s_sp;
-  uint32_t s_mods, s_i, s_nops, s_power, s_lam;
-  uint32_t s_top;          // stack[s_sp - 1] | stack[s_sp - 2] << 8 (0 where absent)
-  uint64_t s_mem;          // stack[0 .. s_sp - 2) packed, byte j at bits 8j (s_sp <= 8)
-
-  __host__ __device__ __forceinline__ void begin() {
-    st.begin();
-    s_pos = -1;
-    s_sp = 0;
-    s_mods = s_i = s_nops = 0;
-    s_power = 1;
-    s_lam = 0;
-    s_top = 0;
-    s_mem = 0;
-  }
-
-  // stack[0 .. sp - 2), the entries below the registers, packed.
-  __host__ __device__ __forceinline__ uint64_t pack_mem(const LaneBytes stk) const {
-    uint64_t w = 0;
-    for (int j = 0; j < st.sp - 2; j++) w |= static_cast<uint64_t>(stk.get(j)) << (8 * j);
-    return w;
-  }
-
-  // At a step boundary right after a backward jump: when the state equals
-  // the snapshot's, execution since the snapshot is periodic and whole periods
-  // are skipped (i += k * P, nops += k * the period's no-ops); the snapshot is
-  // renewed after 1, 2, 4, ... visits.  The two entries in registers are
-  // compared first: a loop's counter usually sits on top, so most visits end
-  // there without reading the stack in memory.
-  __host__ __device__ __forceinline__ void visit(const LaneBytes stk) {
-    const uint32_t top = (st.sp >= 1 ? st.r0 : 0u) | ((st.sp >= 2 ? st.r1 : 0u) << 8);
-    if (st.pos == s_pos && st.sp == s_sp && st.mods == s_mods && top == s_top &&
-        (st.sp <= 2 || pack_mem(stk) == s_mem)) {
-      const uint32_t period = st.i - s_i;
-      const uint32_t k = (kStepLimit - st.i) / period;
-      st.i += k * period;
-      st.nops += k * (st.nops - s_nops);
-    }
-    if (++s_lam == s_power) {
-      s_pos = st.sp <= 8 ? st.pos : -1;  // larger stacks: no snapshot
-      s_sp = st.sp;
-      s_mods = st.mods;
-      s_i = st.i;
-      s_nops = st.nops;
-      s_top = top;
-      s_mem = (st.sp > 2 && st.sp <= 8) ? pack_mem(stk) : 0;
-      s_power <<= 1;
-      s_lam = 0;
-    }
-  }
-  // One step; returns true when the program has ended.
-  __host__ __device__ __forceinline__ bool step(const LaneBytes t, const LaneBytes stk,
-                                                const uint8_t *__restrict__ optab) {
-    bool back;
-    if (ForthLane<kWithReset>::step(t, stk, optab, back)) return true;
-    if (back) {
-      visit(stk);
-      if (st.i >= kStepLimit) return true;
-    }
-    return false;
-  }
-};
-
-template <bool kWithReset>
-__host__ __device__ __forceinline__ uint32_t forth_eval(const LaneBytes t, const LaneBytes stk,
-                                                        const uint8_t *__restrict__ optab,
-                                                        uint32_t *raw) {
-  ForthMachine<kWithReset> m;
-  m.begin();
-  while (!m.step(t, stk, optab)) {
-  }
-  *raw = m.st.i;
-  return m.st.i - m.st.nops;
-}
 
 }  // namespace cubff

@@ -1,7 +1,7 @@
 // interp.cuh — compile-time dispatch to the 13 language interpreters.
-// Every interpreter runs Language::Evaluate(tape, 8192) on one thread's
-// shared-memory pair tape and returns the reference-counted op count
-// (Evaluate's return value), reporting the raw loop iterations in *raw.
+// Every interpreter runs Language::Evaluate(tape, 8192) and gives the
+// reference-counted op count (Evaluate's return value) and the raw loop
+// iterations.
 #pragma once
 
 #include <type_traits>
@@ -13,31 +13,10 @@
 
 namespace cubff {
 
-// ---------------------------------------------------------------------------
-// Per-language dispatch (compile-time).
-
 template <int L>
 struct LangTraits {
-  static constexpr bool kForthFamily = (L >= kForth && L <= kForthtrivialReset);
-  static constexpr bool kNeedsTable = (L <= kForthtrivialReset);
+  static constexpr bool kStaged = (L <= kForthtrivialReset);  // BFF and Forth families
 };
-
-template <int L>
-__host__ __device__ __forceinline__ uint32_t evaluate(const LaneBytes t, const LaneBytes stk,
-                                             const uint8_t *__restrict__ optab,
-                                             uint32_t *raw) {
-  if constexpr (L == kBff) return bff_eval<true, kLogicScan, 0xFF>(t, stk, optab, raw);
-  else if constexpr (L == kBffNoheads) return bff_eval<false, kLogicScan, 0xFF>(t, stk, optab, raw);
-  else if constexpr (L == kBffNoheads4bit) return bff_eval<false, kLogicScan, 0x0F>(t, stk, optab, raw);
-  else if constexpr (L == kBffPerm) return bff_eval<true, kLogicScan, 0xFF>(t, stk, optab, raw);
-  else if constexpr (L == kBff8) return bff_eval<true, kLogicJump8, 0xFF>(t, stk, optab, raw);
-  else if constexpr (L == kBff8Noheads) return bff_eval<false, kLogicJump8, 0xFF>(t, stk, optab, raw);
-  else if constexpr (L == kBffSelfmove) return bff_eval<true, kLogicSelfmove, 0xFF>(t, stk, optab, raw);
-  else if constexpr (L == kForthtrivialReset) return forth_eval<true>(t, stk, optab, raw);
-  else if constexpr (LangTraits<L>::kForthFamily) return forth_eval<false>(t, stk, optab, raw);
-  else if constexpr (L == kSubleq) return subleq_eval(t, stk, raw);
-  else return rsubleq4_eval(t, stk, raw);
-}
 
 // The two machines that run a BFF or Forth program in turn: on a lane, then on
 // a warp (with that warp's shared memory, and whether a program has a stack).
@@ -119,5 +98,26 @@ struct LaneMachine<L, true> {
   uint32_t ops() const { return n; }
   uint32_t raw() const { return i; }
 };
+
+// Language::Evaluate on one tape: on a thread (SUBLEQ), or on the host.
+template <int L>
+__host__ __device__ __forceinline__ uint32_t evaluate(const LaneBytes t, const LaneBytes stk,
+                                                      const uint8_t *__restrict__ optab,
+                                                      uint32_t *raw) {
+  if constexpr (L == kSubleq) {
+    return subleq_eval(t, stk, raw);
+  } else if constexpr (L == kRsubleq4) {
+    return rsubleq4_eval(t, stk, raw);
+  } else {
+    LaneMachine<L> m;
+    Mask128 cmd{0, 0};
+    for (int p = 0; p < kPair; p++) mask_assign(cmd, p, op_of(L, t.get(p)) < kNull);
+    m.begin(t, cmd);
+    while (!m.step(t, stk, LaneNp{nullptr, 0}, optab)) {
+    }
+    *raw = m.raw();
+    return m.ops();
+  }
+}
 
 }  // namespace cubff

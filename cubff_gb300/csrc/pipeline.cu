@@ -21,6 +21,7 @@
 #include <cstdlib>
 
 #include "epoch_body.cuh"
+#include "staged.cuh"
 
 namespace cubff {
 namespace {
@@ -441,48 +442,19 @@ struct LaneServer {
 // epochs with 8 (32 lanes: 76.9, 16: 44.6), one of 1022 bff_noheads programs
 // 2.1 ms for 64 (4.3, 3.0); only the 20 first epochs of a random soup of 2^17
 // are a little faster with 32 (3.07 ms, 8: 3.27).
-__device__ __forceinline__ BffState broadcast(const BffState &s, uint32_t src) {
-  constexpr uint32_t kAll = 0xffffffffu;
-  BffState r;
-  r.q = __shfl_sync(kAll, s.q, src);
-  r.h0 = __shfl_sync(kAll, s.h0, src);
-  r.h1 = __shfl_sync(kAll, s.h1, src);
-  r.i = __shfl_sync(kAll, s.i, src);
-  r.n = __shfl_sync(kAll, s.n, src);
-  r.mods = __shfl_sync(kAll, s.mods, src);
-  return r;
-}
-__device__ __forceinline__ ForthState broadcast(const ForthState &s, uint32_t src) {
-  constexpr uint32_t kAll = 0xffffffffu;
-  ForthState r;
-  r.begin();
-  r.pos = __shfl_sync(kAll, s.pos, src);
-  r.sp = __shfl_sync(kAll, s.sp, src);
-  r.r0 = __shfl_sync(kAll, s.r0, src);
-  r.r1 = __shfl_sync(kAll, s.r1, src);
-  r.i = __shfl_sync(kAll, s.i, src);
-  r.nops = __shfl_sync(kAll, s.nops, src);
-  r.mods = __shfl_sync(kAll, s.mods, src);
-  return r;
-}
-
 template <int L>
 struct StagedServer {
   using LaneM = typename Stages<L>::Lane;
-  using WarpM = typename Stages<L>::template Warp<DeviceWarp>;
-  using Mem = typename Stages<L>::Mem;
-  static constexpr uint32_t kWidth = 8;  // lanes that hold pairs
-  static constexpr size_t kTapes = kWidth * kPair, kStacks = Stages<L>::kStack ? kTapes : 0,
-                          kWarpBytes = kTapes + kStacks + sizeof(Mem);
+  static constexpr uint32_t kWidth = StagedMem<L>::kWidth;
+  static constexpr size_t kWarpBytes = sizeof(StagedMem<L>);
   LaneM m;
+  StagedMem<L> &mem;
   LaneWords<kWidth> t, stk;
-  Mem &mem;
   const uint8_t *optab, *cmdflag;
 
   __device__ __forceinline__ StagedServer(uint8_t *smem, const uint8_t *tables, uint32_t tid)
-      : t{smem + (tid >> 5) * kWarpBytes, tid & 31}, stk{t.s + kStacks, tid & 31},
-        mem(*reinterpret_cast<Mem *>(smem + (tid >> 5) * kWarpBytes + kTapes + kStacks)),
-        optab(tables), cmdflag(tables + 256) {
+      : mem(reinterpret_cast<StagedMem<L> *>(smem)[tid >> 5]), t(mem.tape(tid & 31)),
+        stk(mem.stack(tid & 31)), optab(tables), cmdflag(tables + 256) {
     m.status = LaneM::kEnds;
   }
 
@@ -529,28 +501,18 @@ struct StagedServer {
   __device__ __forceinline__ void run_long(const PipeCtx &b, Lane &ln, uint32_t src,
                                            uint32_t lane, uint32_t slot_ctr) {
     constexpr uint32_t kAll = 0xffffffffu;
-    const auto st = broadcast(m.state(), src);
-    __syncwarp();  // the lane's tape
-    uint32_t *T = reinterpret_cast<uint32_t *>(mem.T);
-    T[lane] = reinterpret_cast<const uint32_t *>(t.s)[lane * kWidth + src];
-    if constexpr (Stages<L>::kStack)
-      reinterpret_cast<uint32_t *>(mem.stk)[lane] =
-          reinterpret_cast<const uint32_t *>(stk.s)[lane * kWidth + src];
-    __syncwarp();
-    WarpM wm(DeviceWarp{lane}, mem, optab);
-    wm.run(st);
-    __syncwarp();
+    const Counts c = run_on_warp(mem, m, src, lane, optab);
     const PipeSoup &sp = b.soups[__shfl_sync(kAll, ln.si, src)];
-    if (wm.mods() != 0 || __shfl_sync(kAll, ln.dirty, src)) {
+    if (c.mods != 0 || __shfl_sync(kAll, ln.dirty, src)) {
       const uint32_t p1 = __shfl_sync(kAll, ln.p1, src), p2 = __shfl_sync(kAll, ln.p2, src);
       // First half, then second half (common_language.h:188-191): of a
       // program paired with itself the second half stays.
       if (lane >= 16 || p1 != p2)
         reinterpret_cast<uint32_t *>(sp.soup + uint64_t(lane < 16 ? p1 : p2) * kTape)[lane & 15] =
-            T[lane];
+            reinterpret_cast<const uint32_t *>(mem.warp.T)[lane];
     }
     __syncwarp();  // the warp's stores before the lane's notifications
-    if (lane == src) finish(sp, ln, slot_ctr, wm.ops(), wm.raw());
+    if (lane == src) finish(sp, ln, slot_ctr, c.ops, c.raw);
   }
 
   __device__ __forceinline__ bool iterate(const PipeCtx &b, const PipeQueue &q, Lane &ln,
@@ -627,12 +589,7 @@ __global__ void __launch_bounds__(kThreads, (L <= kForthtrivialReset) ? 5 : 4)
   uint8_t *tables = smem + server_bytes<L>();
   PipeSoup *soups = reinterpret_cast<PipeSoup *>(tables + 512);
   const uint32_t tid = threadIdx.x, lane = tid & 31;
-  if (LangTraits<L>::kNeedsTable) {
-    for (uint32_t c = tid; c < 256; c += kThreads) {
-      tables[c] = op_of(L, c);
-      tables[256 + c] = op_of(L, c) < kNull;
-    }
-  }
+  if (LangTraits<L>::kStaged) fill_tables<L>(tables);
   {
     const uint32_t *src = reinterpret_cast<const uint32_t *>(pb.soups);
     uint32_t *dst = reinterpret_cast<uint32_t *>(soups);
