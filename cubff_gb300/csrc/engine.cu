@@ -73,7 +73,6 @@ int cubff_soup::ensure_buffers() {
     }
     if (p.pairing == CUBFF_PAIR_PATTERN) {
       CUBFF_CUDA_TRY(cudaMallocHost(&h_pat_ni, size_t(batch) * sizeof(uint64_t)));
-      CUBFF_CUDA_TRY(cudaMallocHost(&h_pat_undecided, size_t(batch) * sizeof(uint32_t)));
     }
     CUBFF_CUDA_TRY(cudaMalloc(&d_counters, kCounterWords * sizeof(unsigned long long)));
     CUBFF_CUDA_TRY(cudaMallocHost(&h_counters, kCounterWords * sizeof(unsigned long long)));
@@ -105,10 +104,8 @@ void cubff_soup::release() {
   if (d_pat_offs) cudaFree(d_pat_offs);
   if (d_pat_tgts) cudaFree(d_pat_tgts);
   if (h_pat_ni) cudaFreeHost(h_pat_ni);
-  if (h_pat_undecided) cudaFreeHost(h_pat_undecided);
   d_pat_offs = d_pat_tgts = nullptr;
   h_pat_ni = nullptr;
-  h_pat_undecided = nullptr;
   if (d_inv) cudaFree(d_inv);
   if (d_readycnt) cudaFree(d_readycnt);
   d_inv = d_readycnt = nullptr;
@@ -152,7 +149,7 @@ int cubff_soup::fill_pairing(uint64_t first, uint32_t count, cudaStream_t st) {
       break;
     case CUBFF_PAIR_PATTERN:
       CUBFF_TRY(launch_pattern(s0, first, count, n, d_pat_offs, d_pat_tgts, d_perm, d_num_indices,
-                               d_scratch, h_pat_undecided, st));
+                               d_scratch, st));
       CUBFF_CUDA_TRY(cudaMemcpyAsync(h_pat_ni, d_num_indices, size_t(count) * sizeof(uint64_t),
                                      cudaMemcpyDeviceToHost, st));
       CUBFF_CUDA_TRY(cudaStreamSynchronize(st));

@@ -58,7 +58,6 @@ struct cubff_soup {
   // num_indices of the cached pairings, copied back to pinned memory.
   uint32_t *d_pat_offs = nullptr, *d_pat_tgts = nullptr;
   uint64_t *h_pat_ni = nullptr;      // [batch] pinned
-  uint32_t *h_pat_undecided = nullptr;  // [batch] pinned (convergence checks)
 
   // Pipelined runs: inverse shuffles, mutation masks and ready counters of
   // the cached epochs (the counters are zero between launches).

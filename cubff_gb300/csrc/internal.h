@@ -129,13 +129,10 @@ int launch_shuffle(uint64_t s0, uint64_t first_epoch, uint32_t n_epochs,
                    uint64_t n, uint32_t *out, void *scratch, cudaStream_t stream);
 // Pattern pairing (common_language.h:435-463) of n_epochs epochs on the
 // device: out[e] = the epoch's shuffle_idx, num_indices[e] its pair count.
-// Synchronises the stream (convergence checks read h_undecided, pinned,
-// n_epochs entries).
 size_t pattern_scratch_bytes(uint64_t n, uint32_t n_epochs);
 int launch_pattern(uint64_t s0, uint64_t first_epoch, uint32_t n_epochs, uint64_t n,
                    const uint32_t *offs, const uint32_t *tgts, uint32_t *out,
-                   uint64_t *num_indices, void *scratch, uint32_t *h_undecided,
-                   cudaStream_t stream);
+                   uint64_t *num_indices, void *scratch, cudaStream_t stream);
 int launch_fixed(uint64_t first_epoch, uint32_t n_epochs, uint64_t n,
                  uint32_t *out, cudaStream_t stream);
 int launch_cyclic(uint64_t first_epoch, uint32_t n_epochs, uint64_t n,

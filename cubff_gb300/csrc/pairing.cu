@@ -18,6 +18,8 @@
 // which strictly increase and so end.
 #include <mutex>
 
+#include <cooperative_groups.h>
+
 #include "internal.h"
 #include "common.cuh"
 
@@ -234,107 +236,121 @@ unsigned blocks_for(uint64_t m, unsigned t) { return static_cast<unsigned>((m + 
 // That is greedy matching in a fixed priority order (the rank of i in the
 // order) over one proposal edge per program, and is rebuilt exactly in
 // parallel (greedy matching in rounds, Blelloch, Fineman and Shun, SPAA
-// 2012): edge e_i is accepted iff no edge of smaller rank that touches i or
-// nb_i is accepted.  The edges that can block e_i are e_{nb_i} and every e_j
-// with nb_j in {i, nb_i}; each round decides the undecided edges whose
-// blockers of smaller rank are all decided (one accepted blocker rejects at
-// once).  The smallest-rank undecided edge is always decidable, so rounds
-// end; with random ranks a few dozen suffice.  Accepted edges are then
-// written in rank order and unused programs in increasing order, both placed
-// by prefix sums.
-enum : uint8_t { kUndecided = 0, kAccepted = 1, kRejected = 2, kNoEdge = 3 };
+// 2012): each round, every undecided edge (i, nb_i) puts its rank into both
+// ends with atomicMin; an edge that is the smallest at both is accepted, one
+// with an end taken by an accepted edge is rejected.  The undecided edge of
+// smallest rank is always accepted, so rounds end; with random ranks a dozen
+// or so suffice.  Accepted edges are then written in rank order and unused
+// programs in increasing order, both placed by prefix sums.
+constexpr uint32_t kMatchThreads = 1024, kMatchCluster = 8;
+constexpr uint32_t kNoRank = 0xFFFFFFFFu;
 
-// nb[e][i] (or -1 for an empty list), and the in-degree counts for the
-// in-lists (cnt[e][v] += 1 for nb = v).
-__global__ void pat_propose(uint64_t s0, uint64_t first_epoch, uint64_t n, uint64_t m,
-                            const uint32_t *offs, const uint32_t *tgts, int32_t *nb,
-                            uint32_t *cnt, uint8_t *status) {
-  const uint64_t idx = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= m) return;
-  const uint64_t e = idx / n, i = idx - e * n;
-  const uint32_t lo = offs[i], len = offs[i + 1] - lo;
-  if (len == 0) {
-    nb[idx] = -1;
-    status[idx] = kNoEdge;
-    return;
-  }
+// The proposals and the matching of one epoch on one cluster.  Bound by the
+// latency of its scattered reads and atomics (the arrays of a few million
+// edges stay in L2), so: a round is two passes over the edges still undecided,
+// each warp keeping its own of them as a dense list (`list`, at the place of
+// its segment of programs), with a cluster barrier after each pass instead of a
+// launch; epochs do not wait for one another, and nothing returns to the host.
+// 32 epochs of 512 x 256 programs, radius 2: 144 us; 8 launches over all edges,
+// in which each undecided one looked at the edges that could block it, took
+// 2370 us, and the in-lists for them a counting sort.  Two arrays of smallest ranks alternate: the
+// second pass clears the next round's at the ends of the edges it keeps, which
+// include all that the next round writes.
+__global__ void __launch_bounds__(kMatchThreads)
+    pat_match(uint64_t s0, uint64_t first_epoch, uint64_t n, const uint32_t *offs,
+              const uint32_t *tgts, const uint32_t *rank_of, int32_t *nb_of, uint32_t *best0,
+              uint32_t *best1, uint32_t *list_of, uint8_t *accepted_of, uint8_t *used_of) {
+  namespace cg = cooperative_groups;
+  __shared__ uint32_t more[2];  // an edge is left undecided, by parity of the round
+  const cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t blocks = cluster.num_blocks(), lane = threadIdx.x & 31;
+  const uint64_t e = blockIdx.x / blocks, base = e * n;
+  const uint32_t warp = cluster.block_rank() * (kMatchThreads / 32) + (threadIdx.x >> 5);
+  const uint64_t warps = uint64_t(blocks) * (kMatchThreads / 32);
+  const uint64_t seg = (n + warps * 32 - 1) / (warps * 32) * 32;
+  const uint64_t lo = warp * seg < n ? warp * seg : n, hi = lo + seg < n ? lo + seg : n;
+  const uint32_t *rank = rank_of + base;
+  int32_t *nb = nb_of + base;
+  uint32_t *list = list_of + base + lo;
+  uint8_t *accepted = accepted_of + base, *used = used_of + base;
+  // Appends the lanes' kept edges to the list; no lane's entry is overwritten
+  // before it was read (the list only shrinks).
+  uint32_t count = 0;
+  const auto keep_edge = [&](bool keep, uint32_t i) {
+    const uint32_t mask = __ballot_sync(0xffffffffu, keep);
+    if (keep) list[count + __popc(mask & ((1u << lane) - 1))] = i;
+    count += __popc(mask);
+  };
+
   const uint64_t ek = seed_from(s0, first_epoch + e);
-  const uint32_t v = tgts[lo + seed_from(s0, ek ^ seed_from(s0, i)) % len];
-  nb[idx] = static_cast<int32_t>(v);
-  status[idx] = kUndecided;
-  atomicAdd(&cnt[e * n + v], 1u);
-}
-
-// bucket[e][start[v] ..] = the programs j with nb_j = v.
-__global__ void pat_fill(uint64_t n, uint64_t m, const int32_t *nb, uint32_t *cnt,
-                         const uint32_t *start, uint32_t *bucket) {
-  const uint64_t idx = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= m || nb[idx] < 0) return;
-  const uint64_t e = idx / n, i = idx - e * n;
-  const uint64_t g = e * n + static_cast<uint32_t>(nb[idx]);
-  bucket[e * n + start[g] + atomicAdd(&cnt[g], 1u)] = static_cast<uint32_t>(i);
-}
-
-// One round over the undecided edges (statuses only move from undecided to
-// final, so reading a neighbour's status from this same round is safe).
-__global__ void pat_round(uint64_t n, uint64_t m, const int32_t *nb, const uint32_t *rank,
-                          const uint32_t *start, const uint32_t *len, const uint32_t *bucket,
-                          uint8_t *status, uint32_t *undecided) {
-  const uint64_t idx = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= m) return;
-  if (static_cast<volatile uint8_t *>(status)[idx] != kUndecided) return;
-  const uint64_t e = idx / n, i = idx - e * n, base = e * n;
-  const volatile uint8_t *st = status + base;
-  const uint32_t r = rank[idx];
-  const uint32_t b = static_cast<uint32_t>(nb[idx]);
-  bool all_decided = true;
-  // e_b, the edge proposed by the neighbour.
-  if (rank[base + b] < r) {
-    const uint8_t x = st[b];
-    if (x == kAccepted) {
-      status[idx] = kRejected;
-      return;
+  for (uint64_t x = lo; x < hi; x += 32) {
+    const uint64_t i = x + lane;
+    bool edge = false;
+    if (i < hi) {
+      const uint32_t first = offs[i], len = offs[i + 1] - first;
+      edge = len != 0;
+      nb[i] = edge ? static_cast<int32_t>(
+                         tgts[first + seed_from(s0, ek ^ seed_from(s0, i)) % len])
+                   : -1;
+      accepted[i] = used[i] = 0;
+      best0[base + i] = best1[base + i] = kNoRank;
     }
-    all_decided &= x != kUndecided;
+    keep_edge(edge, static_cast<uint32_t>(i));
   }
-  // Every e_j with nb_j = i or nb_j = b (e_i itself among the latter).
-  for (int side = 0; side < 2; side++) {
-    const uint32_t v = side ? b : static_cast<uint32_t>(i);
-    const uint32_t s = start[base + v], l = len[base + v];
-    for (uint32_t q = 0; q < l; q++) {
-      const uint32_t j = bucket[base + s + q];
-      if (j == i || rank[base + j] >= r) continue;
-      const uint8_t x = st[j];
-      if (x == kAccepted) {
-        status[idx] = kRejected;
-        return;
+  if (threadIdx.x < 2) more[threadIdx.x] = 0;
+  cluster.sync();
+
+  for (uint64_t round = 0; round < n; round++) {
+    uint32_t *best = (round & 1 ? best1 : best0) + base;
+    uint32_t *next = (round & 1 ? best0 : best1) + base;
+    uint32_t was = count;
+    count = 0;
+    for (uint32_t x = lane; x - lane < was; x += 32) {
+      const uint32_t i = x < was ? list[x] : 0;
+      bool keep = false;
+      if (x < was) {
+        const uint32_t b = static_cast<uint32_t>(nb[i]), r = rank[i];
+        keep = (__ldcg(used + i) | __ldcg(used + b)) == 0;
+        if (keep) {
+          atomicMin(best + i, r);
+          atomicMin(best + b, r);
+        }
       }
-      all_decided &= x != kUndecided;
+      keep_edge(keep, i);
     }
+    cluster.sync();
+    if (threadIdx.x == 0) more[(round + 1) & 1] = 0;
+    was = count;
+    count = 0;
+    for (uint32_t x = lane; x - lane < was; x += 32) {
+      const uint32_t i = x < was ? list[x] : 0;
+      bool keep = false;
+      if (x < was) {
+        const uint32_t b = static_cast<uint32_t>(nb[i]), r = rank[i];
+        keep = __ldcg(best + i) != r || __ldcg(best + b) != r;
+        if (keep) {
+          next[i] = next[b] = kNoRank;
+        } else {
+          used[i] = used[b] = 1;
+          accepted[i] = 1;
+        }
+      }
+      keep_edge(keep, i);
+    }
+    if (__syncthreads_or(count != 0) && threadIdx.x < blocks)
+      *cluster.map_shared_rank(&more[round & 1], threadIdx.x) = 1;
+    cluster.sync();
+    if (more[round & 1] == 0) break;
   }
-  if (all_decided) status[idx] = kAccepted;
-  else atomicAdd(&undecided[e], 1u);
 }
 
-// used[e][v] for both ends of every accepted edge; flags for the two prefix
-// sums: accepted edges by rank, unused programs by id.
-__global__ void pat_flags(uint64_t n, uint64_t m, const uint32_t *order, const int32_t *nb,
-                          const uint8_t *status, uint8_t *used) {
-  const uint64_t idx = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= m) return;
-  if (status[idx] == kAccepted) {
-    const uint64_t e = idx / n;
-    used[idx] = 1;
-    used[e * n + static_cast<uint32_t>(nb[idx])] = 1;
-  }
-}
-
-__global__ void pat_count(uint64_t n, uint64_t m, const uint32_t *order, const uint8_t *status,
+// Flags for the two prefix sums: accepted edges by rank, unused programs by id.
+__global__ void pat_count(uint64_t n, uint64_t m, const uint32_t *order, const uint8_t *accepted,
                           const uint8_t *used, uint32_t *acc_by_rank, uint32_t *unused_by_id) {
   const uint64_t idx = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= m) return;
   const uint64_t e = idx / n;
-  acc_by_rank[idx] = status[e * n + order[idx]] == kAccepted;
+  acc_by_rank[idx] = accepted[e * n + order[idx]];
   unused_by_id[idx] = used[idx] == 0;
 }
 
@@ -342,15 +358,15 @@ __global__ void pat_count(uint64_t n, uint64_t m, const uint32_t *order, const u
 // the unused programs in id order (pos from the second).  num_indices[e] =
 // the number of accepted edges.
 __global__ void pat_write(uint64_t n, uint64_t m, const uint32_t *order, const int32_t *nb,
-                          const uint8_t *status, const uint8_t *used, const uint32_t *acc_pos,
+                          const uint8_t *accepted, const uint8_t *used, const uint32_t *acc_pos,
                           const uint32_t *unused_pos, uint32_t *out, uint64_t *num_indices) {
   const uint64_t idx = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= m) return;
   const uint64_t e = idx / n, t = idx - e * n, base = e * n;
   const uint64_t num = acc_pos[base + n - 1] +
-                       (status[base + order[base + n - 1]] == kAccepted ? 1 : 0);
+                       accepted[base + order[base + n - 1]];
   const uint32_t i = order[idx];
-  if (status[base + i] == kAccepted) {
+  if (accepted[base + i]) {
     const uint32_t p = acc_pos[idx];
     out[base + 2 * p] = i;
     out[base + 2 * p + 1] = static_cast<uint32_t>(nb[base + i]);
@@ -361,19 +377,18 @@ __global__ void pat_write(uint64_t n, uint64_t m, const uint32_t *order, const i
 
 }  // namespace
 
-// Scratch of launch_pattern: the shuffle's own scratch, then order, rank,
-// nb, cnt, start, len, bucket, two scan arrays (uint32 each), status and
-// used (bytes), and one undecided counter per epoch.
+// Scratch of launch_pattern: the shuffle's own scratch, then order, rank, nb,
+// the smallest ranks (later the two scans' flags), the edge lists (later the
+// first scan's sums) and the second scan's sums (uint32 each), accepted and
+// used (bytes).
 size_t pattern_scratch_bytes(uint64_t n, uint32_t n_epochs) {
   const uint64_t m = n * n_epochs;
-  return shuffle_scratch_bytes(n, n_epochs) + 9 * m * sizeof(uint32_t) + 2 * m +
-         size_t(n_epochs) * sizeof(uint32_t) + 64;
+  return shuffle_scratch_bytes(n, n_epochs) + 7 * m * sizeof(uint32_t) + 2 * m;
 }
 
 int launch_pattern(uint64_t s0, uint64_t first_epoch, uint32_t E, uint64_t n,
                    const uint32_t *offs, const uint32_t *tgts, uint32_t *out,
-                   uint64_t *num_indices, void *scratch, uint32_t *h_undecided,
-                   cudaStream_t stream) {
+                   uint64_t *num_indices, void *scratch, cudaStream_t stream) {
   if (n == 0 || E == 0) return CUBFF_OK;
   const uint64_t m = n * E;
   uint8_t *p = static_cast<uint8_t *>(scratch);
@@ -386,48 +401,35 @@ int launch_pattern(uint64_t s0, uint64_t first_epoch, uint32_t E, uint64_t n,
   };
   uint32_t *order = take32(), *rank = take32();
   int32_t *nb = reinterpret_cast<int32_t *>(take32());
-  uint32_t *cnt = take32(), *start = take32(), *len = take32(), *bucket = take32();
-  uint32_t *acc = take32(), *unused = take32();
-  uint8_t *status = p;
-  p += m;
-  uint8_t *used = p;
-  p += m;
-  p = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(p) + 15) & ~uintptr_t(15));
-  uint32_t *undecided = reinterpret_cast<uint32_t *>(p);
+  uint32_t *acc = take32(), *unused = take32(), *acc_pos = take32(), *unused_pos = take32();
+  uint8_t *accepted = p, *used = p + m;
   const unsigned blocks = blocks_for(m, 256);
 
   CUBFF_TRY(launch_shuffle(s0, first_epoch, E, n, order, fy, stream));
   CUBFF_TRY(launch_inverse(order, E, n, rank, stream));
-  CUBFF_CUDA_TRY(cudaMemsetAsync(cnt, 0, m * sizeof(uint32_t), stream));
-  CUBFF_CUDA_TRY(cudaMemsetAsync(used, 0, m, stream));
-  pat_propose<<<blocks, 256, 0, stream>>>(s0, first_epoch, n, m, offs, tgts, nb, cnt, status);
-  // In-degree counts -> lists: len keeps the counts, start their prefix sums.
-  CUBFF_CUDA_TRY(cudaMemcpyAsync(len, cnt, m * sizeof(uint32_t), cudaMemcpyDeviceToDevice, stream));
-  // (also zeroes cnt; the chunk sums go to the shuffle's scratch, free by now)
-  launch_segment_scan(n, E, cnt, start, static_cast<uint32_t *>(fy), stream);
-  pat_fill<<<blocks, 256, 0, stream>>>(n, m, nb, cnt, start, bucket);
-  // Rounds until every edge is decided (checked every 8 rounds).
-  for (int checks = 0;; checks++) {
-    CUBFF_CUDA_TRY(cudaMemsetAsync(undecided, 0, E * sizeof(uint32_t), stream));
-    for (int r = 0; r < 8; r++) {
-      if (r == 7) CUBFF_CUDA_TRY(cudaMemsetAsync(undecided, 0, E * sizeof(uint32_t), stream));
-      pat_round<<<blocks, 256, 0, stream>>>(n, m, nb, rank, start, len, bucket, status, undecided);
-    }
-    CUBFF_CUDA_TRY(cudaMemcpyAsync(h_undecided, undecided, E * sizeof(uint32_t),
-                                   cudaMemcpyDeviceToHost, stream));
-    CUBFF_CUDA_TRY(cudaStreamSynchronize(stream));
-    uint64_t left = 0;
-    for (uint32_t e = 0; e < E; e++) left += h_undecided[e];
-    if (left == 0) break;
-    if (checks > static_cast<int>(n)) return set_error(CUBFF_EDEVICE, "pattern pairing did not converge");
-  }
-  pat_flags<<<blocks, 256, 0, stream>>>(n, m, order, nb, status, used);
-  pat_count<<<blocks, 256, 0, stream>>>(n, m, order, status, used, acc, unused);
+  // As many blocks to a cluster as give each thread about 4 edges or more, up
+  // to the largest portable cluster.
+  uint32_t cluster = 1;
+  while (cluster < kMatchCluster && n > uint64_t(cluster) * kMatchThreads * 4) cluster *= 2;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim = {cluster, 1, 1};
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(E * cluster);
+  cfg.blockDim = dim3(kMatchThreads);
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  CUBFF_CUDA_TRY(cudaLaunchKernelEx(&cfg, pat_match, s0, first_epoch, n, offs, tgts,
+                                    static_cast<const uint32_t *>(rank), nb, acc, unused, acc_pos,
+                                    accepted, used));
+  pat_count<<<blocks, 256, 0, stream>>>(n, m, order, accepted, used, acc, unused);
   // Exclusive prefix sums per epoch (each scan reads its counts, writes the
-  // sums, zeroes the counts).
-  launch_segment_scan(n, E, acc, start, static_cast<uint32_t *>(fy), stream);
-  launch_segment_scan(n, E, unused, len, static_cast<uint32_t *>(fy), stream);
-  pat_write<<<blocks, 256, 0, stream>>>(n, m, order, nb, status, used, start, len, out, num_indices);
+  // sums, zeroes the counts; the chunk sums go to the shuffle's scratch).
+  launch_segment_scan(n, E, acc, acc_pos, static_cast<uint32_t *>(fy), stream);
+  launch_segment_scan(n, E, unused, unused_pos, static_cast<uint32_t *>(fy), stream);
+  pat_write<<<blocks, 256, 0, stream>>>(n, m, order, nb, accepted, used, acc_pos, unused_pos, out,
+                                        num_indices);
   CUBFF_CUDA_TRY(cudaGetLastError());
   return CUBFF_OK;
 }
