@@ -92,15 +92,15 @@ template <uint32_t stride>
 struct LaneWords {
   uint8_t *s;     // the block, 4-byte aligned
   uint32_t lane;
-  __device__ __forceinline__ uint32_t get(int p) const { return s[at(p)]; }
-  __device__ __forceinline__ void set(int p, uint32_t v) const {
+  __host__ __device__ __forceinline__ uint32_t get(int p) const { return s[at(p)]; }
+  __host__ __device__ __forceinline__ void set(int p, uint32_t v) const {
     s[at(p)] = static_cast<uint8_t>(v);
   }
-  __device__ __forceinline__ uint32_t at(int p) const {
+  __host__ __device__ __forceinline__ uint32_t at(int p) const {
     const uint32_t x = static_cast<uint32_t>(p) & (kPair - 1);
     return ((x >> 2) * stride + lane) * 4 + (x & 3);
   }
-  __device__ __forceinline__ uint32_t &word(uint32_t w) const {
+  __host__ __device__ __forceinline__ uint32_t &word(uint32_t w) const {
     return reinterpret_cast<uint32_t *>(s)[w * stride + lane];
   }
 };

@@ -13,10 +13,13 @@ constexpr int kGroups = kThreads / 128;
 // Shared memory per CTA.  SUBLEQ: two per-lane 128-byte areas per thread (the
 // tape and the cycle check's snapshot); the staged languages: their warps', then
 // the op and command tables.
+struct SubleqMem {  // of a warp
+  uint32_t tapes[kPair / 4 * 32], snaps[kPair / 4 * 32];
+};
 template <int L>
 constexpr size_t epoch_smem_bytes() {
   if constexpr (LangTraits<L>::kStaged) return kThreads / 32 * sizeof(StagedMem<L>) + 512;
-  else return 2 * kGroups * kGroupBytes;
+  else return kThreads / 32 * sizeof(SubleqMem);
 }
 
 __device__ __forceinline__ void load_pair(const uint8_t *soup, uint32_t p1, uint32_t p2,
@@ -25,12 +28,26 @@ __device__ __forceinline__ void load_pair(const uint8_t *soup, uint32_t p1, uint
   const uint4 *g2 = reinterpret_cast<const uint4 *>(soup + uint64_t(p2) * kTape);
 #pragma unroll
   for (int q = 0; q < 4; q++) {
-    const uint4 a = g1[q];
-    const uint4 b = g2[q];
+    const uint4 a = __ldcg(g1 + q);
+    const uint4 b = __ldcg(g2 + q);
     w[4 * q + 0] = a.x; w[4 * q + 1] = a.y; w[4 * q + 2] = a.z; w[4 * q + 3] = a.w;
     w[16 + 4 * q + 0] = b.x; w[16 + 4 * q + 1] = b.y;
     w[16 + 4 * q + 2] = b.z; w[16 + 4 * q + 3] = b.w;
   }
+}
+
+// The pair back: first half, then second half (common_language.h:188-191; of a
+// program paired with itself the second half stays).
+__device__ __forceinline__ void store_pair(uint8_t *soup, uint32_t p1, uint32_t p2,
+                                           const uint32_t w[32]) {
+  uint4 *g1 = reinterpret_cast<uint4 *>(soup + uint64_t(p1) * kTape);
+  uint4 *g2 = reinterpret_cast<uint4 *>(soup + uint64_t(p2) * kTape);
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    g1[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    g2[q] = make_uint4(w[16 + 4 * q], w[16 + 4 * q + 1], w[16 + 4 * q + 2], w[16 + 4 * q + 3]);
 }
 
 // Per-byte mutation of MutateAndRunPrograms (common_language.h:172-180):
@@ -63,37 +80,31 @@ __global__ void __launch_bounds__(kThreads) epoch_kernel(EpochArgs a) {
   const uint64_t npairs = a.n / 2;
   const uint64_t k = uint64_t(blockIdx.x) * kThreads + tid;
   const bool active = k < npairs;
-  const LaneBytes t{smem, lane_base(tid)};
-  const LaneBytes snap{smem + kGroups * kGroupBytes, lane_base(tid)};
+  SubleqMem &mem = reinterpret_cast<SubleqMem *>(smem)[tid >> 5];
+  const LaneWords<32> t{reinterpret_cast<uint8_t *>(mem.tapes), tid & 31};
+  const LaneWords<32> snap{reinterpret_cast<uint8_t *>(mem.snaps), tid & 31};
 
-  uint32_t ops = 0, raw = 0;
+  uint32_t ops = 0;  // (SUBLEQ counts every step)
   if (active) {
     const uint32_t p1 = a.perm[2 * k], p2 = a.perm[2 * k + 1];
     uint32_t w[32];
     load_pair(a.soup, p1, p2, w);
     mutate((a.n * a.epoch_key + k) * kPair, a.mutation_prob, w);
 #pragma unroll
-    for (int i = 0; i < kPair; i++) t.set(i, w[i >> 2] >> ((i & 3) * 8));
+    for (int q = 0; q < 32; q++) t.word(q) = w[q];
     const uint64_t num_indices = a.d_num_indices ? *a.d_num_indices : a.num_indices;
-    if (k < num_indices) ops = evaluate<L>(t, snap, nullptr, &raw);
-#pragma unroll
-    for (int q = 0; q < 32; q++) {
-      w[q] = t.get(4 * q) | (t.get(4 * q + 1) << 8) | (t.get(4 * q + 2) << 16) |
-             (t.get(4 * q + 3) << 24);
+    if (k < num_indices) {
+      SubleqMachine<(L == kRsubleq4)> m;
+      m.begin();
+      while (!m.step(t, snap)) {
+      }
+      ops = m.ops();
     }
-    // First half, then second half (common_language.h:188-191): for a
-    // self-pair the second half wins, as in the reference.
-    uint4 *g1 = reinterpret_cast<uint4 *>(a.soup + uint64_t(p1) * kTape);
-    uint4 *g2 = reinterpret_cast<uint4 *>(a.soup + uint64_t(p2) * kTape);
 #pragma unroll
-    for (int q = 0; q < 4; q++)
-      g1[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      g2[q] = make_uint4(w[16 + 4 * q], w[16 + 4 * q + 1], w[16 + 4 * q + 2],
-                         w[16 + 4 * q + 3]);
+    for (int q = 0; q < 32; q++) w[q] = t.word(q);
+    store_pair(a.soup, p1, p2, w);
   }
-  add_counts(a, ops, raw);
+  add_counts(a, ops, ops);
 }
 
 // The staged languages.  A warp takes kWidth consecutive pairs: all lanes load

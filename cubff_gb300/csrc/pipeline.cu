@@ -85,13 +85,12 @@ constexpr int kCountSlots = kPipeCountSlots;  // per-epoch counter slots (spread
 // No global access is consumed in the iteration that issues it where that
 // can be avoided: queue entries and shuffle indices land in registers read
 // back in a later iteration.  Lane states:
-//   idle -> slot (wait for the entry) -> index -> [stage ->] run [-> long]
-//        -> notify -> idle
+//   idle -> slot (wait for the entry) -> index -> run [-> long] -> notify -> idle
 // and `exhausted` once a claim falls past the queue's last task.
 //
 // How a warp runs its pairs depends on the language family (LaneServer,
 // StagedServer).  Launch-shape knobs (PipeTuning, chosen by the host; the BFF
-// family runs a pair to its end and uses only the grid size):
+// and Forth families run a pair to its end and use only the grid size):
 //  * steps_per_visit: interpreter steps a running lane takes per iteration of
 //    its warp after its first (an iteration lasts as long as its busiest
 //    lane, so a lane given more steps holds its warp-mates, and the pairs
@@ -121,7 +120,7 @@ __device__ __forceinline__ void st_release_u32(uint32_t *p, uint32_t v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-enum : uint32_t { kIdle, kSlot, kIndex, kStage, kRun, kLong, kNotify, kExhausted };
+enum : uint32_t { kIdle, kSlot, kIndex, kRun, kLong, kNotify, kExhausted };
 
 // Per-lane state of a held queue slot and its pair.
 struct Lane {
@@ -295,15 +294,16 @@ __device__ __forceinline__ void store_pair(const PipeSoup &sp, const Lane &ln, F
                         word(19 + 4 * qd));
 }
 
-// A finished pair whose bytes have been written: adds its counts and notifies
-// the consumers of its two programs.
-__device__ __forceinline__ void finish(const PipeSoup &sp, Lane &ln, uint32_t slot_ctr,
-                                       uint32_t ops, uint32_t raw) {
-  if (ln.evaluated) {
-    unsigned long long *c = sp.ops + (uint64_t(ln.e) * kCountSlots + slot_ctr) * 2;
-    if (ops) atomicAdd(c, static_cast<unsigned long long>(ops));
-    if (raw) atomicAdd(c + 1, static_cast<unsigned long long>(raw));
-  }
+__device__ __forceinline__ void add_counts(const PipeSoup &sp, uint32_t e, uint32_t slot_ctr,
+                                           uint32_t ops, uint32_t raw) {
+  unsigned long long *c = sp.ops + (uint64_t(e) * kCountSlots + slot_ctr) * 2;
+  if (ops) atomicAdd(c, static_cast<unsigned long long>(ops));
+  if (raw) atomicAdd(c + 1, static_cast<unsigned long long>(raw));
+}
+
+// A finished pair whose bytes have been written: notifies the consumers of its
+// two programs.
+__device__ __forceinline__ void finish(const PipeSoup &sp, Lane &ln) {
   if (ln.has_next) {
     // The fences order the stores before the increments, and make the earlier
     // producer's stores visible to whoever pushes; between them both increments
@@ -343,24 +343,41 @@ __device__ __forceinline__ void push_ready(const PipeCtx &b, const PipeQueue &q,
   if (ln.state == kNotify) ln.state = kIdle;
 }
 
-// The SUBLEQ languages: one pair per lane.  iterate() is one
-// iteration of the warp; it returns true if the lane made progress.
+// The SUBLEQ languages: one pair per lane, staged and run for some steps in one
+// iteration.  Pairs take 4 steps on average; what an epoch takes is the chain of
+// its latencies (index, programs, steps, two counters, queue) and, now and then, a
+// pair of thousands of steps.  64 epochs of 2^17 subleq programs 4.18 ms (5.79 with
+// tapes staged byte by byte, in an iteration of its own), of 40962 rsubleq4
+// programs 3.27 ms (4.27; 3.44 with 32 pairs to a warp).
+// iterate() is one iteration of the warp; it returns true if the lane made
+// progress.
 template <int L>
 struct LaneServer {
-  LaneMachine<L> m;
+  SubleqMachine<(L == kRsubleq4)> m;
   uint32_t visits;
-  uint4 g[8];
-  uint4 mm;
-  LaneBytes t, stk;
-  const uint8_t *optab;
+  LaneWords<32> t, snap;
 
-  static constexpr uint32_t kWidth = 32;                     // lanes that hold pairs
-  static constexpr size_t kWarpBytes = 2 * kGroupBytes / 4;  // of shared memory
+  static constexpr uint32_t kWidth = 16;                   // lanes that hold pairs
+  static constexpr size_t kWarpBytes = sizeof(SubleqMem);  // of shared memory
 
-  __device__ __forceinline__ LaneServer(uint8_t *smem, const uint8_t *tables, uint32_t tid)
-      : visits(0), t{smem, lane_base(tid)}, stk{smem + kGroups * kGroupBytes, lane_base(tid)},
-        optab(tables) {
-    mm = make_uint4(0, 0, 0, 0);
+  __device__ __forceinline__ LaneServer(uint8_t *smem, const uint8_t *, uint32_t tid)
+      : visits(0), t{smem + (tid >> 5) * kWarpBytes, tid & 31},
+        snap{t.s + sizeof(SubleqMem::tapes), tid & 31} {}
+
+  // Stages the pair of a lane in kIndex: bytes into shared memory, mutations.
+  __device__ __forceinline__ void stage(const PipeSoup &sp, Lane &ln) {
+    uint32_t w[32];
+    load_pair(sp.soup, ln.p1, ln.p2, w);
+    const uint4 mm = __ldg(sp.mutmask + uint64_t(ln.e) * sp.npairs + ln.k);
+#pragma unroll
+    for (int q = 0; q < 32; q++) t.word(q) = w[q];
+    ln.dirty = (mm.x | mm.y | mm.z | mm.w) != 0;
+    if (ln.dirty)
+      mutate_bits(sp, ln, mm, [&](int i, uint32_t v) { t.set(i, v); });
+    const uint64_t num_indices = sp.num_indices ? sp.num_indices[ln.e] : sp.npairs;
+    ln.evaluated = ln.k < num_indices;
+    m.begin();
+    visits = 0;
   }
 
   __device__ __forceinline__ bool iterate(const PipeCtx &b, const PipeQueue &q, Lane &ln,
@@ -377,60 +394,42 @@ struct LaneServer {
       // 2. Waiting for the claimed slot's entry (polled in an earlier iteration).
       progressed = poll_slot(b, q, ln);
     } else if (ln.state == kIndex) {
-      // 3. Shuffle indices landed: order after the producers, issue the gather,
-      //    the mutation mask and the next epoch's positions of both programs.
+      // 3. Shuffle indices landed: gather and stage the pair.
       const PipeSoup &sp = b.soups[ln.si];
       take_index(sp, q, ln);
-      const uint4 *g1 = reinterpret_cast<const uint4 *>(sp.soup + uint64_t(ln.p1) * kTape);
-      const uint4 *g2 = reinterpret_cast<const uint4 *>(sp.soup + uint64_t(ln.p2) * kTape);
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        g[i] = __ldcg(g1 + i);
-        g[4 + i] = __ldcg(g2 + i);
-      }
-      mm = __ldg(sp.mutmask + uint64_t(ln.e) * sp.npairs + ln.k);
-      ln.state = kStage;
-      progressed = true;
-    } else if (ln.state == kStage) {
-      // 4. Stage the pair: bytes into shared memory, mutations.
-      const PipeSoup &sp = b.soups[ln.si];
-#pragma unroll
-      for (int qd = 0; qd < 32; qd++) {
-        const uint32_t w = qd % 4 == 0 ? g[qd / 4].x : qd % 4 == 1 ? g[qd / 4].y
-                         : qd % 4 == 2 ? g[qd / 4].z : g[qd / 4].w;
-#pragma unroll
-        for (int bb = 0; bb < 4; bb++) t.set(4 * qd + bb, w >> (8 * bb));
-      }
-      ln.dirty = (mm.x | mm.y | mm.z | mm.w) != 0;
-      if (ln.dirty)
-        mutate_bits(sp, ln, mm, [&](int i, uint32_t v) { t.set(i, v); });
-      const uint64_t num_indices = sp.num_indices ? sp.num_indices[ln.e] : sp.npairs;
-      ln.evaluated = ln.k < num_indices;
-      m.begin(t, Mask128{0, 0});
-      visits = 0;
+      stage(sp, ln);
       ln.state = kRun;
       progressed = true;
-    } else if (ln.state == kRun) {
-      // 5. A few interpreter steps; on the end, write back and notify.
+    }
+    // 4. Some steps; pairs that ended: write back and notify.
+    bool fin = false;
+    if (ln.state == kRun) {
       progressed = true;
-      bool fin = !ln.evaluated;
+      fin = !ln.evaluated;
       const uint32_t steps = visits ? b.tune.steps_per_visit : b.tune.first_visit_steps;
-      for (uint32_t r = 0; r < steps && !fin; r++) fin = m.step(t, stk, LaneNp{nullptr, 0}, optab);
+      for (uint32_t r = 0; r < steps && !fin; r++) fin = m.step(t, snap);
       visits++;
       if (fin) {
         const PipeSoup &sp = b.soups[ln.si];
-        if (ln.dirty || (ln.evaluated && m.mods() != 0)) {
-          uint32_t w[32];
-#pragma unroll
-          for (int qd = 0; qd < 32; qd++)
-            w[qd] = t.get(4 * qd) | (t.get(4 * qd + 1) << 8) | (t.get(4 * qd + 2) << 16) |
-                    (t.get(4 * qd + 3) << 24);
-          store_pair(sp, ln, [&](int qd) { return w[qd]; });
-        }
-        finish(sp, ln, slot_ctr, m.ops(), m.raw());
+        if (ln.dirty || (ln.evaluated && m.mods != 0))
+          store_pair(sp, ln, [&](int qd) { return t.word(qd); });
+        finish(sp, ln);
       }
     }
-    // 6. Push the consumers whose second input this pair was.
+    // The counts of the pairs that ended, summed over those of one soup and
+    // epoch: pairs are so short that the atomics of each would queue up on the
+    // epoch's few counters (64 epochs of 2^17 subleq programs: 4.50 ms, 5.23 with
+    // them).
+    for (uint32_t left = __ballot_sync(0xffffffffu, fin && ln.evaluated); left != 0;) {
+      const int first = __ffs(left) - 1;
+      const uint32_t e = __shfl_sync(0xffffffffu, ln.e, first);
+      const int si = __shfl_sync(0xffffffffu, ln.si, first);
+      const bool mine = ((left >> lane) & 1) && ln.e == e && ln.si == si;
+      const uint32_t ops = __reduce_add_sync(0xffffffffu, mine ? m.ops() : 0);
+      if (lane == static_cast<uint32_t>(first)) add_counts(b.soups[si], e, slot_ctr, ops, ops);
+      left &= ~__ballot_sync(0xffffffffu, mine);
+    }
+    // 5. Push the consumers whose second input this pair was.
     push_ready(b, q, ln, lane);
     return progressed;
   }
@@ -516,7 +515,10 @@ struct StagedServer {
             reinterpret_cast<const uint32_t *>(mem.warp.T)[lane];
     }
     __syncwarp();  // the warp's stores before the lane's notifications
-    if (lane == src) finish(sp, ln, slot_ctr, c.ops, c.raw);
+    if (lane == src) {
+      if (ln.evaluated) add_counts(sp, ln.e, slot_ctr, c.ops, c.raw);
+      finish(sp, ln);
+    }
   }
 
   __device__ __forceinline__ bool iterate(const PipeCtx &b, const PipeQueue &q, Lane &ln,
@@ -558,7 +560,8 @@ struct StagedServer {
         const PipeSoup &sp = b.soups[ln.si];
         if (ln.dirty || (ln.evaluated && m.mods() != 0))
           store_pair(sp, ln, [&](int qd) { return t.word(qd); });
-        finish(sp, ln, slot_ctr, m.ops(), m.raw());
+        if (ln.evaluated) add_counts(sp, ln.e, slot_ctr, m.ops(), m.raw());
+        finish(sp, ln);
       }
     }
     // 6. Push the consumers whose second input this pair was.
