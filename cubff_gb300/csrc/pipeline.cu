@@ -619,6 +619,13 @@ __global__ void __launch_bounds__(kThreads, (L <= kForthtrivialReset) ? 5 : 4)
   }
 }
 
+// The lanes that a launch has at least, if it has as many pairs: 512 warps of 8,
+// about a block per SM, disturb each other little, so of a small soup all pairs
+// of an epoch are in flight (64 epochs of 1022 bff_noheads programs: 1.74 ms, with
+// half of them 2.05; of 8192: 2.49, 2.62; of 16384, where it would be two blocks
+// per SM: 3.61, 3.49).
+constexpr uint64_t kMinLanes = 4096;
+
 template <int L>
 int launch_pipeline_t(const PipeBatch &b, uint64_t total_pairs, uint32_t lanes_per_pair64,
                       int device, cudaStream_t stream) {
@@ -640,9 +647,9 @@ int launch_pipeline_t(const PipeBatch &b, uint64_t total_pairs, uint32_t lanes_p
   // Lanes in flight: enough to keep the SMs busy, few enough that most held
   // pairs are ready (a lane holding a pair of a later epoch only polls).
   // lanes_per_pair64 (x1/64) is tunable; the default keeps half an epoch of
-  // pairs in flight.
+  // pairs in flight, or kMinLanes of them.
   uint64_t want = (total_pairs * uint64_t(lanes_per_pair64 ? lanes_per_pair64 : 32)) / 64;
-  want = std::max<uint64_t>(want, kThreads);
+  want = std::max<uint64_t>(want, std::min<uint64_t>(total_pairs, kMinLanes));
   const uint64_t per_block = kThreads / 32 * Server<L>::kWidth;
   const uint64_t blocks = (want + per_block - 1) / per_block;
   const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(blocks, resident));

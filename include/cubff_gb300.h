@@ -118,10 +118,11 @@ int cubff_shuffle_indices(uint64_t params_seed, uint64_t first_epoch,
  * identical to the per-epoch launches. */
 /* Launch shape of a pipelined launch.  Results never depend on it; only the
  * time does.  Chosen per launch group by the engine's tuner
- * (cubff_engine_tune), or set by hand.  The BFF family uses only
- * lanes_per_pair64: its warps run each pair to the end once they have it. */
+ * (cubff_engine_tune), or set by hand.  The BFF and Forth families use only
+ * lanes_per_pair64: their warps run each pair to the end once they have it. */
 typedef struct {
-  uint32_t lanes_per_pair64;  /* lanes in flight per 64 pairs of an epoch (grid size)    */
+  uint32_t lanes_per_pair64;  /* lanes in flight per 64 pairs of an epoch (grid size);
+                                 at least 4096 if there are as many pairs               */
   uint32_t steps_per_visit;   /* interpreter steps a lane takes per iteration of its warp
                                  after its first                                        */
   uint32_t claim_min;         /* idle lanes a busy warp needs before it claims new pairs  */
