@@ -478,39 +478,7 @@ int cubff_soup_histogram(cubff_soup *soup, uint64_t *counts) {
 int cubff_eval_pair(int lang, uint8_t *tape, uint64_t *ops, uint64_t *raw) {
   if (lang < 0 || lang >= kNumLangs) return set_error(CUBFF_ENOTFOUND, "unknown language %d", lang);
   if (!tape || !ops) return set_error(CUBFF_EINVAL, "eval_pair: null argument");
-  // Two programs, identity pairing, no mutation: exactly one evaluated pair.
-  uint8_t *d = nullptr;
-  CUBFF_CUDA_TRY(cudaMalloc(&d, kPair + 2 * sizeof(uint32_t) + 2 * sizeof(unsigned long long) + 16));
-  uint8_t *d_soup = d;
-  uint32_t *d_perm = reinterpret_cast<uint32_t *>(d + kPair);
-  unsigned long long *d_cnt = reinterpret_cast<unsigned long long *>(d + kPair + 16);
-  const uint32_t perm[2] = {0, 1};
-  unsigned long long cnt[2] = {0, 0};
-  cudaError_t err = cudaMemcpy(d_soup, tape, kPair, cudaMemcpyHostToDevice);
-  if (err == cudaSuccess) err = cudaMemcpy(d_perm, perm, sizeof(perm), cudaMemcpyHostToDevice);
-  if (err == cudaSuccess) err = cudaMemset(d_cnt, 0, sizeof(cnt));
-  int st = CUBFF_OK;
-  if (err == cudaSuccess) {
-    EpochArgs a;
-    a.soup = d_soup;
-    a.perm = d_perm;
-    a.n = 2;
-    a.num_indices = 1;
-    a.d_num_indices = nullptr;
-    a.epoch_key = 0;
-    a.mutation_prob = 0;
-    a.ops = d_cnt;
-    a.raw = d_cnt + 1;
-    st = launch_epoch(lang, a, nullptr);
-  }
-  if (err == cudaSuccess && st == CUBFF_OK) err = cudaMemcpy(tape, d_soup, kPair, cudaMemcpyDeviceToHost);
-  if (err == cudaSuccess && st == CUBFF_OK) err = cudaMemcpy(cnt, d_cnt, sizeof(cnt), cudaMemcpyDeviceToHost);
-  cudaFree(d);
-  if (err != cudaSuccess) return set_error(CUBFF_EDEVICE, "eval_pair: %s", cudaGetErrorString(err));
-  if (st != CUBFF_OK) return st;
-  *ops = cnt[0];
-  if (raw) *raw = cnt[1];
-  return CUBFF_OK;
+  return eval_pair(lang, tape, ops, raw);
 }
 
 int cubff_eval_selfrep(int lang, const uint8_t *program, uint64_t epoch_key, uint64_t *result) {

@@ -5,6 +5,8 @@
 // The op count is reduced per warp (redux) and added with one atomic per warp,
 // as IncreaseInsnCount does (common_language.h:56-63).
 #include <algorithm>
+#include <atomic>
+#include <cstring>
 #include "internal.h"
 #include "epoch_body.cuh"
 
@@ -157,6 +159,98 @@ __global__ void __launch_bounds__(kThreads, 5) staged_selfrep_kernel(const uint8
   }
 }
 
+// One evaluation of one tape: the call's latency is all there is (the kernel
+// takes 8 us of it for a short program), so the tape comes with the launch and
+// one copy brings back the result: 27 us a call of a bff tape.  (As an epoch of one
+// pair in a buffer of the call's own, with two copies in, a memset and two copies
+// out: 156.)
+struct EvalTape {
+  uint32_t words[kPair / 4];
+};
+struct EvalResult {
+  uint32_t words[kPair / 4];
+  uint32_t ops, raw;
+};
+// Results of calls under way, `kEvalSlots` at most; a call takes one for its own.
+constexpr int kEvalSlots = 16;
+__device__ EvalResult g_eval_results[kEvalSlots];
+
+// One warp: as a pair of an epoch, with the other lanes' places empty.  The
+// result goes to *out, or to the slot if out is null.
+template <int L>
+__global__ void __launch_bounds__(32)
+    eval_kernel(const __grid_constant__ EvalTape tape, int slot, EvalResult *out) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const uint32_t lane = threadIdx.x;
+  EvalResult &res = out ? *out : g_eval_results[slot];
+  if constexpr (LangTraits<L>::kStaged) {
+    constexpr uint32_t kWidth = StagedMem<L>::kWidth;
+    StagedMem<L> &mem = *reinterpret_cast<StagedMem<L> *>(smem);
+    uint8_t *tables = smem + sizeof(StagedMem<L>);
+    const uint8_t *optab = tables, *cmdflag = tables + 256;
+    fill_tables<L>(tables);
+    mem.tapes[lane * kWidth] = tape.words[lane];
+    __syncwarp();
+    const LaneWords<kWidth> t = mem.tape(0), stk = mem.stack(0);
+    Mask128 cmd{0, 0};
+    if (L <= kBffSelfmove) {
+      uint32_t w[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        w[q] = __ballot_sync(0xffffffffu, cmdflag[t.get(32 * q + lane)] != 0);
+      cmd = Mask128{w[0] | static_cast<uint64_t>(w[1]) << 32, w[2] | static_cast<uint64_t>(w[3]) << 32};
+    }
+    using LaneM = typename Stages<L>::Lane;
+    LaneM m;
+    m.status = LaneM::kEnds;
+    if (lane == 0) {
+      m.begin(t, cmd, optab);
+      while (m.status == LaneM::kRuns) m.step(t, stk, optab);
+      if (m.status == LaneM::kJumps) m.resolve(t, optab);
+    }
+    if (__any_sync(0xffffffffu, m.status == LaneM::kJumps)) {
+      const Counts c = run_on_warp(mem, m, 0, lane, optab);
+      res.words[lane] = reinterpret_cast<const uint32_t *>(mem.warp.T)[lane];
+      if (lane == 0) {
+        res.ops = c.ops;
+        res.raw = c.raw;
+      }
+    } else {
+      __syncwarp();
+      res.words[lane] = mem.tapes[lane * kWidth];
+      if (lane == 0) {
+        res.ops = m.ops();
+        res.raw = m.raw();
+      }
+    }
+  } else {
+    SubleqMem &mem = *reinterpret_cast<SubleqMem *>(smem);
+    mem.tapes[lane * 32] = tape.words[lane];
+    __syncwarp();
+    if (lane == 0) {
+      const LaneWords<32> t{reinterpret_cast<uint8_t *>(mem.tapes), 0};
+      const LaneWords<32> snap{reinterpret_cast<uint8_t *>(mem.snaps), 0};
+      SubleqMachine<(L == kRsubleq4)> m;
+      m.begin();
+      while (!m.step(t, snap)) {
+      }
+      res.ops = m.ops();
+      res.raw = m.raw();
+    }
+    __syncwarp();
+    res.words[lane] = mem.tapes[lane * 32];
+  }
+}
+
+template <int L>
+int launch_eval_t(const EvalTape &tape, int slot, EvalResult *out, cudaStream_t stream) {
+  size_t smem = sizeof(SubleqMem);
+  if constexpr (LangTraits<L>::kStaged) smem = sizeof(StagedMem<L>) + 512;
+  eval_kernel<L><<<1, 32, smem, stream>>>(tape, slot, out);
+  CUBFF_CUDA_TRY(cudaGetLastError());
+  return CUBFF_OK;
+}
+
 template <int L>
 int launch_epoch_t(const EpochArgs &a, cudaStream_t stream) {
   const uint64_t npairs = a.n / 2;
@@ -214,6 +308,12 @@ struct EpochLauncher {
   static int run(const EpochArgs &a, cudaStream_t s) { return launch_epoch_t<L>(a, s); }
 };
 template <int L>
+struct EvalLauncher {
+  static int run(const EvalTape &tape, int slot, EvalResult *out, cudaStream_t s) {
+    return launch_eval_t<L>(tape, slot, out, s);
+  }
+};
+template <int L>
 struct SelfrepLauncher {
   static int run(const uint8_t *soup, uint64_t key, uint64_t n, uint64_t count,
                  uint64_t *result, cudaStream_t s) {
@@ -225,6 +325,39 @@ struct SelfrepLauncher {
 
 int launch_epoch(int lang, const EpochArgs &a, cudaStream_t stream) {
   return dispatch_lang<EpochLauncher>(lang, a, stream);
+}
+
+int eval_pair(int lang, uint8_t *tape, uint64_t *ops, uint64_t *raw) {
+  // The slots taken, by device (devices 64 apart share theirs).
+  static std::atomic<uint32_t> taken[64];  // (zero-initialised: static storage)
+  int device = 0;
+  CUBFF_CUDA_TRY(cudaGetDevice(&device));
+  std::atomic<uint32_t> &mine = taken[device & 63];
+  uint32_t seen = mine.load();
+  int slot = 0;
+  do {
+    for (slot = 0; slot < kEvalSlots && ((seen >> slot) & 1); slot++) {
+    }
+  } while (slot < kEvalSlots && !mine.compare_exchange_weak(seen, seen | (1u << slot)));
+  EvalResult *out = nullptr;  // of this call, when all slots are taken
+  if (slot == kEvalSlots) CUBFF_CUDA_TRY(cudaMalloc(&out, sizeof(EvalResult)));
+  EvalTape in;
+  EvalResult res;
+  std::memcpy(in.words, tape, kPair);
+  const cudaStream_t stream = nullptr;
+  const int st = dispatch_lang<EvalLauncher>(lang, in, slot, out, stream);
+  cudaError_t err = cudaSuccess;
+  if (st == CUBFF_OK)
+    err = out ? cudaMemcpy(&res, out, sizeof(res), cudaMemcpyDeviceToHost)
+              : cudaMemcpyFromSymbol(&res, g_eval_results, sizeof(res), slot * sizeof(res));
+  if (out) cudaFree(out);
+  else mine.fetch_and(~(1u << slot));
+  if (st != CUBFF_OK) return st;
+  if (err != cudaSuccess) return set_error(CUBFF_EDEVICE, "eval_pair: %s", cudaGetErrorString(err));
+  std::memcpy(tape, res.words, kPair);
+  *ops = res.ops;
+  if (raw) *raw = res.raw;
+  return CUBFF_OK;
 }
 
 int launch_selfrep(int lang, const uint8_t *soup, uint64_t epoch_key, uint64_t n,

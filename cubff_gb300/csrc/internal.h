@@ -114,6 +114,8 @@ int launch_mutation_masks(uint64_t s0, uint64_t e0, uint32_t n_epochs, uint64_t 
 int launch_inverse(const uint32_t *perm, uint32_t n_epochs, uint64_t n, uint32_t *inv,
                    cudaStream_t stream);
 int launch_epoch(int lang, const EpochArgs &a, cudaStream_t stream);
+// Evaluates a 128-byte tape in place, on the current device.
+int eval_pair(int lang, uint8_t *tape, uint64_t *ops, uint64_t *raw);
 int launch_init(uint64_t key, uint64_t n, uint8_t *soup, int zero_init,
                 uint64_t count, cudaStream_t stream);
 int launch_selfrep(int lang, const uint8_t *soup, uint64_t epoch_key,
