@@ -45,6 +45,38 @@ __host__ __device__ __forceinline__ uint64_t seed_from(uint64_t s0, uint64_t x) 
   return splitmix64(s0 ^ splitmix64(x));
 }
 
+// The 32 draws from key0 on of a pair's mutations (common_language.h:172-180) as
+// a word: bit b is set iff bits [8, 38) of SplitMix64(key0 + b) are below prob,
+// and byte b of the 32 becomes the draw's low byte.  What the keys have in common
+// is taken out: the high half of the sum, its share of the first product, and the
+// shifted-in bits; so a draw is some 16 instructions instead of 25.  (The masks of
+// 20 epochs of 2^17 programs: 129 us, 171 draw by draw.)
+__host__ __device__ __forceinline__ uint32_t mutation_word(uint64_t key0, uint32_t prob) {
+  if (prob >= 1u << 30) return ~0u;
+  const uint64_t z0 = key0 + 0x9e3779b97f4a7c15ULL;
+  const uint32_t lo = static_cast<uint32_t>(z0), hi = static_cast<uint32_t>(z0 >> 32);
+  uint32_t m = 0;
+  if ((lo >> 30) != ((lo + 31) >> 30)) {  // the keys differ above bit 29
+    for (int b = 0; b < 32; b++)
+      m |= static_cast<uint32_t>(
+               (static_cast<uint32_t>(splitmix64(key0 + b) >> 8) & ((1u << 30) - 1)) < prob) << b;
+    return m;
+  }
+  const uint32_t in = hi << 2 | lo >> 30;  // the low half of z >> 30
+  const uint64_t of_hi = static_cast<uint64_t>((hi ^ (hi >> 30)) * 0x1ce4e5b9u) << 32;
+#pragma unroll 8
+  for (int b = 0; b < 32; b++) {
+    const uint32_t x = (lo + b) ^ in;
+    uint64_t z = static_cast<uint64_t>(x) * 0x1ce4e5b9u + of_hi;
+    z += static_cast<uint64_t>(x * 0xbf58476du) << 32;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebULL;
+    // Bits [6, 38) of the draw: prob * 4 has none of the lowest two.
+    const uint32_t v = static_cast<uint32_t>(z >> 6) ^ static_cast<uint32_t>(z >> 37);
+    m |= static_cast<uint32_t>(v < prob * 4) << b;
+  }
+  return m;
+}
+
 // Shared-memory tape layout.  Threads come in groups of four warps.  The
 // four warps of a group share one 16 KiB block in which byte p of the tape of
 // lane l of warp w sits at  p * 128 + l * 4 + (w & 3):  every lane of a warp

@@ -50,16 +50,14 @@ __device__ __forceinline__ void store_pair(uint8_t *soup, uint32_t p1, uint32_t 
     g2[q] = make_uint4(w[16 + 4 * q], w[16 + 4 * q + 1], w[16 + 4 * q + 2], w[16 + 4 * q + 3]);
 }
 
-// Per-byte mutation of MutateAndRunPrograms (common_language.h:172-180):
-// r = SplitMix64(key0 + i); if bits [8, 38) of r < mutation_prob, byte i = r.
-__device__ __forceinline__ void mutate(uint64_t key0, uint32_t prob, uint32_t w[32]) {
-#pragma unroll
-  for (int i = 0; i < kPair; i++) {
-    const uint64_t r = splitmix64(key0 + i);
-    if (static_cast<uint32_t>(r >> 8) % (1u << 30) < prob) {
-      const int sh = (i & 3) * 8;
-      w[i >> 2] = (w[i >> 2] & ~(0xFFu << sh)) | ((static_cast<uint32_t>(r) & 0xFFu) << sh);
-    }
+// Sets the bytes of the 32 draws from key0 on that mutate: set(b, byte).
+template <class F>
+__device__ __forceinline__ void mutate(uint64_t key0, uint32_t prob, F set) {
+  uint32_t bits = mutation_word(key0, prob);
+  while (bits) {
+    const int b = __ffs(bits) - 1;
+    bits &= bits - 1;
+    set(b, static_cast<uint32_t>(splitmix64(key0 + b)) & 0xFFu);
   }
 }
 
@@ -89,9 +87,12 @@ __global__ void __launch_bounds__(kThreads) epoch_kernel(EpochArgs a) {
     const uint32_t p1 = a.perm[2 * k], p2 = a.perm[2 * k + 1];
     uint32_t w[32];
     load_pair(a.soup, p1, p2, w);
-    mutate((a.n * a.epoch_key + k) * kPair, a.mutation_prob, w);
 #pragma unroll
     for (int q = 0; q < 32; q++) t.word(q) = w[q];
+    const uint64_t key0 = (a.n * a.epoch_key + k) * kPair;
+#pragma unroll 1
+    for (int q = 0; q < kPair; q += 32)
+      mutate(key0 + q, a.mutation_prob, [&](int i, uint32_t v) { t.set(q + i, v); });
     const uint64_t num_indices = a.d_num_indices ? *a.d_num_indices : a.num_indices;
     if (k < num_indices) {
       SubleqMachine<(L == kRsubleq4)> m;
@@ -108,7 +109,7 @@ __global__ void __launch_bounds__(kThreads) epoch_kernel(EpochArgs a) {
 }
 
 // The staged languages.  A warp takes kWidth consecutive pairs: all lanes load
-// and mutate them together (a pair's 128 mutation draws are four per lane),
+// and mutate them together (32 of their draws per lane),
 // its first lanes run the first part of one each, and the pairs that go on run
 // on the whole warp one after the other.  The launch lasts as long as its
 // longest pairs, so a warp holds few.
@@ -139,19 +140,14 @@ __global__ void __launch_bounds__(kThreads, 5) staged_epoch_kernel(EpochArgs a) 
   for (uint32_t j = 0; j < kWidth; j++)
     if (j < count) mem.tapes[lane * kWidth + j] = soup[uint64_t(mine[j]) * 16 + (lane & 15)];
   __syncwarp();
-  // Mutations (common_language.h:172-180).
-  if (a.mutation_prob != 0) {
-    for (uint32_t j = 0; j < count; j++) {
-      const uint64_t key = (a.n * a.epoch_key + k0 + j) * kPair + lane;
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const uint64_t r = splitmix64(key + 32 * q);
-        if (static_cast<uint32_t>(r >> 8) % (1u << 30) < a.mutation_prob)
-          mem.tape(j).set(32 * q + lane, static_cast<uint32_t>(r));
-      }
-    }
-    __syncwarp();
+  // Mutations: lane l draws for 32 bytes of pair l / 4.
+  static_assert(kWidth * 4 == 32);
+  if (lane / 4 < count) {
+    const uint32_t q = lane % 4 * 32;
+    mutate((a.n * a.epoch_key + k0 + lane / 4) * kPair + q, a.mutation_prob,
+           [&](int i, uint32_t v) { mem.tape(lane / 4).set(q + i, v); });
   }
+  __syncwarp();
   const uint64_t num_indices = a.d_num_indices ? *a.d_num_indices : a.num_indices;
   LaneM m;
   m.status = LaneM::kEnds;

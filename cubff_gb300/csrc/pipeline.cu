@@ -46,23 +46,21 @@ constexpr uint64_t kDefaultWaitLimitNs = 10ull * 1000 * 1000 * 1000;
 std::atomic<uint64_t> g_wait_limit_ns{kDefaultWaitLimitNs};
 
 // Mutation masks of MutateAndRunPrograms (common_language.h:172-180) for
-// epochs [e0, e0 + E): bit i of mask[e][k] is set iff draw i of pair k,
-// r = SplitMix64((n * seed(e0 + e) + k) * 128 + i), has bits [8, 38) below
-// mutation_prob.  One thread per 32 draws; words are stored coalesced.
-__global__ void mutation_mask_kernel(uint64_t s0, uint64_t e0, uint64_t npairs, uint64_t words,
-                                     uint64_t n, uint32_t prob, uint32_t *out) {
-  const uint64_t idx = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= words) return;
-  const uint64_t pair = idx >> 2, q = idx & 3;
-  const uint64_t e = pair / npairs, k = pair - e * npairs;
-  const uint64_t key0 = (n * seed_from(s0, e0 + e) + k) * kPair + q * 32;
-  uint32_t m = 0;
-#pragma unroll 8
-  for (int b = 0; b < 32; b++) {
-    const uint64_t r = splitmix64(key0 + b);
-    m |= static_cast<uint32_t>((static_cast<uint32_t>(r >> 8) % (1u << 30)) < prob) << b;
+// epochs [e0, e0 + E): bit i of mask[e][k] is set iff draw i of pair k, with key
+// (n * seed(e0 + e) + k) * 128 + i, mutates byte i.  Bound by the draws' integer
+// arithmetic; a thread takes a pair, so that the epoch's seed costs little.
+__global__ void __launch_bounds__(256)
+    mutation_mask_kernel(uint64_t s0, uint64_t e0, uint32_t n_epochs, uint64_t npairs, uint64_t n,
+                         uint32_t prob, uint4 *out) {
+  const uint64_t k = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k >= npairs) return;
+  for (uint32_t e = blockIdx.y; e < n_epochs; e += gridDim.y) {
+    const uint64_t key0 = (n * seed_from(s0, e0 + e) + k) * kPair;
+    uint32_t m[4];
+#pragma unroll 1
+    for (int q = 0; q < 4; q++) m[q] = mutation_word(key0 + 32 * q, prob);
+    out[e * npairs + k] = make_uint4(m[0], m[1], m[2], m[3]);
   }
-  out[idx] = m;
 }
 
 constexpr int kCountSlots = kPipeCountSlots;  // per-epoch counter slots (spread the atomics)
@@ -722,10 +720,10 @@ int launch_pipeline(const PipeBatch &b, uint64_t total_pairs, uint32_t lanes_per
 
 int launch_mutation_masks(uint64_t s0, uint64_t e0, uint32_t n_epochs, uint64_t n, uint32_t prob,
                           uint4 *out, cudaStream_t stream) {
-  const uint64_t words = (n / 2) * n_epochs * 4;
-  if (words == 0) return CUBFF_OK;
-  mutation_mask_kernel<<<static_cast<unsigned>((words + 255) / 256), 256, 0, stream>>>(
-      s0, e0, n / 2, words, n, prob, reinterpret_cast<uint32_t *>(out));
+  const uint64_t npairs = n / 2;
+  if (npairs == 0 || n_epochs == 0) return CUBFF_OK;
+  const dim3 grid(static_cast<unsigned>((npairs + 255) / 256), std::min(n_epochs, 65535u));
+  mutation_mask_kernel<<<grid, 256, 0, stream>>>(s0, e0, n_epochs, npairs, n, prob, out);
   CUBFF_CUDA_TRY(cudaGetLastError());
   return CUBFF_OK;
 }
