@@ -599,7 +599,10 @@ struct ForthWarp {
           visit(st.pos);
           if (st.i >= kStepLimit) return;
         }
-        if (--plain == 0) decode();
+        if (--plain == 0) {
+          decode();
+          last = -1;  // (the last step's visit, if any, was for this very state)
+        }
         continue;
       }
       const uint32_t e = m.E[st.pos], r = m.R[st.pos];
