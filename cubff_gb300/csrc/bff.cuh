@@ -157,9 +157,10 @@ static_assert(sizeof(BffMem) % 16 == 0, "BffMem");
 //    iterations in a row without a changed byte and without leaving mean that
 //    none will ever come: the loop runs to the step limit.
 //
-// Uniform stores are made by all lanes together (the same value to the same
-// place; every branch here is uniform, so the lanes stay together), and every
-// lane reads its own; lane-wise ones are followed by a sync.
+// Uniform stores are made by every lane (the same value to the same place) after
+// a sync: by then all lanes have read what the store changes and made the one
+// before, so a lane that is ahead or behind reads nothing else, and every lane
+// reads at least its own.  Lane-wise stores are between two syncs.
 template <class W, int kLogic, uint32_t kNullMask>
 struct BffWarp {
   static constexpr uint32_t kSettle = 8;  // micro-op loop iterations before the first visit
@@ -255,6 +256,7 @@ struct BffWarp {
 
   // Writes v over o != v at position p.
   __host__ __device__ __forceinline__ void write(int p, uint32_t o, uint32_t v) {
+    w.sync();
     m.T[p] = static_cast<uint8_t>(v);
     st.mods++;
     if (optab[v] != optab[o]) changed_op(p, p);
@@ -312,6 +314,7 @@ struct BffWarp {
         if (b >= 0) r = static_cast<uint32_t>(b);
       }
     }
+    w.sync();
     m.M[q] = static_cast<uint16_t>(r);
     if (r != kNone) m.M[r & 127] = static_cast<uint16_t>(static_cast<uint32_t>(q) | (r & 128));
     return r;
@@ -352,6 +355,7 @@ struct BffWarp {
   // Compiles the loop from '[' at s to ']' at e, with no brackets between and
   // no op changed since the decode; false when it has too many micro-ops.
   __host__ __device__ __forceinline__ bool compile(int s, int e) {
+    w.sync();
     le = -1;
     int k = 0, d0 = 0, d1 = 0, m0 = 0, m1 = 0;
     uint32_t cmds = 1, last = kNoop, u = 0, first = 0;
@@ -392,6 +396,7 @@ struct BffWarp {
         last = kNoop;
       }
     }
+    w.sync();
     ls = s;
     le = e;
     net0 = m0;
@@ -633,6 +638,7 @@ struct BffWarp {
             if (lo <= hi) changed_op(lo, hi);
             return bail(k);
           }
+          w.sync();
           m.T[p] = static_cast<uint8_t>(v);
           st.mods++;
           lo = p < lo ? p : lo;
@@ -642,7 +648,6 @@ struct BffWarp {
       } while (((u >> 16) & 3) != kTest);
       st.h0 = (st.h0 + static_cast<int>(u)) & (kPair - 1);
       st.h1 = (st.h1 + static_cast<int>(u >> 8)) & (kPair - 1);
-      w.sync();
       st.i += len;
       st.n += lcmds;
       from = le;
@@ -790,7 +795,6 @@ struct BffWarp {
         from = st.q;
         next = en >> 8;
       } else {
-        w.sync();
         from = bracket(c, &back);
         if (from == kEnd) return;
         if (from != kRedo) {

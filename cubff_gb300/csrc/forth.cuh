@@ -18,16 +18,20 @@
 namespace cubff {
 
 template <class Tape>
-static __host__ __device__ __noinline__ void forth_reset(const Tape t, int pos) {
+static __host__ __device__ __noinline__ uint64_t reset_seed(const Tape t) {
   uint64_t seed = 0;
   for (int i = 0; i < kPair; i++) seed = splitmix64(seed ^ t.get(i));
+  return seed;
+}
+template <class Tape>
+static __host__ __device__ __noinline__ void reset_with(const Tape t, uint64_t seed, int pos) {
   for (int i = 0; i < kTape; i++)
     t.set(i, static_cast<uint32_t>(splitmix64(seed * kTape * kTape +
                                               static_cast<uint64_t>(pos * kTape) +
                                               static_cast<uint64_t>(i))));
 }
 
-// A tape that all lanes of a warp access alike, or a stack.
+// A tape that all lanes of a warp access alike.
 struct SharedBytes {
   uint8_t *s;
   __host__ __device__ __forceinline__ uint32_t get(int p) const { return s[p & (kPair - 1)]; }
@@ -56,22 +60,40 @@ struct Written {
     return (lo0 <= hi && hi0 >= lo) || (lo1 <= hi && hi1 >= lo);
   }
 };
-// A shared tape that notes what is written.
+// A warp's tape: all lanes have read before any writes (ForthWarp), and what is
+// written is noted.
+template <class W>
 struct TrackedBytes {
+  const W &w;
   uint8_t *s;
   Written &written;
   __host__ __device__ __forceinline__ uint32_t get(int p) const { return s[p & (kPair - 1)]; }
   __host__ __device__ __forceinline__ void set(int p, uint32_t v) const {
+    w.sync();
     s[p & (kPair - 1)] = static_cast<uint8_t>(v);
     written.add(p);
   }
 };
+// A warp's stack.
+template <class W>
+struct StackBytes {
+  const W &w;
+  uint8_t *s;
+  __host__ __device__ __forceinline__ uint32_t get(int p) const { return s[p & (kPair - 1)]; }
+  __host__ __device__ __forceinline__ void set(int p, uint32_t v) const {
+    w.sync();
+    s[p & (kPair - 1)] = static_cast<uint8_t>(v);
+  }
+};
 template <class Tape>
 __host__ __device__ __forceinline__ void reset_tape(const Tape t, int pos) {
-  forth_reset(t, pos);
+  reset_with(t, reset_seed(t), pos);
 }
-__host__ __device__ __forceinline__ void reset_tape(const TrackedBytes t, int pos) {
-  forth_reset(SharedBytes{t.s}, pos);
+template <class W>
+__host__ __device__ __forceinline__ void reset_tape(const TrackedBytes<W> t, int pos) {
+  const uint64_t seed = reset_seed(SharedBytes{t.s});
+  t.w.sync();
+  reset_with(SharedBytes{t.s}, seed, pos);
   t.written.lo0 = 0;
   t.written.hi0 = kTape - 1;
 }
@@ -284,6 +306,10 @@ struct alignas(16) ForthMem {
 // position and depth it repeats to the step limit whatever is on the stack;
 // and one that leaves the stack deeper by d without having met its bottom
 // repeats, d deeper each time, until the stack overflows.
+//
+// Stores to the tape and the stack are made by every lane alike, each after a
+// sync (as in BffWarp): by then all lanes have read what it changes and made the
+// store before it.
 template <class W, bool kWithReset>
 struct ForthWarp {
   static constexpr uint32_t kConstant = 64, kOut = 62, kPending = 63;  // codes
@@ -439,6 +465,7 @@ struct ForthWarp {
   __host__ __device__ __forceinline__ void write(int a, uint32_t v) {
     blind = false;
     if (m.T[a] != v) {
+      w.sync();
       m.T[a] = static_cast<uint8_t>(v);
       ln.st.mods++;
       written.add(a);
@@ -462,7 +489,10 @@ struct ForthWarp {
       st.overflow = true;
       return;
     }
-    if (st.sp >= 2) m.stk[st.sp - 2] = static_cast<uint8_t>(st.r1);
+    if (st.sp >= 2) {
+      w.sync();
+      m.stk[st.sp - 2] = static_cast<uint8_t>(st.r1);
+    }
     st.r1 = st.r0;
     st.r0 = v;
     st.sp++;
@@ -561,11 +591,9 @@ struct ForthWarp {
     }
   }
   __host__ __device__ __forceinline__ void reset() {
-    forth_reset(SharedBytes{m.T}, ln.st.pos - 1);
+    reset_tape(TrackedBytes<W>{w, m.T, written}, ln.st.pos - 1);
     ln.st.mods++;
     blind = false;
-    written.lo0 = 0;
-    written.hi0 = kTape - 1;
   }
 
   // The state at the start of a program.
@@ -589,12 +617,11 @@ struct ForthWarp {
     uint32_t plain = 0;  // steps to take one by one
     int last = -1;
     while (true) {
-      w.sync();
       if (plain != 0) {
-        const TrackedBytes t{m.T, written};
+        const TrackedBytes<W> t{w, m.T, written};
         bool back;
         blind = false;  // (not tracked here)
-        if (ln.step(t, SharedBytes{m.stk}, optab, back)) return;
+        if (ln.step(t, StackBytes<W>{w, m.stk}, optab, back)) return;
         if (back) {
           visit(st.pos);
           if (st.i >= kStepLimit) return;
