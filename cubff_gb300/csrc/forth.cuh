@@ -17,28 +17,35 @@
 
 namespace cubff {
 
+// Byte i that a reset at position pos writes.
+__host__ __device__ __forceinline__ uint8_t reset_byte(uint64_t seed, int pos, uint32_t i) {
+  return static_cast<uint8_t>(
+      splitmix64(seed * kTape * kTape + static_cast<uint64_t>(pos * kTape) + i));
+}
 template <class Tape>
-static __host__ __device__ __noinline__ uint64_t reset_seed(const Tape t) {
+static __host__ __device__ __noinline__ void forth_reset(const Tape t, int pos) {
   uint64_t seed = 0;
   for (int i = 0; i < kPair; i++) seed = splitmix64(seed ^ t.get(i));
+  for (int i = 0; i < kTape; i++) t.set(i, reset_byte(seed, pos, i));
+}
+// The seed of a reset on the whole warp, of a tape in 4-byte aligned words: a chain
+// of 128 draws, for which the next word is on its way.  (The 64 bytes written are
+// then two to a lane.  Soups of forthtrivial_reset that had evolved for 1024 epochs,
+// 64 epochs: 2^14 programs 119 ms, 2^17 191 ms; byte by byte on every lane 188 and
+// 288, one pair a lane 147 and 187.)
+static __host__ __device__ __noinline__ uint64_t reset_seed(const uint8_t *tape) {
+  const uint32_t *words = reinterpret_cast<const uint32_t *>(tape);
+  uint64_t seed = 0;
+  uint32_t next = words[0];
+  for (int q = 0; q < kPair / 4; q++) {
+    const uint32_t w = next;
+    next = words[(q + 1) % (kPair / 4)];
+#pragma unroll
+    for (int b = 0; b < 4; b++) seed = splitmix64(seed ^ ((w >> (8 * b)) & 0xFF));
+  }
   return seed;
 }
-template <class Tape>
-static __host__ __device__ __noinline__ void reset_with(const Tape t, uint64_t seed, int pos) {
-  for (int i = 0; i < kTape; i++)
-    t.set(i, static_cast<uint32_t>(splitmix64(seed * kTape * kTape +
-                                              static_cast<uint64_t>(pos * kTape) +
-                                              static_cast<uint64_t>(i))));
-}
 
-// A tape that all lanes of a warp access alike.
-struct SharedBytes {
-  uint8_t *s;
-  __host__ __device__ __forceinline__ uint32_t get(int p) const { return s[p & (kPair - 1)]; }
-  __host__ __device__ __forceinline__ void set(int p, uint32_t v) const {
-    s[p & (kPair - 1)] = static_cast<uint8_t>(v);
-  }
-};
 // Positions written in each half of a tape: [lo, hi] (none: lo > hi).
 struct Written {
   int lo0, hi0, lo1, hi1;
@@ -87,13 +94,16 @@ struct StackBytes {
 };
 template <class Tape>
 __host__ __device__ __forceinline__ void reset_tape(const Tape t, int pos) {
-  reset_with(t, reset_seed(t), pos);
+  forth_reset(t, pos);
 }
 template <class W>
 __host__ __device__ __forceinline__ void reset_tape(const TrackedBytes<W> t, int pos) {
-  const uint64_t seed = reset_seed(SharedBytes{t.s});
+  const uint64_t seed = reset_seed(t.s);
   t.w.sync();
-  reset_with(SharedBytes{t.s}, seed, pos);
+  t.w.each([&](uint32_t l) {
+    for (uint32_t i = l; i < kTape; i += kWarp) t.s[i] = reset_byte(seed, pos, i);
+  });
+  t.w.sync();
   t.written.lo0 = 0;
   t.written.hi0 = kTape - 1;
 }
