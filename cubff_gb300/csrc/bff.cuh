@@ -459,7 +459,11 @@ struct BffWarp {
 
   // At most one copy.  Lane j is iteration j: it reads from src + j * ds,
   // writes to dst + j * dd, and the ']' reads test + j * net0.  Iterations are
-  // cut where one would read what an earlier one of the same batch changed.
+  // cut where one would read what an earlier one of the same batch changed: `most`
+  // after the first that changes a byte.  (Heads that part ways, as in a copy
+  // backwards, leave just that one, but once copied nothing changes any more: 64
+  // epochs of 2^17 bff_noheads_4bit programs evolved for 4096 58 ms, 96 with one
+  // iteration at a time throughout.)
   __host__ __device__ __forceinline__ int loop_copy(uint32_t len) {
     const uint32_t u = m.P[0], act = (u >> 16) & 3;
     const bool to1 = act == kTo1;
@@ -495,7 +499,7 @@ struct BffWarp {
       if (st.i + kWarp * len > kStepLimit) room = (kStepLimit - st.i) / len;
       const int t0 = st.h0 + net0, s0 = act == kTo0 ? st.h1 + a1 : st.h0 + a0;
       const int w0 = to1 ? st.h1 + a1 : st.h0 + a0;
-      uint32_t cut = most < room ? most : room;
+      uint32_t cut = room;
       const auto at = w.map([&](uint32_t l) { return (w0 + dd * static_cast<int>(l)) & (kPair - 1); });
       const auto x = w.map([&](uint32_t l) {
         return uint32_t(m.T[(s0 + ds * static_cast<int>(l)) & (kPair - 1)]);
@@ -506,6 +510,7 @@ struct BffWarp {
         return copies && p == at(l) ? x(l) : uint32_t(m.T[p]);
       });
       uint32_t changed = copies ? w.ballot([&](uint32_t l) { return x(l) != y(l); }) : 0u;
+      if (changed != 0 && low32(changed) + most < cut) cut = low32(changed) + most;
       if (copies && (changed != 0 || dd == 0)) {
         if (dd == 0) {
           // One byte written over and over: cut before an iteration that reads

@@ -25,6 +25,7 @@ struct Schedule {
   int kind[kWarp];          // of the collective a lane waits at
   bool value[kWarp];
   uint32_t result, current;
+  uint32_t rounds;          // collectives of the last run
   void (*body)(uint32_t);
 };
 thread_local Schedule g;
@@ -57,6 +58,7 @@ bool run_lanes(void (*body)(uint32_t), uint32_t order) {
     g.done[l] = false;
   }
   for (uint64_t round = 0;; round++) {
+    g.rounds = static_cast<uint32_t>(round);
     const uint32_t turn = order < 2 ? (order ? 31 : 0)
                                     : static_cast<uint32_t>(splitmix64(order + round)) & 31;
     uint32_t finished = 0, ballot = 0;
@@ -213,6 +215,10 @@ int run_lang(uint32_t stride, uint8_t *tape, uint32_t lane, uint32_t order, Coun
 }
 
 }  // namespace
+
+// Collectives (syncs and votes) of the last run's second stage: its work, on
+// every lane alike.
+extern "C" uint32_t lanes_rounds() { return g.rounds; }
 
 // Evaluates a tape in place, on lane `lane` of words interleaved by `stride`
 // (8, 16 or 32), the long part with the lanes taking turns in `order`.

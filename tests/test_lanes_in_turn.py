@@ -114,3 +114,15 @@ def test_subleq_on_words_matches_oracle(lanes_lib, lang, stride):
         tape = np.zeros(128, dtype=np.uint8)
         tape[:len(prog)] = np.frombuffer(prog, dtype=np.uint8)
         check(lanes_lib, lang, tape, stride, 5, 0)
+
+
+def test_copy_backwards_of_equal_bytes_runs_in_batches(lanes_lib):
+    """A copy loop whose heads part ways on a palindrome: nothing changes, so its
+    iterations run 32 at a time until the heads have been around."""
+    half = np.arange(1, 65, dtype=np.uint8) + 150
+    tape = np.concatenate([half, half[::-1]])
+    prog = b"+[{.>]"
+    tape[:len(prog)] = list(prog)
+    tape[128 - len(prog):] = list(prog[::-1])
+    check(lanes_lib, "bff_noheads", tape, 8, 3, 0)
+    assert 0 < lanes_lib.lanes_rounds() < 100, lanes_lib.lanes_rounds()
