@@ -8,7 +8,8 @@
 //
 // Two machines that a program runs on in turn:
 //  * BffLane, one pair per lane: runs a program until it ends or first jumps
-//    (most random programs never do);
+//    (most random programs never do), and on to its end where most of a warp's
+//    programs jump (bff8, bff8_noheads: soups of self-replicators);
 //  * BffWarp, one pair per warp, which takes over from there.
 #pragma once
 
@@ -29,6 +30,13 @@ struct BffState {
   uint32_t mods;     // writes that changed a byte
 };
 
+// What a lane's cycle check keeps of a program: the state at a taken backward
+// jump (q -1: none yet), on Brent's schedule (cycle.cuh).
+struct BffCycle {
+  int q, h0, h1;
+  uint32_t i, n, mods, power, lam;
+};
+
 // The forward part of a program on one lane.  The lanes of a warp are at
 // different commands, so a step is one straight line of instructions for all
 // of them: head moves and value writes all computed and selected.  S marks
@@ -37,6 +45,7 @@ struct BffState {
 // a run of no-ops is crossed by finding the next one.
 template <bool kHeads, int kLogic, uint32_t kNullMask>
 struct BffLane {
+  using Cycle = BffCycle;
   enum Status : uint32_t { kRuns, kEnds, kJumps };
   BffState st;
   uint32_t status;
@@ -74,6 +83,12 @@ struct BffLane {
   template <class Tape>
   __host__ __device__ __forceinline__ void step(const Tape t, const Tape,
                                                 const uint8_t *__restrict__ optab) {
+    act(t, optab);
+    fetch(t, optab, st.q + 1);
+  }
+  // What the command at q does but for a jump.
+  template <class Tape>
+  __host__ __device__ __forceinline__ void act(const Tape t, const uint8_t *__restrict__ optab) {
     st.h0 = (st.h0 + (c == kInc0) - (c == kDec0)) & (kPair - 1);
     st.h1 = (st.h1 + (c == kInc1 || (kLogic == kLogicSelfmove && c == kCopy10)) - (c == kDec1)) &
             (kPair - 1);
@@ -88,7 +103,6 @@ struct BffLane {
     }
     st.n += c < kNull;
     st.i++;
-    fetch(t, optab, st.q + 1);
   }
 
   // A taken ']' with no '[' before it ends the program (bff8: one that would
@@ -108,9 +122,60 @@ struct BffLane {
     status = kEnds;
   }
 
+  __host__ __device__ __forceinline__ static void begin_cycle(BffCycle &y) {
+    y.q = -1;
+    y.power = 1;
+    y.lam = 0;
+  }
+  // For a program that goes on: the command at q, which may jump; kEnds when it was
+  // the program's last.
+  template <class Tape>
+  __host__ __device__ __forceinline__ void step_on(const Tape t, const Tape,
+                                                   const uint8_t *__restrict__ optab,
+                                                   BffCycle &y) {
+    static_assert(kLogic == kLogicJump8);  // (jumps that need no match)
+    const int q = st.q, from = status != kJumps ? q : c == kLoopStart ? q + 8 : q - 8;
+    act(t, optab);
+    if (from < 0 || from >= kPair) {
+      status = kEnds;
+      return;
+    }
+    fetch(t, optab, from + 1);
+    if (from < q && status != kEnds && st.i < kStepLimit) visit(y);
+    if (st.i >= kStepLimit) status = kEnds;
+  }
+  // On to a command, for the warp to go on from.
+  template <class Tape>
+  __host__ __device__ __forceinline__ void settle(const Tape t, const Tape stk,
+                                                  const uint8_t *__restrict__ optab) {
+    while (status == kRuns && c >= kNull) {
+      step(t, stk, optab);
+      if (st.i >= kStepLimit) status = kEnds;
+    }
+  }
+  __host__ __device__ __forceinline__ void visit(BffCycle &y) {
+    if (st.q == y.q && st.h0 == y.h0 && st.h1 == y.h1 && st.mods == y.mods) {
+      const uint32_t len = st.i - y.i, k = (kStepLimit - st.i) / len;
+      st.i += k * len;
+      st.n += k * (st.n - y.n);
+    }
+    if (++y.lam == y.power) {
+      y.q = st.q;
+      y.h0 = st.h0;
+      y.h1 = st.h1;
+      y.i = st.i;
+      y.n = st.n;
+      y.mods = st.mods;
+      y.power <<= 1;
+      y.lam = 0;
+    }
+  }
+
   __host__ __device__ __forceinline__ const BffState &state() const { return st; }
   __host__ __device__ __forceinline__ uint32_t ops() const { return st.n; }
-  __host__ __device__ __forceinline__ uint32_t raw() const { return st.i; }
+  __host__ __device__ __forceinline__ uint32_t raw() const {
+    return st.i < kStepLimit ? st.i : kStepLimit;
+  }
   __host__ __device__ __forceinline__ uint32_t mods() const { return st.mods; }
 };
 

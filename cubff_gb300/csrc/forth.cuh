@@ -8,7 +8,8 @@
 //
 // Two machines that a program runs on in turn:
 //  * ForthFirst, one pair per lane, for a program's first steps (most random
-//    programs end in them);
+//    programs end in them), and for the rest where most of a warp's programs
+//    go on (a soup of self-replicators);
 //  * ForthWarp, one pair per warp, which takes over from there.
 #pragma once
 
@@ -254,9 +255,19 @@ struct ForthLane {
   }
 };
 
-// The first steps of a program on one lane.
+// What a lane's cycle check keeps of a program.
+struct ForthCycle {
+  int pos, sp;  // of the snapshot (pos -1: none)
+  uint32_t i, nops, mods, top, power, lam;
+  uint64_t mem;
+};
+
+// The first steps of a program on one lane; and any number more (step_on), with
+// exact cycle fast-forward at backward jumps on Brent's schedule (cycle.cuh), for
+// stacks of up to 8 entries, compared byte by byte, and an unchanged tape.
 template <bool kWithReset>
 struct ForthFirst {
+  using Cycle = ForthCycle;
   // Most random programs end within 24 steps (90 % of those of a soup of 2^15
   // forth programs after 256 epochs).
   static constexpr uint32_t kSteps = 24;
@@ -277,6 +288,56 @@ struct ForthFirst {
   }
   template <class Tape>
   __host__ __device__ __forceinline__ void resolve(const Tape, const uint8_t *) {}
+
+  __host__ __device__ __forceinline__ static void begin_cycle(ForthCycle &y) {
+    y.pos = -1;
+    y.power = 1;
+    y.lam = 0;
+  }
+  // A step of a program that goes on (kJumps); kEnds when it was the last.
+  template <class Tape>
+  __host__ __device__ __forceinline__ void step_on(const Tape t, const Tape stk,
+                                                   const uint8_t *__restrict__ optab,
+                                                   ForthCycle &y) {
+    bool back;
+    bool ends = ln.step(t, stk, optab, back);
+    if (!ends && back) {
+      visit(stk, y);
+      ends = ln.st.i >= kStepLimit;
+    }
+    if (ends) status = kEnds;
+  }
+  template <class Tape>
+  __host__ __device__ __forceinline__ void settle(const Tape, const Tape, const uint8_t *) {}
+  // stack[0 .. sp - 2), the entries below the registers, packed.
+  template <class Tape>
+  __host__ __device__ __forceinline__ uint64_t below(const Tape stk) const {
+    uint64_t w = 0;
+    for (int j = 0; j < ln.st.sp - 2; j++) w |= static_cast<uint64_t>(stk.get(j)) << (8 * j);
+    return w;
+  }
+  template <class Tape>
+  __host__ __device__ __forceinline__ void visit(const Tape stk, ForthCycle &y) {
+    ForthState &st = ln.st;
+    const uint32_t top = (st.sp >= 1 ? st.r0 : 0u) | (st.sp >= 2 ? st.r1 : 0u) << 8;
+    if (st.pos == y.pos && top == y.top && st.sp == y.sp && st.mods == y.mods &&
+        (st.sp <= 2 || below(stk) == y.mem)) {
+      const uint32_t len = st.i - y.i, k = (kStepLimit - st.i) / len;
+      st.i += k * len;
+      st.nops += k * (st.nops - y.nops);
+    }
+    if (++y.lam == y.power) {
+      y.pos = st.sp <= 8 ? st.pos : -1;  // larger stacks: no snapshot
+      y.sp = st.sp;
+      y.mods = st.mods;
+      y.i = st.i;
+      y.nops = st.nops;
+      y.top = top;
+      y.mem = st.sp > 2 && st.sp <= 8 ? below(stk) : 0;
+      y.power <<= 1;
+      y.lam = 0;
+    }
+  }
   __host__ __device__ __forceinline__ const ForthState &state() const { return ln.st; }
   __host__ __device__ __forceinline__ uint32_t ops() const { return ln.st.i - ln.st.nops; }
   __host__ __device__ __forceinline__ uint32_t raw() const { return ln.st.i; }

@@ -32,6 +32,10 @@ struct Stages {
   using Warp = BffWarp<W, kLogic, kNullMask>;
   using Mem = BffMem;
   static constexpr bool kStack = false;
+  // Of 8 pairs of a warp, how many have to go on past their first stage for its
+  // lanes to take them on side by side (0: never, where the warp runs loops by
+  // many iterations at a time).
+  static constexpr uint32_t kCrowd = kLogic == kLogicJump8 ? 8 : 0;
 };
 template <int L>
 struct Stages<L, false> {
@@ -40,6 +44,7 @@ struct Stages<L, false> {
   using Warp = ForthWarp<W, (L == kForthtrivialReset)>;
   using Mem = ForthMem;
   static constexpr bool kStack = true;
+  static constexpr uint32_t kCrowd = 6;
 };
 
 // A resumable SUBLEQ interpreter of language L behind one interface: begin()

@@ -437,25 +437,42 @@ struct LaneServer {
 // pair each (BFF: up to the first jump; Forth: a few steps): most random
 // programs end there, and those pairs are written back and their consumers
 // notified at once.  The pairs that go on are kept (kLong) and run one after the
-// other on the whole warp, one per iteration, so that slots held by other lanes are still polled in between.  So that
-// pairs wait behind few others, a warp holds 8 and there are many warps: a soup
-// of 2^17 bff programs taken over by self-replicators takes 35.4 ms for 16
+// other on the whole warp, one per iteration, so that slots held by other lanes are
+// still polled in between.
+//
+// Where the warp would run such a pair command by command (Forth, and the BFF
+// languages without matched brackets), and most pairs of a claim go on, as in a
+// soup of self-replicators, the lanes take them on side by side instead: their
+// programs are much alike, and a command of 8 costs what a command of one does.
+// Once that was so, the next claim's are run so from the start, however few of
+// them are there yet.  (64 epochs of forthtrivial evolved for 4096: 2^14 programs
+// 82 ms, one after the other 594; bff8 2^17: 178, 340.  With 5 of 8 instead of 6
+// Forth soups with some long pairs lose 5 to 15 %, as each waits for the slowest;
+// with 7 instead of all of 8 bff8 soups up to 30 %.)
+//
+// So that pairs wait behind few others, a warp holds 8 and there are many warps: a
+// soup of 2^17 bff programs taken over by self-replicators takes 35.4 ms for 16
 // epochs with 8 (32 lanes: 76.9, 16: 44.6), one of 1022 bff_noheads programs
 // 2.1 ms for 64 (4.3, 3.0); only the 20 first epochs of a random soup of 2^17
 // are a little faster with 32 (3.07 ms, 8: 3.27).
-template <int L>
+template <int L, uint32_t kLanes>
 struct StagedServer {
   using LaneM = typename Stages<L>::Lane;
-  static constexpr uint32_t kWidth = StagedMem<L>::kWidth;
-  static constexpr size_t kWarpBytes = sizeof(StagedMem<L>);
+  using Mem = StagedMem<L, kLanes>;
+  static constexpr uint32_t kWidth = kLanes;
+  static constexpr size_t kWarpBytes = sizeof(Mem);
   LaneM m;
-  StagedMem<L> &mem;
+  Mem &mem;
   LaneWords<kWidth> t, stk;
   const uint8_t *optab, *cmdflag;
+  static constexpr int kCrowd = static_cast<int>(Stages<L>::kCrowd * kLanes / 8);
+  static constexpr int kCrowdSteps = 256;  // of a lane in an iteration
+  bool crowd;   // the lanes take pairs on themselves
+  int went_on;  // pairs of this claim that went on
 
   __device__ __forceinline__ StagedServer(uint8_t *smem, const uint8_t *tables, uint32_t tid)
-      : mem(reinterpret_cast<StagedMem<L> *>(smem)[tid >> 5]), t(mem.tape(tid & 31)),
-        stk(mem.stack(tid & 31)), optab(tables), cmdflag(tables + 256) {
+      : mem(reinterpret_cast<Mem *>(smem)[tid >> 5]), t(mem.tape(tid & 31)),
+        stk(mem.stack(tid & 31)), optab(tables), cmdflag(tables + 256), crowd(false), went_on(0) {
     m.status = LaneM::kEnds;
   }
 
@@ -521,14 +538,32 @@ struct StagedServer {
 
   __device__ __forceinline__ bool iterate(const PipeCtx &b, const PipeQueue &q, Lane &ln,
                                           uint32_t lane, uint32_t slot_ctr) {
-    // 1. The next long pair, or a bulk claim of queue slots by idle lanes.
+    // 1. The long pairs, or the next of them, or a bulk claim of queue slots by idle
+    // lanes.
     const uint32_t lng = __ballot_sync(0xffffffffu, ln.state == kLong);
-    if (lng) {
+    bool together = false;
+    if constexpr (kCrowd != 0) {
+      crowd |= __popc(lng) >= kCrowd;
+      together = crowd && lng != 0;
+      if (together && ln.state == kLong) {
+        for (int r = 0; r < kCrowdSteps && m.status != LaneM::kEnds; r++)
+          m.step_on(t, stk, optab, mem.cycles[lane]);
+        m.settle(t, stk, optab);
+        if (m.status == LaneM::kEnds) ln.state = kRun;
+      }
+    }
+    if (!together && lng != 0) {
       run_long(b, ln, static_cast<uint32_t>(__ffs(lng) - 1), lane, slot_ctr);
-    } else {
+    } else if (lng == 0) {
       const uint32_t idle = __ballot_sync(0xffffffffu, ln.state == kIdle);
       const uint32_t busy = __ballot_sync(0xffffffffu, ln.state != kIdle && ln.state != kExhausted);
-      if (idle && busy == 0) claim(b, q, ln, idle, lane);
+      if (idle && busy == 0) {
+        if (kCrowd != 0) {
+          crowd = went_on >= kCrowd;
+          went_on = 0;
+        }
+        claim(b, q, ln, idle, lane);
+      }
     }
     bool progressed = lng != 0;
 
@@ -554,6 +589,7 @@ struct StagedServer {
       if (m.status == LaneM::kJumps) m.resolve(t, optab);
       if (m.status == LaneM::kJumps) {
         ln.state = kLong;
+        if (kCrowd != 0) LaneM::begin_cycle(mem.cycles[lane]);
       } else {
         const PipeSoup &sp = b.soups[ln.si];
         if (ln.dirty || (ln.evaluated && m.mods() != 0))
@@ -562,36 +598,39 @@ struct StagedServer {
         finish(sp, ln);
       }
     }
+    if (kCrowd != 0)
+      went_on += __popc(__ballot_sync(0xffffffffu, ln.state == kLong) & ~lng);
     // 6. Push the consumers whose second input this pair was.
     push_ready(b, q, ln, lane);
     return progressed;
   }
 };
 
-template <int L>
-using Server = std::conditional_t<(L <= kForthtrivialReset), StagedServer<L>, LaneServer<L>>;
+template <int L, uint32_t kLanes>
+using Server =
+    std::conditional_t<(L <= kForthtrivialReset), StagedServer<L, kLanes>, LaneServer<L>>;
 
 // Shared memory of a pipelined launch: the servers' (tapes and so on), the op
 // and command tables, then the soup descriptors.
-template <int L>
+template <int L, uint32_t kLanes>
 __host__ __device__ constexpr size_t server_bytes() {
-  return (kThreads / 32) * Server<L>::kWarpBytes;
+  return (kThreads / 32) * Server<L, kLanes>::kWarpBytes;
 }
 
-template <int L>
+template <int L, uint32_t kLanes>
 size_t pipeline_smem_bytes(int n_soups) {
-  return server_bytes<L>() + 512 + size_t(n_soups) * sizeof(PipeSoup);
+  return server_bytes<L, kLanes>() + 512 + size_t(n_soups) * sizeof(PipeSoup);
 }
 
 // The persistent kernel of a pipelined launch over soups of language L.
 // Blocks per SM set the register budget: the BFF machines take 96 without
 // spills that matter (6 blocks, 80 registers: 39.9 ms instead of 35.1 on the
 // self-replicators above), the lanes' shared memory allows the others 4.
-template <int L>
+template <int L, uint32_t kLanes>
 __global__ void __launch_bounds__(kThreads, (L <= kForthtrivialReset) ? 5 : 4)
     pipeline_kernel(const __grid_constant__ PipeBatch pb) {
   extern __shared__ __align__(16) uint8_t smem[];
-  uint8_t *tables = smem + server_bytes<L>();
+  uint8_t *tables = smem + server_bytes<L, kLanes>();
   PipeSoup *soups = reinterpret_cast<PipeSoup *>(tables + 512);
   const uint32_t tid = threadIdx.x, lane = tid & 31;
   if (LangTraits<L>::kStaged) fill_tables<L>(tables);
@@ -605,10 +644,10 @@ __global__ void __launch_bounds__(kThreads, (L <= kForthtrivialReset) ? 5 : 4)
   const uint32_t warp = blockIdx.x * (kThreads / 32) + (tid >> 5);
   const PipeCtx b{soups, pb.error, pb.wait_limit_ns, pb.tune};
   const PipeQueue q = pb.queue;
-  Server<L> server(smem, tables, tid);
+  Server<L, kLanes> server(smem, tables, tid);
   Lane ln;
   ln.begin();
-  if (lane >= Server<L>::kWidth) ln.state = kExhausted;
+  if (lane >= server.kWidth) ln.state = kExhausted;
   // A warp serves the queue until every lane has claimed past its last task.
   while (true) {
     const bool progressed = server.iterate(b, q, ln, lane, warp % kCountSlots);
@@ -624,23 +663,23 @@ __global__ void __launch_bounds__(kThreads, (L <= kForthtrivialReset) ? 5 : 4)
 // per SM: 3.61, 3.49).
 constexpr uint64_t kMinLanes = 4096;
 
-template <int L>
-int launch_pipeline_t(const PipeBatch &b, uint64_t total_pairs, uint32_t lanes_per_pair64,
+template <int L, uint32_t kLanes>
+int launch_pipeline_w(const PipeBatch &b, uint64_t total_pairs, uint32_t lanes_per_pair64,
                       int device, cudaStream_t stream) {
   static std::atomic<int> sms_cache[64];  // (zero-initialised: static storage)
-  const size_t smem_max = pipeline_smem_bytes<L>(kMaxPipeSoups);
+  const size_t smem_max = pipeline_smem_bytes<L, kLanes>(kMaxPipeSoups);
   if (sms_cache[device & 63].load() == 0) {
-    CUBFF_CUDA_TRY(cudaFuncSetAttribute(pipeline_kernel<L>,
+    CUBFF_CUDA_TRY(cudaFuncSetAttribute(pipeline_kernel<L, kLanes>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(smem_max)));
     int sms = 0;
     CUBFF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     sms_cache[device & 63].store(sms);
   }
-  const size_t smem = pipeline_smem_bytes<L>(b.n_soups);
+  const size_t smem = pipeline_smem_bytes<L, kLanes>(b.n_soups);
   int per_sm = 0;
-  CUBFF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pipeline_kernel<L>,
-                                                               kThreads, smem));
+  CUBFF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &per_sm, pipeline_kernel<L, kLanes>, kThreads, smem));
   const uint64_t resident = uint64_t(std::max(1, per_sm)) * sms_cache[device & 63].load();
   // Lanes in flight: enough to keep the SMs busy, few enough that most held
   // pairs are ready (a lane holding a pair of a later epoch only polls).
@@ -648,12 +687,18 @@ int launch_pipeline_t(const PipeBatch &b, uint64_t total_pairs, uint32_t lanes_p
   // pairs in flight, or kMinLanes of them.
   uint64_t want = (total_pairs * uint64_t(lanes_per_pair64 ? lanes_per_pair64 : 32)) / 64;
   want = std::max<uint64_t>(want, std::min<uint64_t>(total_pairs, kMinLanes));
-  const uint64_t per_block = kThreads / 32 * Server<L>::kWidth;
+  const uint64_t per_block = kThreads / 32 * Server<L, kLanes>::kWidth;
   const uint64_t blocks = (want + per_block - 1) / per_block;
   const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(blocks, resident));
-  pipeline_kernel<L><<<grid, kThreads, smem, stream>>>(b);
+  pipeline_kernel<L, kLanes><<<grid, kThreads, smem, stream>>>(b);
   CUBFF_CUDA_TRY(cudaGetLastError());
   return CUBFF_OK;
+}
+
+template <int L>
+int launch_pipeline_t(const PipeBatch &b, uint64_t total_pairs, uint32_t lanes_per_pair64,
+                      int device, cudaStream_t stream) {
+  return launch_pipeline_w<L, 8>(b, total_pairs, lanes_per_pair64, device, stream);
 }
 
 }  // namespace

@@ -9,11 +9,12 @@ namespace cubff {
 
 // A warp's shared memory: the tapes (and stacks) of kWidth lanes, interleaved,
 // and the warp machine's.
-template <int L>
+template <int L, uint32_t kLanes = 8>
 struct StagedMem {
-  static constexpr uint32_t kWidth = 8;  // lanes that hold pairs
+  static constexpr uint32_t kWidth = kLanes;  // lanes that hold pairs
   uint32_t tapes[kWidth * kPair / 4];
   uint32_t stacks[Stages<L>::kStack ? kWidth * kPair / 4 : 4];
+  typename Stages<L>::Lane::Cycle cycles[Stages<L>::kCrowd ? kWidth : 1];
   typename Stages<L>::Mem warp;
 
   __device__ __forceinline__ LaneWords<kWidth> tape(uint32_t lane) {
@@ -55,11 +56,10 @@ struct Counts {
 
 // Runs the pair of lane `src` (machine m there) to its end on the whole warp;
 // its tape is then in mem.warp.T.
-template <int L>
-__device__ __forceinline__ Counts run_on_warp(StagedMem<L> &mem,
+template <int L, uint32_t kWidth>
+__device__ __forceinline__ Counts run_on_warp(StagedMem<L, kWidth> &mem,
                                               const typename Stages<L>::Lane &m, uint32_t src,
                                               uint32_t lane, const uint8_t *optab) {
-  constexpr uint32_t kWidth = StagedMem<L>::kWidth;
   const auto st = broadcast(m.state(), src);
   __syncwarp();  // the lane's tape
   reinterpret_cast<uint32_t *>(mem.warp.T)[lane] = mem.tapes[lane * kWidth + src];

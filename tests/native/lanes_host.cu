@@ -144,7 +144,8 @@ template <int L> thread_local Counts3 Long<L>::counts[kWarp];
 // 0: as one program; 1: neighbours' bytes changed; 2: the lanes did not meet;
 // 3: the lanes' counts differ.
 template <int L, uint32_t stride>
-int run_staged(uint8_t *tape, uint32_t lane, uint32_t order, const uint8_t *optab, Counts3 *out) {
+int run_staged(uint8_t *tape, uint32_t lane, uint32_t order, uint32_t steps_on,
+               const uint8_t *optab, Counts3 *out) {
   uint32_t tapes[stride * kPair / 4], stacks[stride * kPair / 4];
   fill<stride>(tapes);
   fill<stride>(stacks);
@@ -159,9 +160,18 @@ int run_staged(uint8_t *tape, uint32_t lane, uint32_t order, const uint8_t *opta
   Lane &m = Long<L>::first;
   m.begin(t, cmd, optab);
   while (m.status == Lane::kRuns) m.step(t, stk, optab);
-  if (m.status == Lane::kJumps) m.resolve(t, optab);
+  if (m.status == Lane::kJumps) {
+    m.resolve(t, optab);
+    if constexpr (Stages<L>::kCrowd != 0) {
+      typename Lane::Cycle cycle;
+      Lane::begin_cycle(cycle);
+      for (uint32_t r = 0; r < steps_on && m.status != Lane::kEnds; r++)
+        m.step_on(t, stk, optab, cycle);
+      m.settle(t, stk, optab);
+    }
+  }
   if (!kept<stride>(tapes, lane) || !kept<stride>(stacks, lane)) return 1;
-  if (m.status != Lane::kJumps) {
+  if (m.status == Lane::kEnds) {
     for (int p = 0; p < kPair; p++) tape[p] = static_cast<uint8_t>(t.get(p));
     *out = {m.ops(), m.raw(), m.mods()};
     return 0;
@@ -200,7 +210,8 @@ int run_subleq(uint8_t *tape, uint32_t lane, Counts3 *out) {
 }
 
 template <int L>
-int run_lang(uint32_t stride, uint8_t *tape, uint32_t lane, uint32_t order, Counts3 *out) {
+int run_lang(uint32_t stride, uint8_t *tape, uint32_t lane, uint32_t order, uint32_t steps_on,
+             Counts3 *out) {
   uint8_t optab[256];
   for (int c = 0; c < 256; c++) optab[c] = op_of(L, c);
   lane %= stride;
@@ -208,9 +219,9 @@ int run_lang(uint32_t stride, uint8_t *tape, uint32_t lane, uint32_t order, Coun
     return stride == 16 ? run_subleq<(L == kRsubleq4), 16>(tape, lane, out)
                         : run_subleq<(L == kRsubleq4), 32>(tape, lane, out);
   } else {
-    return stride == 8    ? run_staged<L, 8>(tape, lane, order, optab, out)
-           : stride == 16 ? run_staged<L, 16>(tape, lane, order, optab, out)
-                          : run_staged<L, 32>(tape, lane, order, optab, out);
+    return stride == 8    ? run_staged<L, 8>(tape, lane, order, steps_on, optab, out)
+           : stride == 16 ? run_staged<L, 16>(tape, lane, order, steps_on, optab, out)
+                          : run_staged<L, 32>(tape, lane, order, steps_on, optab, out);
   }
 }
 
@@ -220,26 +231,28 @@ int run_lang(uint32_t stride, uint8_t *tape, uint32_t lane, uint32_t order, Coun
 // every lane alike.
 extern "C" uint32_t lanes_rounds() { return g.rounds; }
 
+
 // Evaluates a tape in place, on lane `lane` of words interleaved by `stride`
-// (8, 16 or 32), the long part with the lanes taking turns in `order`.
+// (8, 16 or 32); of a program that goes on, steps_on more steps on the lane, then
+// the rest with the lanes taking turns in `order`.
 extern "C" int lanes_evaluate(int lang, uint8_t *tape, uint32_t stride, uint32_t lane,
-                              uint32_t order, uint32_t *ops, uint32_t *raw, uint32_t *changed) {
+                              uint32_t order, uint32_t steps_on, uint32_t *ops, uint32_t *raw, uint32_t *changed) {
   Counts3 c{};
   int st = -1;
   switch (lang) {
-    case kBff: st = run_lang<kBff>(stride, tape, lane, order, &c); break;
-    case kBffNoheads: st = run_lang<kBffNoheads>(stride, tape, lane, order, &c); break;
-    case kBffNoheads4bit: st = run_lang<kBffNoheads4bit>(stride, tape, lane, order, &c); break;
-    case kBffPerm: st = run_lang<kBffPerm>(stride, tape, lane, order, &c); break;
-    case kBff8: st = run_lang<kBff8>(stride, tape, lane, order, &c); break;
-    case kBff8Noheads: st = run_lang<kBff8Noheads>(stride, tape, lane, order, &c); break;
-    case kBffSelfmove: st = run_lang<kBffSelfmove>(stride, tape, lane, order, &c); break;
-    case kForth: st = run_lang<kForth>(stride, tape, lane, order, &c); break;
-    case kForthcopy: st = run_lang<kForthcopy>(stride, tape, lane, order, &c); break;
-    case kForthtrivial: st = run_lang<kForthtrivial>(stride, tape, lane, order, &c); break;
-    case kForthtrivialReset: st = run_lang<kForthtrivialReset>(stride, tape, lane, order, &c); break;
-    case kSubleq: st = run_lang<kSubleq>(stride, tape, lane, order, &c); break;
-    case kRsubleq4: st = run_lang<kRsubleq4>(stride, tape, lane, order, &c); break;
+    case kBff: st = run_lang<kBff>(stride, tape, lane, order, steps_on, &c); break;
+    case kBffNoheads: st = run_lang<kBffNoheads>(stride, tape, lane, order, steps_on, &c); break;
+    case kBffNoheads4bit: st = run_lang<kBffNoheads4bit>(stride, tape, lane, order, steps_on, &c); break;
+    case kBffPerm: st = run_lang<kBffPerm>(stride, tape, lane, order, steps_on, &c); break;
+    case kBff8: st = run_lang<kBff8>(stride, tape, lane, order, steps_on, &c); break;
+    case kBff8Noheads: st = run_lang<kBff8Noheads>(stride, tape, lane, order, steps_on, &c); break;
+    case kBffSelfmove: st = run_lang<kBffSelfmove>(stride, tape, lane, order, steps_on, &c); break;
+    case kForth: st = run_lang<kForth>(stride, tape, lane, order, steps_on, &c); break;
+    case kForthcopy: st = run_lang<kForthcopy>(stride, tape, lane, order, steps_on, &c); break;
+    case kForthtrivial: st = run_lang<kForthtrivial>(stride, tape, lane, order, steps_on, &c); break;
+    case kForthtrivialReset: st = run_lang<kForthtrivialReset>(stride, tape, lane, order, steps_on, &c); break;
+    case kSubleq: st = run_lang<kSubleq>(stride, tape, lane, order, steps_on, &c); break;
+    case kRsubleq4: st = run_lang<kRsubleq4>(stride, tape, lane, order, steps_on, &c); break;
   }
   *ops = c.ops;
   *raw = c.raw;

@@ -37,18 +37,18 @@ def lanes_lib():
     L = ctypes.CDLL(SO)
     u32, vp = ctypes.c_uint32, ctypes.c_void_p
     L.lanes_evaluate.restype = ctypes.c_int
-    L.lanes_evaluate.argtypes = [ctypes.c_int, vp, u32, u32, u32, vp, vp, vp]
+    L.lanes_evaluate.argtypes = [ctypes.c_int, vp, u32, u32, u32, u32, vp, vp, vp]
     return L
 
 
-def check(L, lang, tape, stride, lane, order):
+def check(L, lang, tape, stride, lane, order, steps_on=0):
     want = tape.copy()
     ops, raw = O.evaluate(lang, want)
     got = tape.copy()
     c = np.zeros(3, dtype=np.uint32)
-    st = L.lanes_evaluate(LANGUAGES.index(lang), got.ctypes.data, stride, lane, order,
+    st = L.lanes_evaluate(LANGUAGES.index(lang), got.ctypes.data, stride, lane, order, steps_on,
                           c[0:].ctypes.data, c[1:].ctypes.data, c[2:].ctypes.data)
-    case = (lang, order, bytes(tape).hex())
+    case = (lang, order, steps_on, bytes(tape).hex())
     assert st == 0, (st, case)
     assert (int(c[0]), int(c[1])) == (ops, raw), case
     assert np.array_equal(got, want), case
@@ -114,6 +114,16 @@ def test_subleq_on_words_matches_oracle(lanes_lib, lang, stride):
         tape = np.zeros(128, dtype=np.uint8)
         tape[:len(prog)] = np.frombuffer(prog, dtype=np.uint8)
         check(lanes_lib, lang, tape, stride, 5, 0)
+
+
+CROWDS = [lang for lang in STAGED if lang.startswith(("forth", "bff8"))]
+
+
+@pytest.mark.parametrize("lang", CROWDS)
+def test_programs_taken_on_by_a_lane(lanes_lib, lang):
+    """All of a program on its lane, or so many steps before the warp takes it."""
+    for i, tape in enumerate(tapes_of(lang, 1500, 47)):
+        check(lanes_lib, lang, tape, 8, i, ORDERS[i % 3], (1 << 14, 7, 256, 1, 40)[i // 4 % 5])
 
 
 def test_copy_backwards_of_equal_bytes_runs_in_batches(lanes_lib):
