@@ -109,6 +109,14 @@ constexpr int kPipeCountSlots = 32;
 // in flight per 64 of them (0 = default).
 int launch_pipeline(const PipeBatch &b, uint64_t total_pairs, uint32_t lanes_per_pair64,
                     int device, cudaStream_t stream);
+// Its kernel and grid (launch_plan.h).
+struct PipePlan;
+int plan_pipeline(int lang, int n_soups, uint64_t total_pairs, uint32_t lanes_per_pair64,
+                  int device, PipePlan *out);
+// The kernels of the staged families (pipeline_bff.cu, pipeline_forth.cu).
+struct PipeKernels;
+PipeKernels bff_pipe_kernels(int lang);
+PipeKernels forth_pipe_kernels(int lang);
 int launch_mutation_masks(uint64_t s0, uint64_t e0, uint32_t n_epochs, uint64_t n, uint32_t prob,
                           uint4 *out, cudaStream_t stream);
 int launch_inverse(const uint32_t *perm, uint32_t n_epochs, uint64_t n, uint32_t *inv,

@@ -32,10 +32,11 @@ struct Stages {
   using Warp = BffWarp<W, kLogic, kNullMask>;
   using Mem = BffMem;
   static constexpr bool kStack = false;
-  // Of 8 pairs of a warp, how many have to go on past their first stage for its
-  // lanes to take them on side by side (0: never, where the warp runs loops by
-  // many iterations at a time).
-  static constexpr uint32_t kCrowd = kLogic == kLogicJump8 ? 8 : 0;
+  // Whether the lanes of a warp may take on their long pairs side by side (not where
+  // the warp runs loops by many iterations at a time), and how many of its pairs
+  // have to go on past their first stage for that.
+  static constexpr bool kCrowds = kLogic == kLogicJump8;
+  static constexpr int crowd(int pairs) { return pairs == 8 ? 8 : pairs * 7 / 8; }
 };
 template <int L>
 struct Stages<L, false> {
@@ -44,7 +45,8 @@ struct Stages<L, false> {
   using Warp = ForthWarp<W, (L == kForthtrivialReset)>;
   using Mem = ForthMem;
   static constexpr bool kStack = true;
-  static constexpr uint32_t kCrowd = 6;
+  static constexpr bool kCrowds = true;
+  static constexpr int crowd(int pairs) { return pairs * 6 / 8; }
 };
 
 // A resumable SUBLEQ interpreter of language L behind one interface: begin()

@@ -14,7 +14,7 @@ struct StagedMem {
   static constexpr uint32_t kWidth = kLanes;  // lanes that hold pairs
   uint32_t tapes[kWidth * kPair / 4];
   uint32_t stacks[Stages<L>::kStack ? kWidth * kPair / 4 : 4];
-  typename Stages<L>::Lane::Cycle cycles[Stages<L>::kCrowd ? kWidth : 1];
+  typename Stages<L>::Lane::Cycle cycles[Stages<L>::kCrowds ? kWidth : 1];
   typename Stages<L>::Mem warp;
 
   __device__ __forceinline__ LaneWords<kWidth> tape(uint32_t lane) {

@@ -162,7 +162,7 @@ int run_staged(uint8_t *tape, uint32_t lane, uint32_t order, uint32_t steps_on,
   while (m.status == Lane::kRuns) m.step(t, stk, optab);
   if (m.status == Lane::kJumps) {
     m.resolve(t, optab);
-    if constexpr (Stages<L>::kCrowd != 0) {
+    if constexpr (Stages<L>::kCrowds) {
       typename Lane::Cycle cycle;
       Lane::begin_cycle(cycle);
       for (uint32_t r = 0; r < steps_on && m.status != Lane::kEnds; r++)
