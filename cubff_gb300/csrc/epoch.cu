@@ -96,15 +96,79 @@ __global__ void __launch_bounds__(kThreads) selfrep_kernel(const uint8_t *soup,
 // programs with self-replicators about; now 35.)
 constexpr int kScored = 4;
 
+// The chains of a program on the lanes of a warp.
+template <int L>
+struct ChainMem {
+  static constexpr uint32_t kLanes = 16;
+  uint32_t tapes[kLanes * kPair / 4];
+  uint32_t stacks[Stages<L>::kStack ? kLanes * kPair / 4 : 4];
+  typename Stages<L>::Lane::Cycle cycles[kLanes];
+};
+
 template <int L>
 struct ScoreMem {
   typename Stages<L>::Mem warps[kThreads / 32];
   uint8_t fin[kScored][kIters][kPair];
   uint8_t prog[kScored][kTape];
+  ChainMem<L> chains[Stages<L>::kCrowds ? kScored : 1];
   uint32_t votes[kScored][2];
-  uint32_t claimed;
+  uint32_t claimed, left;
+  uint8_t list[kScored * kIters];  // chains left for whole warps
   uint8_t tables[512];
 };
+
+// The 13 chains of program p, a lane each, if in the first generation so many of
+// them go on past their first stage (Stages) that it is worth it; false if not.
+// (2^13 forthtrivial programs evolved for 2112 epochs: 9.6 ms, chain by chain on
+// whole warps 107, one program a lane 44; random ones, which gain nothing by it:
+// 5.8, 4.0 and 24.)
+template <int L>
+__device__ __noinline__ bool chains_on_lanes(ScoreMem<L> &sm, uint32_t p, uint64_t local_seed,
+                                             uint32_t lane) {
+  using LaneM = typename Stages<L>::Lane;
+  constexpr uint32_t kLanes = ChainMem<L>::kLanes;
+  constexpr int kCrowd = Stages<L>::crowd(kIters);
+  ChainMem<L> &mem = sm.chains[p];
+  const bool mine = lane < kIters;
+  const uint32_t it = mine ? lane : 0;
+  const uint8_t *optab = sm.tables, *cmdflag = sm.tables + 256;
+  const LaneWords<kLanes> t{reinterpret_cast<uint8_t *>(mem.tapes), it};
+  const LaneWords<kLanes> stk{reinterpret_cast<uint8_t *>(mem.stacks), it};
+  // (The partner's bytes wait where the final tape's second half will be.)
+  uint32_t *fin = reinterpret_cast<uint32_t *>(sm.fin[p][it]);
+  const uint32_t *prog = reinterpret_cast<const uint32_t *>(sm.prog[p]);
+  if (mine)
+    for (uint32_t j = 0; j < kTape; j++)
+      sm.fin[p][it][kTape + j] = static_cast<uint8_t>(noise(local_seed, it, j));
+  LaneM m;
+  m.status = LaneM::kEnds;
+  for (int g = 0; g <= kGens; g++) {
+    if (mine) {
+      for (uint32_t q = 0; q < kTape / 4; q++) {
+        t.word(q) = g == 0 ? prog[q] : t.word(kTape / 4 + q);
+        t.word(kTape / 4 + q) = fin[kTape / 4 + q];
+      }
+      Mask128 cmd{0, 0};
+      if (L <= kBffSelfmove)
+        for (int b = 0; b < kPair; b++) mask_assign(cmd, b, cmdflag[t.get(b)] != 0);
+      m.begin(t, cmd, optab);
+    }
+    while (__any_sync(0xffffffffu, m.status == LaneM::kRuns))
+      if (m.status == LaneM::kRuns) m.step(t, stk, optab);
+    if (m.status == LaneM::kJumps) m.resolve(t, optab);
+    const bool goes_on = m.status == LaneM::kJumps;
+    const int going = __popc(__ballot_sync(0xffffffffu, goes_on));
+    if (g == 0 && going < kCrowd) return false;
+    if (goes_on) {
+      LaneM::begin_cycle(mem.cycles[it]);
+      while (m.status != LaneM::kEnds) m.step_on(t, stk, optab, mem.cycles[it]);
+    }
+    __syncwarp();
+  }
+  if (mine)
+    for (uint32_t q = 0; q < kPair / 4; q++) fin[q] = t.word(q);
+  return true;
+}
 
 template <int L>
 __global__ void __launch_bounds__(kThreads, 5) staged_selfrep_kernel(const uint8_t *soup,
@@ -120,14 +184,24 @@ __global__ void __launch_bounds__(kThreads, 5) staged_selfrep_kernel(const uint8
   for (uint32_t b = tid; b < programs * kTape; b += kThreads)
     sm.prog[0][b] = soup[first * kTape + b];
   if (tid < 2 * kScored) sm.votes[0][tid] = 0;
-  if (tid == 0) sm.claimed = 0;
+  if (tid == 0) sm.claimed = sm.left = 0;
   __syncthreads();
+  if constexpr (Stages<L>::kCrowds) {
+    static_assert(kScored == kThreads / 32);
+    const uint32_t p = tid >> 5;
+    if (p < programs && !chains_on_lanes(sm, p, splitmix64(n * epoch_key + first + p), lane) &&
+        lane < kIters)
+      sm.list[atomicAdd(&sm.left, 1u)] = static_cast<uint8_t>(p * kIters + lane);
+    __syncthreads();
+  }
+  const uint32_t chains = Stages<L>::kCrowds ? sm.left : programs * kIters;
   typename Stages<L>::Mem &mem = sm.warps[tid >> 5];
   while (true) {
     uint32_t chain = 0;
     if (lane == 0) chain = atomicAdd(&sm.claimed, 1u);
     chain = __shfl_sync(0xffffffffu, chain, 0);
-    if (chain >= programs * kIters) break;
+    if (chain >= chains) break;
+    if (Stages<L>::kCrowds) chain = sm.list[chain];
     const uint32_t p = chain / kIters, it = chain % kIters;
     const uint64_t local_seed = splitmix64(n * epoch_key + first + p);
     const uint32_t n0 = noise(local_seed, it, lane), n1 = noise(local_seed, it, 32 + lane);
@@ -209,7 +283,7 @@ __global__ void __launch_bounds__(32)
       if (m.status == LaneM::kJumps) m.resolve(t, optab);
     }
     if (__any_sync(0xffffffffu, m.status == LaneM::kJumps)) {
-      const Counts c = run_on_warp(mem, m, 0, lane, optab);
+      const Counts c = run_on_warp<L>(mem.warp, mem, 0, broadcast(m.state(), 0), lane, optab);
       res.words[lane] = reinterpret_cast<const uint32_t *>(mem.warp.T)[lane];
       if (lane == 0) {
         res.ops = c.ops;
@@ -251,21 +325,47 @@ int launch_eval_t(const EvalTape &tape, int slot, EvalResult *out, cudaStream_t 
   return CUBFF_OK;
 }
 
+template <int L, uint32_t kWidth>
+int launch_staged_epoch(const EpochArgs &a, uint64_t npairs, int device, cudaStream_t stream) {
+  constexpr size_t smem = epoch_smem_bytes<L, kWidth>();
+  if constexpr (smem > 48 << 10) {
+    static std::atomic<uint64_t> raised;  // by device (zero-initialised)
+    const uint64_t bit = 1ull << (device & 63);
+    if (!(raised.load() & bit)) {
+      CUBFF_CUDA_TRY(cudaFuncSetAttribute(staged_epoch_kernel<L, kWidth>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(smem)));
+      raised.fetch_or(bit);
+    }
+  }
+  constexpr uint64_t per_block = kThreads / 32 * kWidth;
+  staged_epoch_kernel<L, kWidth>
+      <<<static_cast<unsigned>((npairs + per_block - 1) / per_block), kThreads, smem, stream>>>(a);
+  CUBFF_CUDA_TRY(cudaGetLastError());
+  return CUBFF_OK;
+}
+
 template <int L>
 int launch_epoch_t(const EpochArgs &a, cudaStream_t stream) {
   const uint64_t npairs = a.n / 2;
   if (npairs == 0) return CUBFF_OK;
-  const size_t smem = epoch_smem_bytes<L>();
   if constexpr (LangTraits<L>::kStaged) {
-    const uint64_t per_block = kThreads / 32 * StagedMem<L>::kWidth;
-    staged_epoch_kernel<L><<<static_cast<unsigned>((npairs + per_block - 1) / per_block), kThreads,
-                             smem, stream>>>(a);
+    if constexpr (Stages<L>::kCrowds) {
+      int device = 0, sms = 0;
+      CUBFF_CUDA_TRY(cudaGetDevice(&device));
+      CUBFF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+      // From 3 warps of 32 pairs per SM on, as in a pipelined launch.
+      if (npairs >= uint64_t(sms) * 3 * 32) return launch_staged_epoch<L, 32>(a, npairs, device, stream);
+      return launch_staged_epoch<L, 8>(a, npairs, device, stream);
+    } else {
+      return launch_staged_epoch<L, 8>(a, npairs, 0, stream);
+    }
   } else {
-    epoch_kernel<L><<<static_cast<unsigned>((npairs + kThreads - 1) / kThreads), kThreads, smem,
-                      stream>>>(a);
+    epoch_kernel<L><<<static_cast<unsigned>((npairs + kThreads - 1) / kThreads), kThreads,
+                      epoch_smem_bytes<L>(), stream>>>(a);
+    CUBFF_CUDA_TRY(cudaGetLastError());
+    return CUBFF_OK;
   }
-  CUBFF_CUDA_TRY(cudaGetLastError());
-  return CUBFF_OK;
 }
 
 template <int L>

@@ -16,9 +16,18 @@ constexpr int kGroups = kThreads / 128;
 struct SubleqMem {  // of a warp
   uint32_t tapes[kPair / 4 * 32], snaps[kPair / 4 * 32];
 };
-template <int L>
+// The pairs of a block that go on past their first stage.
+template <int L, uint32_t kWidth>
+struct LongPairs {
+  static constexpr uint32_t kPairs = kThreads / 32 * kWidth;
+  typename Stages<L>::State state[kPairs];  // by warp and lane
+  uint32_t list[kPairs];
+  uint32_t count, claimed;
+};
+template <int L, uint32_t kWidth = 8>
 constexpr size_t epoch_smem_bytes() {
-  if constexpr (LangTraits<L>::kStaged) return kThreads / 32 * sizeof(StagedMem<L>) + 512;
+  if constexpr (LangTraits<L>::kStaged)
+    return kThreads / 32 * sizeof(StagedMem<L, kWidth>) + 512 + sizeof(LongPairs<L, kWidth>);
   else return kThreads / 32 * sizeof(SubleqMem);
 }
 
@@ -109,43 +118,52 @@ __global__ void __launch_bounds__(kThreads) epoch_kernel(EpochArgs a) {
 }
 
 // The staged languages.  A warp takes kWidth consecutive pairs: all lanes load
-// and mutate them together (32 of their draws per lane),
-// its first lanes run the first part of one each, and the pairs that go on run
-// on the whole warp one after the other.  The launch lasts as long as its
-// longest pairs, so a warp holds few.
-template <int L>
-__global__ void __launch_bounds__(kThreads, 5) staged_epoch_kernel(EpochArgs a) {
+// and mutate them together, 8 pairs at a time (32 of their draws per lane), its
+// first lanes run the first part of one each, and, where most of them go on and
+// lanes may (Stages), all of it.  The other pairs that go on run on whole warps:
+// those of a block wherever one is free, as the launch lasts as long as its slowest
+// warp.  (One epoch of 2^17 programs evolved for 4096: forthtrivial 1.2 ms, bff8
+// 1.6, bff 1.65; with 8 pairs to a warp, all run by that warp one after the other,
+// 21, 7.0 and 1.9; one pair a lane 0.75, 1.1 and 1.25.)
+template <int L, uint32_t kWidth>
+__global__ void __launch_bounds__(kThreads, kWidth == 8 ? 5 : 4) staged_epoch_kernel(EpochArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   using LaneM = typename Stages<L>::Lane;
-  constexpr uint32_t kWidth = StagedMem<L>::kWidth;
-  uint8_t *tables = smem + kThreads / 32 * sizeof(StagedMem<L>);
+  uint8_t *tables = smem + kThreads / 32 * sizeof(StagedMem<L, kWidth>);
   const uint8_t *optab = tables, *cmdflag = tables + 256;
+  LongPairs<L, kWidth> &longs = *reinterpret_cast<LongPairs<L, kWidth> *>(tables + 512);
+  if (threadIdx.x == 0) longs.count = longs.claimed = 0;
   fill_tables<L>(tables);
   __syncthreads();
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t npairs = a.n / 2;
   const uint64_t k0 = (uint64_t(blockIdx.x) * (kThreads / 32) + warp) * kWidth;
-  if (k0 >= npairs) return;
-  const uint32_t count = static_cast<uint32_t>(npairs - k0 < kWidth ? npairs - k0 : kWidth);
-  StagedMem<L> &mem = reinterpret_cast<StagedMem<L> *>(smem)[warp];
+  const uint32_t count =
+      k0 >= npairs ? 0 : static_cast<uint32_t>(npairs - k0 < kWidth ? npairs - k0 : kWidth);
+  StagedMem<L, kWidth> *mems = reinterpret_cast<StagedMem<L, kWidth> *>(smem);
+  StagedMem<L, kWidth> &mem = mems[warp];
   const LaneWords<kWidth> t = mem.tape(lane), stk = mem.stack(lane);
   uint32_t *soup = reinterpret_cast<uint32_t *>(a.soup);
 
   // Lane l holds word l of each pair: program `mine` of it, word l % 16.
-  uint32_t mine[kWidth];
+#pragma unroll 1
+  for (uint32_t j0 = 0; j0 < count; j0 += 8) {
+    uint32_t mine[8];
 #pragma unroll
-  for (uint32_t j = 0; j < kWidth; j++)
-    mine[j] = j < count ? a.perm[2 * (k0 + j) + (lane >> 4)] : 0;
+    for (uint32_t j = 0; j < 8; j++)
+      mine[j] = j0 + j < count ? a.perm[2 * (k0 + j0 + j) + (lane >> 4)] : 0;
 #pragma unroll
-  for (uint32_t j = 0; j < kWidth; j++)
-    if (j < count) mem.tapes[lane * kWidth + j] = soup[uint64_t(mine[j]) * 16 + (lane & 15)];
-  __syncwarp();
-  // Mutations: lane l draws for 32 bytes of pair l / 4.
-  static_assert(kWidth * 4 == 32);
-  if (lane / 4 < count) {
-    const uint32_t q = lane % 4 * 32;
-    mutate((a.n * a.epoch_key + k0 + lane / 4) * kPair + q, a.mutation_prob,
-           [&](int i, uint32_t v) { mem.tape(lane / 4).set(q + i, v); });
+    for (uint32_t j = 0; j < 8; j++)
+      if (j0 + j < count)
+        mem.tapes[lane * kWidth + j0 + j] = soup[uint64_t(mine[j]) * 16 + (lane & 15)];
+    __syncwarp();
+    // Mutations: lane l draws for 32 bytes of pair l / 4.
+    const uint32_t j = j0 + lane / 4;
+    if (j < count) {
+      const uint32_t q = lane % 4 * 32;
+      mutate((a.n * a.epoch_key + k0 + j) * kPair + q, a.mutation_prob,
+             [&](int i, uint32_t v) { mem.tape(j).set(q + i, v); });
+    }
   }
   __syncwarp();
   const uint64_t num_indices = a.d_num_indices ? *a.d_num_indices : a.num_indices;
@@ -172,29 +190,46 @@ __global__ void __launch_bounds__(kThreads, 5) staged_epoch_kernel(EpochArgs a) 
   }
   uint32_t ops = 0, raw = 0;
   if (evaluated && m.status == LaneM::kJumps) m.resolve(t, optab);
-  uint32_t longs = __ballot_sync(0xffffffffu, evaluated && m.status == LaneM::kJumps);
-  if (evaluated && m.status == LaneM::kEnds) {
+  // (bff8: 8 lanes are too few to be worth their dearer steps here.)
+  if constexpr (Stages<L>::kCrowds && (kWidth > 8 || L > kBffSelfmove)) {
+    constexpr int kCrowd = Stages<L>::crowd(kWidth);
+    const bool goes_on = evaluated && m.status == LaneM::kJumps;
+    if (__popc(__ballot_sync(0xffffffffu, goes_on)) >= kCrowd && goes_on) {
+      LaneM::begin_cycle(mem.cycles[lane]);
+      while (m.status != LaneM::kEnds) m.step_on(t, stk, optab, mem.cycles[lane]);
+    }
+  }
+  if (evaluated && m.status == LaneM::kJumps) {
+    longs.state[warp * kWidth + lane] = m.state();
+    longs.list[atomicAdd(&longs.count, 1u)] = warp * kWidth + lane;
+  } else if (evaluated) {
     ops = m.ops();
     raw = m.raw();
   }
-  while (longs) {
-    const uint32_t src = static_cast<uint32_t>(__ffs(longs) - 1);
-    longs &= longs - 1;
-    const Counts c = run_on_warp(mem, m, src, lane, optab);
-    mem.tapes[lane * kWidth + src] = reinterpret_cast<const uint32_t *>(mem.warp.T)[lane];
-    if (lane == src) {
-      ops = c.ops;
-      raw = c.raw;
+  __syncthreads();
+  while (true) {
+    uint32_t next = 0;
+    if (lane == 0) next = atomicAdd(&longs.claimed, 1u);
+    next = __shfl_sync(0xffffffffu, next, 0);
+    if (next >= longs.count) break;
+    const uint32_t pair = longs.list[next], src = pair % kWidth;
+    StagedMem<L, kWidth> &of = mems[pair / kWidth];
+    const Counts c = run_on_warp<L>(mem.warp, of, src, longs.state[pair], lane, optab);
+    of.tapes[lane * kWidth + src] = reinterpret_cast<const uint32_t *>(mem.warp.T)[lane];
+    if (lane == 0) {
+      ops += c.ops;
+      raw += c.raw;
     }
   }
-  __syncwarp();
+  __syncthreads();
   // First half, then second half (common_language.h:188-191): of a program
   // paired with itself the second half stays.
-#pragma unroll
-  for (uint32_t j = 0; j < kWidth; j++) {
-    const uint32_t other = __shfl_xor_sync(0xffffffffu, mine[j], 16);
-    if (j < count && (lane >= 16 || mine[j] != other))
-      soup[uint64_t(mine[j]) * 16 + (lane & 15)] = mem.tapes[lane * kWidth + j];
+#pragma unroll 8
+  for (uint32_t j = 0; j < count; j++) {
+    const uint32_t mine = a.perm[2 * (k0 + j) + (lane >> 4)];
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 16);
+    if (lane >= 16 || mine != other)
+      soup[uint64_t(mine) * 16 + (lane & 15)] = mem.tapes[lane * kWidth + j];
   }
   add_counts(a, ops, raw);
 }

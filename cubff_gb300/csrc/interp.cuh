@@ -31,12 +31,13 @@ struct Stages {
   template <class W>
   using Warp = BffWarp<W, kLogic, kNullMask>;
   using Mem = BffMem;
+  using State = BffState;
   static constexpr bool kStack = false;
   // Whether the lanes of a warp may take on their long pairs side by side (not where
   // the warp runs loops by many iterations at a time), and how many of its pairs
   // have to go on past their first stage for that.
   static constexpr bool kCrowds = kLogic == kLogicJump8;
-  static constexpr int crowd(int pairs) { return pairs == 8 ? 8 : pairs * 7 / 8; }
+  __host__ __device__ static constexpr int crowd(int pairs) { return pairs == 8 ? 8 : pairs * 7 / 8; }
 };
 template <int L>
 struct Stages<L, false> {
@@ -44,9 +45,10 @@ struct Stages<L, false> {
   template <class W>
   using Warp = ForthWarp<W, (L == kForthtrivialReset)>;
   using Mem = ForthMem;
+  using State = ForthState;
   static constexpr bool kStack = true;
   static constexpr bool kCrowds = true;
-  static constexpr int crowd(int pairs) { return pairs * 6 / 8; }
+  __host__ __device__ static constexpr int crowd(int pairs) { return pairs * 6 / 8; }
 };
 
 // A resumable SUBLEQ interpreter of language L behind one interface: begin()

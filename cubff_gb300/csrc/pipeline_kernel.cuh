@@ -510,7 +510,7 @@ struct StagedServer {
   __device__ __forceinline__ void run_long(const PipeCtx &b, Lane &ln, uint32_t src,
                                            uint32_t lane, uint32_t slot_ctr) {
     constexpr uint32_t kAll = 0xffffffffu;
-    const Counts c = run_on_warp(mem, m, src, lane, optab);
+    const Counts c = run_on_warp<L>(mem.warp, mem, src, broadcast(m.state(), src), lane, optab);
     const PipeSoup &sp = b.soups[__shfl_sync(kAll, ln.si, src)];
     if (c.mods != 0 || __shfl_sync(kAll, ln.dirty, src)) {
       const uint32_t p1 = __shfl_sync(kAll, ln.p1, src), p2 = __shfl_sync(kAll, ln.p2, src);

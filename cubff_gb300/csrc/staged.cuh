@@ -54,19 +54,19 @@ struct Counts {
   uint32_t ops, raw, mods;
 };
 
-// Runs the pair of lane `src` (machine m there) to its end on the whole warp;
-// its tape is then in mem.warp.T.
+// Runs the pair of lane `src` of a warp's memory `of`, from state st, to its end on
+// the whole warp; its tape is then in work.T.
 template <int L, uint32_t kWidth>
-__device__ __forceinline__ Counts run_on_warp(StagedMem<L, kWidth> &mem,
-                                              const typename Stages<L>::Lane &m, uint32_t src,
-                                              uint32_t lane, const uint8_t *optab) {
-  const auto st = broadcast(m.state(), src);
+__device__ __forceinline__ Counts run_on_warp(typename Stages<L>::Mem &work,
+                                              const StagedMem<L, kWidth> &of, uint32_t src,
+                                              const typename Stages<L>::State &st, uint32_t lane,
+                                              const uint8_t *optab) {
   __syncwarp();  // the lane's tape
-  reinterpret_cast<uint32_t *>(mem.warp.T)[lane] = mem.tapes[lane * kWidth + src];
+  reinterpret_cast<uint32_t *>(work.T)[lane] = of.tapes[lane * kWidth + src];
   if constexpr (Stages<L>::kStack)
-    reinterpret_cast<uint32_t *>(mem.warp.stk)[lane] = mem.stacks[lane * kWidth + src];
+    reinterpret_cast<uint32_t *>(work.stk)[lane] = of.stacks[lane * kWidth + src];
   __syncwarp();
-  typename Stages<L>::template Warp<DeviceWarp> wm(DeviceWarp{lane}, mem.warp, optab);
+  typename Stages<L>::template Warp<DeviceWarp> wm(DeviceWarp{lane}, work, optab);
   wm.run(st);
   __syncwarp();
   return {wm.ops(), wm.raw(), wm.mods()};
