@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(32)
       }
     }
   } else {
-    SubleqMem &mem = *reinterpret_cast<SubleqMem *>(smem);
+    SubleqMem<> &mem = *reinterpret_cast<SubleqMem<> *>(smem);
     mem.tapes[lane * 32] = tape.words[lane];
     __syncwarp();
     if (lane == 0) {
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(32)
 
 template <int L>
 int launch_eval_t(const EvalTape &tape, int slot, EvalResult *out, cudaStream_t stream) {
-  size_t smem = sizeof(SubleqMem);
+  size_t smem = sizeof(SubleqMem<>);
   if constexpr (LangTraits<L>::kStaged) smem = sizeof(StagedMem<L>) + 512;
   eval_kernel<L><<<1, 32, smem, stream>>>(tape, slot, out);
   CUBFF_CUDA_TRY(cudaGetLastError());

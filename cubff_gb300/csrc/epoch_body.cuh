@@ -13,8 +13,9 @@ constexpr int kGroups = kThreads / 128;
 // Shared memory per CTA.  SUBLEQ: two per-lane 128-byte areas per thread (the
 // tape and the cycle check's snapshot); the staged languages: their warps', then
 // the op and command tables.
-struct SubleqMem {  // of a warp
-  uint32_t tapes[kPair / 4 * 32], snaps[kPair / 4 * 32];
+template <uint32_t kWidth = 32>
+struct SubleqMem {  // of a warp, kWidth lanes of which hold pairs
+  uint32_t tapes[kPair / 4 * kWidth], snaps[kPair / 4 * kWidth];
 };
 // The pairs of a block that go on past their first stage.
 template <int L, uint32_t kWidth>
@@ -28,7 +29,7 @@ template <int L, uint32_t kWidth = 8>
 constexpr size_t epoch_smem_bytes() {
   if constexpr (LangTraits<L>::kStaged)
     return kThreads / 32 * sizeof(StagedMem<L, kWidth>) + 512 + sizeof(LongPairs<L, kWidth>);
-  else return kThreads / 32 * sizeof(SubleqMem);
+  else return kThreads / 32 * sizeof(SubleqMem<>);
 }
 
 __device__ __forceinline__ void load_pair(const uint8_t *soup, uint32_t p1, uint32_t p2,
@@ -87,7 +88,7 @@ __global__ void __launch_bounds__(kThreads) epoch_kernel(EpochArgs a) {
   const uint64_t npairs = a.n / 2;
   const uint64_t k = uint64_t(blockIdx.x) * kThreads + tid;
   const bool active = k < npairs;
-  SubleqMem &mem = reinterpret_cast<SubleqMem *>(smem)[tid >> 5];
+  SubleqMem<> &mem = reinterpret_cast<SubleqMem<> *>(smem)[tid >> 5];
   const LaneWords<32> t{reinterpret_cast<uint8_t *>(mem.tapes), tid & 31};
   const LaneWords<32> snap{reinterpret_cast<uint8_t *>(mem.snaps), tid & 31};
 

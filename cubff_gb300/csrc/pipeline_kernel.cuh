@@ -324,21 +324,22 @@ __device__ __forceinline__ void push_ready(const PipeCtx &b, const PipeQueue &q,
 // its latencies (index, programs, steps, two counters, queue) and, now and then, a
 // pair of thousands of steps.  64 epochs of 2^17 subleq programs 4.18 ms (5.79 with
 // tapes staged byte by byte, in an iteration of its own), of 40962 rsubleq4
-// programs 3.27 ms (4.27; 3.44 with 32 pairs to a warp).
+// programs 3.27 ms (4.27; 3.44 with 32 pairs to a warp); shared memory for those 16
+// lanes alone, instead of for 32, 5 to 8 % less for subleq.
 // iterate() is one iteration of the warp; it returns true if the lane made
 // progress.
 template <int L>
 struct LaneServer {
   SubleqMachine<(L == kRsubleq4)> m;
   uint32_t visits;
-  LaneWords<32> t, snap;
-
-  static constexpr uint32_t kWidth = 16;                   // lanes that hold pairs
-  static constexpr size_t kWarpBytes = sizeof(SubleqMem);  // of shared memory
+  static constexpr uint32_t kWidth = 16;  // lanes that hold pairs
+  using Mem = SubleqMem<kWidth>;
+  static constexpr size_t kWarpBytes = sizeof(Mem);  // of shared memory
+  LaneWords<kWidth> t, snap;
 
   __device__ __forceinline__ LaneServer(uint8_t *smem, const uint8_t *, uint32_t tid)
       : visits(0), t{smem + (tid >> 5) * kWarpBytes, tid & 31},
-        snap{t.s + sizeof(SubleqMem::tapes), tid & 31} {}
+        snap{t.s + sizeof(Mem::tapes), tid & 31} {}
 
   // Stages the pair of a lane in kIndex: bytes into shared memory, mutations.
   __device__ __forceinline__ void stage(const PipeSoup &sp, Lane &ln) {
@@ -610,10 +611,10 @@ __host__ __device__ constexpr size_t server_bytes() {
 
 // The persistent kernel of a pipelined launch over soups of language L.
 // Blocks per SM set the register budget: the BFF machines take 96 without
-// spills that matter (6 blocks, 80 registers: 39.9 ms instead of 35.1 on the
-// self-replicators above), the lanes' shared memory allows the others 4.
+// spills that matter (6 blocks, 80 registers: 13 % slower on the self-replicators
+// above); SUBLEQ needs 76.
 template <int L, uint32_t kLanes>
-__global__ void __launch_bounds__(kThreads, (L <= kForthtrivialReset) ? 5 : 4)
+__global__ void __launch_bounds__(kThreads, (L <= kForthtrivialReset) ? 5 : 6)
     pipeline_kernel(const __grid_constant__ PipeBatch pb) {
   extern __shared__ __align__(16) uint8_t smem[];
   uint8_t *tables = smem + server_bytes<L, kLanes>();
