@@ -1,4 +1,4 @@
-// launch_plan.h — how a pipelined launch is laid out on the device (host only).
+// launch_plan.h — how a pipelined launch is laid out on the device.
 #pragma once
 
 #include <algorithm>
@@ -57,6 +57,12 @@ struct PipePlan {
   uint32_t grid;  // blocks of kPipeWarps warps
 };
 constexpr uint32_t kPipeWarps = 4;
+
+// Whether a busy warp claims new pairs when so many of the `width` lanes that hold
+// pairs are idle: claim_min of 32, in proportion.
+__host__ __device__ constexpr bool idle_enough(uint32_t idle, uint32_t width, uint32_t claim_min) {
+  return idle * 32 >= claim_min * width;
+}
 
 // The lanes that a launch has at least, if it has as many pairs: 512 warps of 8,
 // about a block per SM, disturb each other little, so of a small soup all pairs

@@ -363,7 +363,7 @@ struct LaneServer {
     const uint32_t idle = __ballot_sync(0xffffffffu, ln.state == kIdle);
     const uint32_t busy = __ballot_sync(0xffffffffu, ln.state != kIdle && ln.state != kExhausted);
     const uint32_t lng = __ballot_sync(0xffffffffu, ln.state == kRun && visits >= b.tune.long_visits);
-    if (idle && (busy == 0 || (lng == 0 && __popc(idle) >= b.tune.claim_min)))
+    if (idle && (busy == 0 || (lng == 0 && idle_enough(__popc(idle), kWidth, b.tune.claim_min))))
       claim(b, q, ln, idle, lane);
     bool progressed = false;
 

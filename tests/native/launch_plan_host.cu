@@ -3,6 +3,10 @@
 
 using namespace cubff;
 
+extern "C" int claims(uint32_t idle, uint32_t width, uint32_t claim_min) {
+  return idle_enough(idle, width, claim_min);
+}
+
 // Pairs to a warp and blocks of a launch of total_pairs pairs, with narrow_per_sm
 // blocks of the narrow kernel and per_sm of the chosen one resident on an SM.
 extern "C" void launch_plan(int lang, uint64_t total_pairs, uint32_t lanes_per_pair64, int sms,

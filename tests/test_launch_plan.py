@@ -34,13 +34,26 @@ def plan():
     L.launch_plan.argtypes = [ctypes.c_int, ctypes.c_uint64, u32, ctypes.c_int, ctypes.c_int,
                               ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
 
+    L.claims.argtypes = [u32, u32, u32]
+
     def run(lang, pairs, lanes_per_pair64=32):
         out = np.zeros(2, dtype=np.uint32)
         L.launch_plan(LANGUAGES.index(lang), pairs, lanes_per_pair64, SMS, NARROW, WIDE,
                       out[0:].ctypes.data, out[1:].ctypes.data)
         return int(out[0]), int(out[1])
 
+    run.claims = L.claims
     return run
+
+
+def test_every_claim_threshold_can_be_met(plan):
+    """A busy warp (one lane of those that hold pairs is) claims under every
+    threshold but the highest, and sooner under a lower one."""
+    for width in (8, 16, 32):
+        needs = [next(i for i in range(width + 1) if plan.claims(i, width, c)) for c in range(1, 33)]
+        assert needs == sorted(needs) and needs[-1] == width
+        assert all(n < width for n in needs[:32 - 32 // width])
+        assert needs[19] == -(-20 * width // 32)
 
 
 @pytest.mark.parametrize("lang", LANGUAGES)
