@@ -64,20 +64,21 @@ __host__ __device__ constexpr bool idle_enough(uint32_t idle, uint32_t width, ui
   return idle * 32 >= claim_min * width;
 }
 
-// The lanes that a launch has at least, if it has as many pairs: 512 warps of 8,
-// about a block per SM, disturb each other little, so of a small soup all pairs
-// of an epoch are in flight (64 epochs of 1022 bff_noheads programs: 1.74 ms, with
-// half of them 2.05; of 8192: 2.49, 2.62; of 16384, where it would be two blocks
-// per SM: 3.61, 3.49).
-constexpr uint64_t kMinLanes = 4096;
-
 // Lanes in flight: enough to keep the SMs busy, few enough that most held
 // pairs are ready (a lane holding a pair of a later epoch only polls).
-// lanes_per_pair64 (x1/64) is tunable; the default keeps half an epoch of
-// pairs in flight, or kMinLanes of them.
-inline uint64_t lanes_wanted(uint64_t total_pairs, uint32_t lanes_per_pair64) {
-  const uint64_t want = total_pairs * uint64_t(lanes_per_pair64 ? lanes_per_pair64 : 32) / 64;
-  return std::max<uint64_t>(want, std::min<uint64_t>(total_pairs, kMinLanes));
+// lanes_per_pair64 (x1/64) is tunable; the default, kDefaultLanes, keeps half an
+// epoch of pairs in flight.  With that or more of them a launch has at least
+// kMinLanesPerSm to an SM, if it has as many pairs: so few warps disturb each other
+// little, so of a small soup all pairs of an epoch are in flight (64 epochs of 1022
+// bff_noheads programs: 1.74 ms, with half of them 2.05; of 8192: 2.49, 2.62; of
+// 16384, where it would be twice as many warps: 3.61, 3.49).  A caller who asks for
+// fewer, to leave room for other work, gets them.
+constexpr uint32_t kDefaultLanes = 32, kMinLanesPerSm = 27;
+inline uint64_t lanes_wanted(uint64_t total_pairs, uint32_t lanes_per_pair64, int sms) {
+  const uint64_t per64 = lanes_per_pair64 ? lanes_per_pair64 : kDefaultLanes;
+  const uint64_t want = std::max<uint64_t>(1, total_pairs * per64 / 64);
+  if (per64 < kDefaultLanes) return want;
+  return std::max<uint64_t>(want, std::min<uint64_t>(total_pairs, uint64_t(kMinLanesPerSm) * sms));
 }
 
 // Which width a launch of so many lanes takes.

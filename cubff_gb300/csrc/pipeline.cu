@@ -104,7 +104,7 @@ int plan_pipeline(int lang, int n_soups, uint64_t total_pairs, uint32_t lanes_pe
   int per_sm = 0;
   const PipeWidths widths = pipe_widths(lang);
   CUBFF_TRY(blocks_per_sm(k.kernel[0], lang, 0, n_soups, device, &per_sm));
-  const uint64_t lanes = lanes_wanted(total_pairs, lanes_per_pair64);
+  const uint64_t lanes = lanes_wanted(total_pairs, lanes_per_pair64, sms);
   const int w = choose_width(widths, lanes, sms, per_sm);
   if (w != 0) CUBFF_TRY(blocks_per_sm(k.kernel[w], lang, w, n_soups, device, &per_sm));
   *out = PipePlan{w, grid_of(widths.width[w], lanes, sms, per_sm)};

@@ -121,11 +121,13 @@ int cubff_shuffle_indices(uint64_t params_seed, uint64_t first_epoch,
  * (cubff_engine_tune), or set by hand.  The BFF and Forth families use only
  * lanes_per_pair64: their warps run each pair to the end once they have it. */
 typedef struct {
-  uint32_t lanes_per_pair64;  /* lanes in flight per 64 pairs of an epoch (grid size);
-                                 at least 4096 if there are as many pairs               */
+  uint32_t lanes_per_pair64;  /* lanes in flight per 64 pairs of an epoch (grid size); from
+                                 32, the default, on at least 27 per SM if there are as
+                                 many pairs                                             */
   uint32_t steps_per_visit;   /* interpreter steps a lane takes per iteration of its warp
                                  after its first                                        */
-  uint32_t claim_min;         /* idle lanes a busy warp needs before it claims new pairs  */
+  uint32_t claim_min;         /* idle lanes, of 32 in proportion, that a busy warp needs
+                                 before it claims new pairs                             */
   uint32_t long_visits;       /* a pair running longer than this many visits keeps its
                                  warp from claiming (0 = never)                           */
   uint32_t first_visit_steps; /* steps of a pair's first visit (most pairs end in it; a

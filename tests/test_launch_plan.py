@@ -80,6 +80,17 @@ def test_width_by_the_size_of_the_launch(plan, lang, programs, pairs_of_a_warp):
     assert plan(lang, programs // 2)[0] == pairs_of_a_warp
 
 
+@pytest.mark.parametrize("lang", ["bff", "forth", "subleq"])
+def test_fewer_lanes_are_had_by_asking(plan, lang):
+    """The minimum of lanes is for launches that ask for the default or more: one
+    that leaves room for others gets as few as it asks for, on any device."""
+    pairs = 2000
+    assert plan(lang, pairs, 64) == plan(lang, pairs, 32)  # all pairs at once
+    grids = [plan(lang, pairs, per64)[1] for per64 in (1, 4, 8, 16, 24, 31, 32)]
+    assert grids == sorted(grids) and len(set(grids[:5])) == 5
+    assert grids[3] <= grids[-1] // 3
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("lang,n,count", [("bff8", 29182, 1), ("bff8_noheads", 29186, 1),
                                           ("forth", 58366, 1), ("forthtrivial", 58370, 1),
