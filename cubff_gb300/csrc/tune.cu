@@ -3,27 +3,27 @@
 //
 // The reference launches every epoch with one fixed shape: ceil(N/64)
 // blocks of 32 threads, one thread per pair (common_language.h:348,
-// :490-493).  The pipelined launch here has five knobs (cubff_tuning): lanes
-// in flight per 64 pairs, steps per visit (the first, and the later ones),
-// the claim threshold of busy warps and the visit count after which a pair
+// :490-493).  The pipelined launch here has up to five knobs (cubff_tuning): lanes
+// in flight per 64 pairs and, for SUBLEQ, steps per visit (the first, and the later
+// ones), the claim threshold of busy warps and the visit count after which a pair
 // keeps its warp from claiming.  The best values depend on the language
 // (step cost, how long pairs run), on the number of programs in the launch
 // and on how many soups share it, so the engine keeps one shape per
 // (language, log2 programs, log2 soups) key.
 //
 // Tuning runs a few epochs of scratch copies of the caller's soups under
-// candidate shapes (coordinate descent from the default: each knob in turn
-// over a short list of values, the others fixed; two passes), per language,
-// timed on the host around the synchronous run.  Every candidate must give
-// the same op counts (shapes change timing only); a disagreement is an error.
+// candidate shapes (tune_search.h; those that give the same launch are run once),
+// per language, timed on the host around the synchronous run.  Every candidate must
+// give the same op counts (shapes change timing only); a disagreement is an error.
 #include <algorithm>
 #include <chrono>
-#include <cstring>
 #include <vector>
 
 #include "common.cuh"
 #include "engine_impl.h"
 #include "internal.h"
+#include "launch_plan.h"
+#include "tune_search.h"
 
 using namespace cubff;
 
@@ -83,56 +83,52 @@ int run_trial(cubff_engine *eng, std::vector<Clone> &clones, uint32_t epochs,
   return CUBFF_OK;
 }
 
-bool same_shape(const cubff_tuning &a, const cubff_tuning &b) {
-  return std::memcmp(&a, &b, sizeof(a)) == 0;
+// Whether two shapes give the clones of one language the same launches: the same
+// kernel and grid for every launch group, and the same knobs of its lanes.
+int same_launch(cubff_engine *eng, const std::vector<Clone> &clones, bool visits,
+                const cubff_tuning &a, const cubff_tuning &b, bool *same) {
+  *same = !visits || (a.steps_per_visit == b.steps_per_visit && a.claim_min == b.claim_min &&
+                      a.long_visits == b.long_visits && a.first_visit_steps == b.first_visit_steps);
+  for (size_t g0 = 0; *same && g0 < clones.size(); g0 += kMaxPipeSoups) {
+    const size_t g1 = std::min(clones.size(), g0 + kMaxPipeSoups);
+    uint64_t pairs = 0;
+    for (size_t i = g0; i < g1; i++) pairs += clones[i].orig->p.num_programs / 2;
+    PipePlan pa, pb;
+    const int lang = clones[g0].orig->p.lang, n = static_cast<int>(g1 - g0);
+    CUBFF_TRY(plan_pipeline(lang, n, pairs, a.lanes_per_pair64, eng->device, &pa));
+    CUBFF_TRY(plan_pipeline(lang, n, pairs, b.lanes_per_pair64, eng->device, &pb));
+    *same = pa.which == pb.which && pa.grid == pb.grid;
+  }
+  return CUBFF_OK;
 }
 
-// Coordinate descent for the clones of one language.
+// The search for the clones of one language.
 int tune_language(cubff_engine *eng, std::vector<Clone> &clones, uint32_t epochs,
                   cubff_tuning *best_out) {
-  static const uint32_t kLanes[] = {16, 24, 32, 48, 64};
-  static const uint32_t kSteps[] = {16, 32, 64, 128, 256};
-  static const uint32_t kClaim[] = {8, 14, 20, 26, 32};
-  static const uint32_t kLong[] = {0, 1, 2, 4, 8};
-  static const uint32_t kFirst[] = {4, 8, 16, 32, 64};
   cubff_tuning best = default_shape();
-  Trial warm, ref;
-  CUBFF_TRY(run_trial(eng, clones, epochs, best, &warm));  // pairings cached, caches warm
-  CUBFF_TRY(run_trial(eng, clones, epochs, best, &ref));
-  double best_s = std::min(warm.seconds, ref.seconds);
-  auto time_of = [&](const cubff_tuning &cand, double *sec) -> int {
-    Trial a, b;
-    CUBFF_TRY(run_trial(eng, clones, epochs, cand, &a));
-    CUBFF_TRY(run_trial(eng, clones, epochs, cand, &b));
-    if (a.ops != ref.ops || b.ops != ref.ops)
-      return set_error(CUBFF_EDEVICE, "tune: launch shapes gave different op counts");
-    *sec = std::min(a.seconds, b.seconds);
-    return CUBFF_OK;
-  };
-  for (int pass = 0; pass < 2; pass++) {
-    for (int knob = 0; knob < 5; knob++) {
-      const uint32_t *vals = knob == 0 ? kLanes : knob == 1 ? kSteps : knob == 2 ? kClaim
-                             : knob == 3 ? kLong : kFirst;
-      cubff_tuning round_best = best;
-      for (int v = 0; v < 5; v++) {
-        cubff_tuning cand = best;
-        uint32_t *field = knob == 0 ? &cand.lanes_per_pair64
-                          : knob == 1 ? &cand.steps_per_visit
-                          : knob == 2 ? &cand.claim_min
-                          : knob == 3 ? &cand.long_visits
-                                      : &cand.first_visit_steps;
-        *field = vals[v];
-        if (same_shape(cand, best)) continue;
-        double sec = 0;
-        CUBFF_TRY(time_of(cand, &sec));
-        if (sec < best_s) {
-          best_s = sec;
-          round_best = cand;
-        }
-      }
-      best = round_best;
-    }
-  }
+  Trial ref;
+  CUBFF_TRY(run_trial(eng, clones, epochs, best, &ref));  // pairings cached, caches warm
+  const bool visits = clones[0].orig->p.lang > kForthtrivialReset;
+  int failed = CUBFF_OK;
+  const int st = search_shape(
+      visits, &best,
+      [&](const cubff_tuning &cand, double *sec) -> int {
+        CUBFF_TRY(failed);
+        Trial a, b;
+        CUBFF_TRY(run_trial(eng, clones, epochs, cand, &a));
+        CUBFF_TRY(run_trial(eng, clones, epochs, cand, &b));
+        if (a.ops != ref.ops || b.ops != ref.ops)
+          return set_error(CUBFF_EDEVICE, "tune: launch shapes gave different op counts");
+        *sec = std::min(a.seconds, b.seconds);
+        return CUBFF_OK;
+      },
+      [&](const cubff_tuning &a, const cubff_tuning &b) {
+        bool same = false;
+        if (failed == CUBFF_OK) failed = same_launch(eng, clones, visits, a, b, &same);
+        return same;
+      });
+  CUBFF_TRY(st);
+  CUBFF_TRY(failed);
   *best_out = best;
   return CUBFF_OK;
 }
