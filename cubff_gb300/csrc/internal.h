@@ -43,7 +43,7 @@ struct EpochArgs {
   unsigned long long *raw;              // += raw iterations (nullable)
 };
 
-// A pipelined launch runs epochs of one or more soups (pipeline.cu).  Soups
+// A pipelined launch runs epochs of one or more soups (pipeline_kernel.cuh).  Soups
 // are listed grouped by language; each language has one ready queue.
 struct PipeSoup {
   uint8_t *soup;
@@ -77,7 +77,8 @@ struct PipeQueue {
 // lanes in flight per 64 pairs; results never depend on them).
 struct PipeTuning {
   uint32_t steps_per_visit;  // interpreter steps a running lane takes per warp iteration
-  uint32_t claim_min;        // idle lanes a busy warp needs before it claims new pairs
+  uint32_t claim_min;        // idle lanes, of 32 in proportion, that a busy warp needs
+                             // before it claims new pairs
   uint32_t long_visits;      // visits after which a pair counts as long: its warp stops
                              // claiming, so the pair runs without new warp-mates
   uint32_t first_visit_steps;  // steps of a pair's first visit

@@ -65,8 +65,9 @@ constexpr int kCountSlots = kPipeCountSlots;  // per-epoch counter slots (spread
 // and `exhausted` once a claim falls past the queue's last task.
 //
 // How a warp runs its pairs depends on the language family (LaneServer,
-// StagedServer).  Launch-shape knobs (PipeTuning, chosen by the host; the BFF
-// and Forth families run a pair to its end and use only the grid size):
+// StagedServer), how many it holds at once on the size of the launch (launch_plan.h).
+// Launch-shape knobs (PipeTuning, chosen by the host; the BFF and Forth families run
+// a pair to its end and use none of them):
 //  * steps_per_visit: interpreter steps a running lane takes per iteration of
 //    its warp after its first (an iteration lasts as long as its busiest
 //    lane, so a lane given more steps holds its warp-mates, and the pairs
@@ -77,8 +78,9 @@ constexpr int kCountSlots = kPipeCountSlots;  // per-epoch counter slots (spread
 //    them holds the others (whose consumers wait on them) before they can
 //    write back;
 //  * claim_min: a warp with running lanes claims new slots only once this
-//    many of its lanes are idle (an idle warp claims at once), so a slot held
-//    by a busy warp is polled only between its long iterations;
+//    many of 32 of its lanes, in proportion, are idle (an idle warp claims at once;
+//    at 32, the default, no other does), so a slot held by a busy warp is polled
+//    only between its long iterations;
 //  * long_visits: a pair still running after this many visits is long.  A
 //    warp holding a long pair claims nothing new: its other lanes drain, and
 //    the long pair, which the next epochs' pairs wait on, steps without

@@ -119,7 +119,8 @@ int cubff_shuffle_indices(uint64_t params_seed, uint64_t first_epoch,
 /* Launch shape of a pipelined launch.  Results never depend on it; only the
  * time does.  Chosen per launch group by the engine's tuner
  * (cubff_engine_tune), or set by hand.  The BFF and Forth families use only
- * lanes_per_pair64: their warps run each pair to the end once they have it. */
+ * lanes_per_pair64: their warps run each pair to the end once they have it.
+ * The defaults: 32, 64, 32, 1, 64. */
 typedef struct {
   uint32_t lanes_per_pair64;  /* lanes in flight per 64 pairs of an epoch (grid size); from
                                  32, the default, on at least 27 per SM if there are as
