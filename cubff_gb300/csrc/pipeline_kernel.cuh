@@ -430,7 +430,8 @@ struct LaneServer {
 // 82 ms, one after the other 594; bff8 2^17: 178, 340.  With 5 of 8 instead of 6
 // Forth soups with some long pairs lose 5 to 15 %, as each waits for the slowest;
 // with 7 instead of all of 8 bff8 soups up to 30 %, and with 20 of 32 instead of 28
-// as much again.)
+// as much again.  The last eighth of a warp's pairs goes back to the whole warp in
+// bff8: 2^16 evolved programs 84 ms, 104 if not; forthtrivial 2^12 would lose half.)
 //
 // So that pairs wait behind few others, a warp holds 8 unless there are very many
 // (launch_plan.h): a soup of 2^17 bff programs taken over by self-replicators takes
@@ -446,7 +447,7 @@ struct StagedServer {
   Mem &mem;
   LaneWords<kWidth> t, stk;
   const uint8_t *optab, *cmdflag;
-  static constexpr int kCrowd = Stages<L>::crowd(kLanes);
+  static constexpr int kCrowd = Stages<L>::crowd(kLanes), kLast = Stages<L>::last(kLanes);
   static constexpr int kCrowdSteps = 256;  // of a lane in an iteration
   bool crowd;   // the lanes take pairs on themselves
   int went_on;  // pairs of this claim that went on
@@ -538,7 +539,7 @@ struct StagedServer {
     bool together = false;
     if constexpr (Stages<L>::kCrowds) {
       crowd |= __popc(lng) >= kCrowd;
-      together = crowd && lng != 0;
+      together = crowd && __popc(lng) > kLast;
       if (together && ln.state == kLong) {
         LaneM x = m;
         take_on(x, t, stk, optab, mem.cycles[lane]);
